@@ -8,7 +8,7 @@
    The checkout is the directory named by ``--reference DIR`` or the
    ``EMERALD_REFERENCE_ROOT`` environment variable, else the build
    container's read-only copy at ``/root/reference``. Built only where that
-   directory exists; the built file is git-ignored but travels with the
+   directory holds the sources; the built file is git-ignored but travels with the
    working tree.
 
 3. ``oracle/libfp64_oracle.so`` — the FP64 GPU oracle of the five solvers'
@@ -107,7 +107,8 @@ def build_fp64(force=False):
 
 
 def build_reference(force=False):
-    if not os.path.isdir(REF_ROOT):
+    # an empty directory stands for a checkout that was not mounted
+    if not os.path.isfile(os.path.join(REF_ROOT, REF_SOURCES[0])):
         return REF_SO if os.path.exists(REF_SO) else None
     shim = os.path.join(HERE, "ref_shim")
     deps = [os.path.join(REF_ROOT, s) for s in REF_SOURCES]
