@@ -262,6 +262,9 @@ Engine::Engine(uint32_t fluid_capacity, uint32_t solid_capacity, int max_scenes)
     stile_scene_.assign(S / kTile, -1);
     upload_tiles();
     update_extent();
+    // the clears above ran on the legacy default stream, which the stream a
+    // caller sets next may not wait for
+    cudaStreamSynchronize(nullptr);
     check("engine allocation");
 }
 
@@ -553,7 +556,10 @@ void Engine::build_near_map(Scene& sc, float const* solid_xy, uint32_t n_solid) 
             }
         }
     }
-    if (cudaMemcpy(d_near_ + begin, bits.data(), 4 * words, cudaMemcpyHostToDevice) != cudaSuccess) {
+    // on the engine's stream: a request loop's streams do not wait for the
+    // legacy default stream, whose copy could land after the sub-step
+    if (cudaMemcpyAsync(d_near_ + begin, bits.data(), 4 * words, cudaMemcpyHostToDevice, st_) !=
+        cudaSuccess) {
         near_words_.release(begin, uint32_t(words));
         check("near map upload");
         return;

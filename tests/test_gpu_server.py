@@ -105,3 +105,18 @@ def test_server_footprint_matches_allocation(E):
     assert st["device_bytes"] <= (256 << 20)
     # allocation granularity and the loop's stream and events on top
     assert st["device_bytes"] <= used <= st["device_bytes"] + (64 << 20), (used, st)
+
+
+def test_bursts_on_several_lanes_equal_alone(E):
+    """Requests that several lanes admit and step at the same time: the copies
+    of one lane's admission are ordered before its own sub-steps."""
+    srv = E.Server(64 << 20, "dfsph_p", max_scenes=16, lanes=4)
+    scenes = [scene(E, 40 + 9 * k, 20 + k) for k in range(6)]
+    want = [alone(E, sc, 4) for sc in scenes]
+    for burst in range(12):
+        ids = [srv.submit_block_scene(sc, 4) for sc in scenes]
+        for k, rid in enumerate(ids):
+            x, v, _, _ = srv.wait(rid, 60000)
+            assert_bitwise(x, want[k][0], "burst %d request %d x" % (burst, k))
+            assert_bitwise(v, want[k][1], "burst %d request %d v" % (burst, k))
+    srv.close()
