@@ -15,7 +15,9 @@ BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libemerald_b200.so")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
-SOURCES = ["build_kernels.cu", "solve_kernels.cu", "sort_kernels.cu", "engine.cu", "capi.cu",
+SOURCES = ["build_kernels.cu", "solve_kernels.cu",
+           "resident_dfsph.cu", "resident_iisph.cu", "resident_iisph_ap.cu",
+           "resident_iisph_pseudo_ap.cu", "resident_pcisph.cu", "sort_kernels.cu", "engine.cu", "capi.cu",
            "scene.cpp", "noalloc.cu", "reorder_kernels.cu", "server.cpp", "common_ops.cu",
            "solver_ops.cu", "sort_ops.cu"]
 

@@ -68,9 +68,12 @@ public:
     // (request-loop lanes, size classes without a tuned entry) start there.
     struct Tuning {
         int apply = 1, divergence = 4, iisph_sum = 4, iisph_beta = 4;
+        // sub-steps run the resident solve where it fits (the kernels above
+        // then serve what it does not cover)
+        bool resident = true;
         bool operator==(Tuning const& o) const {
             return apply == o.apply && divergence == o.divergence && iisph_sum == o.iisph_sum &&
-                   iisph_beta == o.iisph_beta;
+                   iisph_beta == o.iisph_beta && resident == o.resident;
         }
     };
     struct TuneReport {
@@ -244,6 +247,13 @@ private:
     void destroy_graphs();
     void capture_frame(int32_t method, bool reorder);
     void prepare_substep(int32_t method);
+    // The resident solve (resident_kernels.cu): whether sub-steps of `method`
+    // run it now, and its division of the active scenes among blocks.
+    bool use_resident(int32_t method);
+    int graph_key(int32_t method, bool reorder);
+    void plan_resident(int32_t method);
+    void divide_scenes(uint32_t blocks);
+    ResidentLimits const& limits_of(int32_t method);
     int64_t frames_launched_ = 0;
     bool frame_graphs_ok_ = true;
     void host_wait(cudaStream_t s) {
@@ -251,8 +261,17 @@ private:
         cudaStreamSynchronize(s);
     }
     int64_t host_waits_ = 0;
+    std::map<int32_t, ResidentLimits> limits_;  // key: method * 2 + compensated
+    ResidentPlan plans_[5] = {};       // per method
+    std::vector<GangPart> parts_;
+    bool parts_valid_ = false;  // false: the scenes changed since parts_ was made
+    uint32_t largest_share_ = 1;
+    uint64_t total_tiles_ = 0;
+    GangPart* d_parts_ = nullptr;
+    uint32_t* d_nparts_ = nullptr;
+    uint32_t parts_cap_ = 0;
     cudaStream_t frame_st_ = nullptr;                  // frame-loop body capture
-    std::map<int32_t, cudaGraphExec_t> frame_graphs_;  // key: method * 2 + reorder
+    std::map<int32_t, cudaGraphExec_t> frame_graphs_;  // key: graph_key
     std::map<int32_t, int64_t> frame_fixed_kernels_;   // per graph, outside the loop
     int64_t frame_body_kernels_[5] = {0, 0, 0, 0, 0};  // per method, one frame iteration
     int max_iterations(int kind) const;
@@ -298,7 +317,7 @@ private:
     cudaStream_t body_st_ = nullptr;
     cudaStream_t side_st_ = nullptr;  // parallel branch of a sub-step
     cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
-    std::map<int32_t, cudaGraphExec_t> graphs_;        // key: method * 2 + reorder
+    std::map<int32_t, cudaGraphExec_t> graphs_;        // key: graph_key
     std::map<int32_t, int64_t> graph_fixed_kernels_;
 #ifndef EMERALD_REORDER_EVERY
 #define EMERALD_REORDER_EVERY 16

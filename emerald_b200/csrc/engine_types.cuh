@@ -30,7 +30,7 @@ enum Method : int { kPcisph = 0, kIisph = 1, kIisphAp = 2, kIisphPseudoAp = 3, k
 enum StepMode : int { kFixedDt = 0, kFrame = 1 };
 
 // Error bits reported through SceneState::error.
-enum ErrorBits : int { kErrTableFull = 1, kErrNonFinite = 2 };
+enum ErrorBits : int { kErrTableFull = 1, kErrNonFinite = 2, kErrStalled = 4 };
 
 // External force terms, the reference's force functions
 // (emerald/sph2d_box/forces.cpp): gravity (accumulate_gravity_forces,
@@ -83,6 +83,10 @@ struct SceneParams {
     int32_t force_array;
     ForceTerm force_terms[kMaxForceTerms];
     float fixed_t;  // the caller's sub-step time (fixed-dt mode)
+    // Error sums below which an average passes its threshold, per loop kind 0
+    // to 2 (iisph_err_avg, dfsph_dens_avg, dfsph_div_avg): the test
+    // float(double(sum) / (1000 n)) <= threshold is monotone in the sum.
+    uint64_t sum_limit[3];
 };
 
 // Mutable per-scene state, device resident.
@@ -109,6 +113,31 @@ struct SceneState {
     double stat_avg_exact, stat_div_avg_exact;
 };
 
+// What the blocks that solve one scene together (its gang, see
+// resident_solve.cuh) share: arrivals at their barriers, and whether some
+// block needs the barrier form. Cleared by k_begin_substep.
+struct alignas(64) GangState {
+    uint32_t arrive;
+    uint32_t plain;
+};
+
+// A block's error sums of one solver iteration: 32 bits of value and the tag
+// above them in every word (the sum's low part and the maximum, the whole sum,
+// the exact sum).
+struct alignas(16) GangRecord {
+    unsigned long long w[6];
+};
+
+// One block's share of a scene in the resident solve: warp tiles
+// [tile, tile + tiles) of the scene (32 particles each), as block `rank` of
+// the `size` blocks of its gang.
+struct GangPart {
+    int32_t scene;
+    uint32_t tile, tiles;
+    uint32_t rank, size;
+    uint32_t base;  // index of the gang's first share
+};
+
 // Raw device pointers of an arena, passed by value to every kernel.
 struct Arena {
     SceneParams const* sp;
@@ -123,6 +152,11 @@ struct Arena {
     int32_t* loop_scene;
     uint32_t* loop_wt0;
     uint32_t* loop_n;
+    // resident solve: per-scene gang states, the next share to take, and the
+    // shares' error records (two each)
+    GangState* gangs;
+    uint32_t* gang_ticket;
+    GangRecord* records;
     int32_t batch;  // the arena holds more than one scene slot (loop kernels walk the work list)
     int32_t const* tile_scene;   // fluid tile -> scene (-1: free)
     int32_t const* stile_scene;  // solid tile -> scene

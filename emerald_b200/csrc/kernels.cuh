@@ -136,4 +136,32 @@ void launch_pc_density(Arena const& a, uint32_t tiles, cudaStream_t st, bool com
 void launch_pc_forces(Arena const& a, uint32_t tiles, cudaStream_t st, bool comp);
 void launch_pc_final(Arena const& a, uint32_t tiles, cudaStream_t st);
 
+// resident solve (resident_kernels.cu): everything of a sub-step after the
+// neighbour lists as one cooperative launch
+constexpr int kResidentForms = 4;
+struct ResidentLimits {
+    uint32_t blocks;  // blocks that are resident together (0: not available)
+    uint32_t share;   // warp tiles of a block at most
+    uint32_t smem;    // dynamic shared memory of a block at most
+    // per compiled form: warps of a block that solve tiles at most (one more
+    // keeps the exit test), and tiles of each at most (0: any number)
+    uint32_t warps[kResidentForms];
+    uint32_t tiles[kResidentForms];
+};
+struct ResidentPlan {
+    GangPart const* parts;   // device: the shares, a gang's consecutive
+    uint32_t const* nparts;  // device
+    uint32_t grid, threads, smem;
+    uint32_t form;
+    uint32_t share;          // warp tiles of a share at most
+};
+template <int METHOD>
+bool resident_limits_of(bool comp, ResidentLimits& l);
+// Shared memory a block asks for when its shares have at most `tiles` warp
+// tiles: room for 24 list rows a tile, `most` at most.
+template <int METHOD>
+uint32_t resident_smem_of(uint32_t tiles, uint32_t most);
+template <int METHOD>
+cudaError_t launch_resident_of(Arena const& a, ResidentPlan const& p, bool comp, cudaStream_t st);
+
 }  // namespace emerald

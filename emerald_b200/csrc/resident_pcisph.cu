@@ -1,0 +1,12 @@
+// The resident solve of one method (its own source file, so that the methods
+// compile in parallel).
+#include "resident_solve.cuh"
+
+namespace emerald {
+
+template bool resident_limits_of<kPcisph>(bool, ResidentLimits&);
+template uint32_t resident_smem_of<kPcisph>(uint32_t, uint32_t);
+template cudaError_t launch_resident_of<kPcisph>(Arena const&, ResidentPlan const&, bool,
+                                            cudaStream_t);
+
+}  // namespace emerald

@@ -15,6 +15,7 @@
 
 #include "engine_types.cuh"
 #include "kernels.cuh"
+#include "solve_math.cuh"
 #include "sph_math.cuh"
 
 namespace emerald {
@@ -22,14 +23,6 @@ namespace emerald {
 namespace {
 
 constexpr double kFlicksPerSecond = 705600000.0;
-
-// Block-level setup shared by the per-particle kernels. A tile belongs to
-// one scene, so the scene checks are uniform across the block.
-struct Ctx {
-    int32_t s;
-    uint32_t i;
-    bool live;
-};
 
 __device__ __forceinline__ bool enter(Arena const& a, bool skip_done, Ctx& c) {
     c.s = a.tile_scene[blockIdx.x];
@@ -132,6 +125,8 @@ __device__ int to_int_x86(double d) {
 __global__ void k_begin_substep(Arena a, int nscenes) {
     int const s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nscenes) return;
+    if (s == 0) *a.gang_ticket = 0u;
+    a.gangs[s] = GangState{};
     SceneParams const& P = a.sp[s];
     SceneState& S = a.ss[s];
     if (!S.active) return;
@@ -219,10 +214,6 @@ __global__ void k_zero_kappas(Arena a) {
     if (!enter(a, false, c) || !c.live) return;
     a.kdiv[c.i] = 0.0f;
     a.kdens[c.i] = 0.0f;
-}
-
-__device__ __forceinline__ int iteration_cap(SceneParams const& P, int kind) {
-    return kind == 0 ? P.iisph_max_iter : (kind == 3 ? 6 : P.dfsph_max_iter);
 }
 
 // Rebuilds the solver-loop work list (Arena::loop_scene, loop_wt0,
@@ -335,51 +326,15 @@ __device__ void exit_test(Arena const& a, int nscenes, int kind, int* running,
         unsigned long long const err_sum = fresh ? atomicAdd(&S.err_sum, 0ull) : S.err_sum;
         uint32_t const err_max = fresh ? atomicMax(&S.err_max, 0u) : S.err_max;
         double const err_sum_d = fresh ? atomicAdd(&S.err_sum_d, 0.0) : S.err_sum_d;
-        double const n = static_cast<double>(1000ull * P.fluid_count);
-        float const avg = P.fluid_count
-                            ? static_cast<float>(static_cast<double>(err_sum) / n)
-                            : 0.0f;
-        // the exact mean of the errors, reported beside the reference's
-        // metric (which drops each particle's error below 0.1%)
-        double const exact = P.fluid_count ? err_sum_d / static_cast<double>(P.fluid_count) : 0.0;
-        float const mx = __uint_as_float(err_max);
-        bool conv = false;
-        int const max_iter = iteration_cap(P, kind);
-        if (kind == 0) {
-            conv = S.iter > 1 && avg <= P.iisph_err_avg && mx <= P.iisph_err_max;
-            S.stat_avg = avg;
-            S.stat_max = mx;
-        } else if (kind == 1) {
-            if (S.iter > 1) {
-                conv = avg <= P.dfsph_dens_avg && mx <= P.dfsph_dens_max;
-                S.stat_avg = avg;
-                S.stat_max = mx;
-                S.stat_avg_exact = exact;
-            }
-        } else if (kind == 2) {
-            if (S.iter > 0) {
-                conv = avg <= P.dfsph_div_avg && mx <= P.dfsph_div_max;
-                S.stat_div_avg = avg;
-                S.stat_div_max = mx;
-                S.stat_div_avg_exact = exact;
-            }
-        } else {
-            if (S.iter > 1) {
-                conv = (mx / P.rho0) <= 0.01f;
-                S.stat_max = mx / P.rho0;
-            }
-        }
+        bool const ends = loop_ends(P, kind, S.iter, err_sum, err_max);
+        report_loop(P, S, kind, S.iter, err_sum, err_max, ends);
+        report_exact_mean(P, S, kind, S.iter, err_sum_d);
         S.iter += 1;
         S.err_sum = 0ull;
         S.err_max = 0u;
         S.err_sum_d = 0.0;
-        if (conv || S.iter >= max_iter) {
+        if (ends) {
             S.done = 1;
-            if (kind == 2) {
-                S.stat_div_iters = S.iter;
-            } else {
-                S.stat_iters = S.iter;
-            }
         } else {
             any = 1;
         }
@@ -423,18 +378,203 @@ __device__ __forceinline__ void fused_exit_test(Arena const& a, LoopCheck const&
     }
 }
 
-// --------------------------------------------------------- shared SPH sums
+// The per-particle functions of solve_math.cuh over the arena's own lists and
+// values, their results written to the arena.
 
-// Visits particle i's fluid list in list order, CH entries at a time: a
-// chunk first loads its indices and kernel gradients, then every gathered
-// neighbour value, then folds them into the sum in order. The loads of a
-// chunk are independent, so they are in flight together; the sum is the
-// same sequence of operations as a plain loop. The chunk of each kernel is
-// a launch-time choice among 1, 4 and 8 (Tuning, set by the autotuner).
-// These two are the chunks of callers that pass none (the IISPH final
-// velocity update); the engine's DFSPH launches pass their Tuning's.
-constexpr int kDivergenceChunk = 8;
-constexpr int kPressureChunk = 4;
+template <bool K, int CH>
+__device__ __forceinline__ float divergence_at(Arena const& a, SceneParams const& P, uint32_t i) {
+    return divergence_of<K, CH>(P, a.nf_cnt[i], a.ns_cnt[i], a.v[i], ArenaSource<float2>{a.v},
+                                ArenaList{a, i}, ArenaBoundary{a, i, P.rho0});
+}
+
+template <bool K, int CH = kPressureChunk>
+__device__ __forceinline__ float2 apply_pressure_at(Arena const& a, SceneParams const& P,
+                                                    uint32_t i, float2 v, float const* q,
+                                                    float dt) {
+    return apply_pressure_of<K, CH>(P, a.nf_cnt[i], a.ns_cnt[i], v, q[i], ArenaSource<float>{q},
+                                    dt, ArenaList{a, i}, ArenaBoundary{a, i, P.rho0});
+}
+
+template <bool K>
+__device__ __forceinline__ float2 pressure_accel_at(Arena const& a, SceneParams const& P,
+                                                    uint32_t i) {
+    return pressure_accel_of<K>(P, a.nf_cnt[i], a.ns_cnt[i], a.qdens[i],
+                                ArenaSource<float>{a.qdens}, ArenaList{a, i},
+                                ArenaBoundary{a, i, P.rho0});
+}
+
+// Density, alpha, the per-frame kappa reset, and the p/rho^2 caches of both
+// warm starts.
+template <bool K>
+__device__ __forceinline__ void dfsph_density_alpha_at(Arena const& a, Ctx const& c) {
+    uint32_t const i = c.i;
+    float rho, alpha;
+    dfsph_density_alpha<K>(a, a.sp[c.s], i, a.nf_cnt[i], a.ns_cnt[i], ArenaList{a, i}, rho, alpha);
+    a.rho[i] = rho;
+    a.alpha[i] = alpha;
+    float kdiv = a.kdiv[i];
+    float kdens = a.kdens[i];
+    if (a.ss[c.s].new_frame) {
+        kdiv = 0.0f;
+        kdens = 0.0f;
+        a.kdiv[i] = kdiv;
+        a.kdens[i] = kdens;
+    }
+    a.qdiv[i] = p_over_rho2(kdiv, rho);
+    a.qdens[i] = p_over_rho2(kdens, rho);
+}
+
+__device__ __forceinline__ float dfsph_divergence_step_at(Arena const& a, SceneParams const& P,
+                                                          uint32_t i, float dt, float d) {
+    DfsphStep const r = dfsph_divergence_step(P, dt, a.rho[i], a.alpha[i], d);
+    a.rho_star[i] = r.star;
+    a.kdiv[i] = r.kappa;
+    a.qdiv[i] = r.q;
+    return r.err;
+}
+
+__device__ __forceinline__ float dfsph_density_step_at(Arena const& a, SceneParams const& P,
+                                                       uint32_t i, float dt, float rho,
+                                                       float div) {
+    DfsphStep const r = dfsph_density_step(P, dt, rho, a.alpha[i], div);
+    a.rho_star[i] = r.star;
+    a.kdens[i] = r.kappa;
+    a.qdens[i] = r.q;
+    return r.err;
+}
+
+// compute_densities, integrate_velocities_in_place and iisph_compute_diis
+// (iisph_ops.cpp:20-90), plus the zero initial pressures (iisph.cpp:76).
+template <bool K>
+__device__ __forceinline__ void iisph_density_dii_at(Arena const& a, Ctx const& c) {
+    SceneParams const& P = a.sp[c.s];
+    uint32_t const i = c.i;
+    float const dt = a.ss[c.s].dt;
+    float const d = density_of<K>(a, P, i);
+    a.rho[i] = d;
+    a.v[i] = integrate_external(a, P, i, a.v[i], dt);
+    a.dii[i] = iisph_dii<K>(P, dt, d, a.nf_cnt[i], a.ns_cnt[i], ArenaList{a, i},
+                            ArenaBoundary{a, i, P.rho0});
+    a.pbuf0[i] = 0.0f;
+}
+
+struct ArenaRhoV {
+    Arena const& a;
+    __device__ __forceinline__ RhoV at(uint32_t j) const { return RhoV{a.rho[j], a.v[j]}; }
+};
+
+template <bool K>
+__device__ __forceinline__ void iisph_aii_at(Arena const& a, Ctx const& c) {
+    SceneParams const& P = a.sp[c.s];
+    uint32_t const i = c.i;
+    float aii, star;
+    iisph_aii<K>(P, a.ss[c.s].dt, a.rho[i], a.v[i], a.dii[i], a.nf_cnt[i], a.ns_cnt[i],
+                 ArenaRhoV{a}, ArenaList{a, i}, ArenaBoundary{a, i, P.rho0}, aii, star);
+    a.aii[i] = aii;
+    a.rho_star[i] = star;
+}
+
+struct ArenaPRho {
+    Arena const& a;
+    float const* p;
+    __device__ __forceinline__ float2 at(uint32_t j) const { return mk2(p[j], a.rho[j]); }
+};
+
+template <bool K, int CH>
+__device__ __forceinline__ void iisph_sum_dij_at(Arena const& a, Ctx const& c) {
+    SceneState const& S = a.ss[c.s];
+    a.sdp[c.i] = iisph_sum_dij<K, CH>(a.sp[c.s], S.dt, a.nf_cnt[c.i],
+                                      ArenaPRho{a, pressures_cur(a, S)}, ArenaList{a, c.i});
+}
+
+struct ArenaIisph {
+    Arena const& a;
+    float const* p;
+    __device__ __forceinline__ IisphNeighbor at(uint32_t j) const {
+        return IisphNeighbor{a.rho[j], p[j], a.sdp[j], a.dii[j]};
+    }
+};
+
+// Returns whether the particle's error counts (a_ii != 0).
+template <bool K, int CH>
+__device__ __forceinline__ bool iisph_beta_pressure_at(Arena const& a, Ctx const& c, SceneState* S,
+                                                       float& err) {
+    SceneParams const& P = a.sp[c.s];
+    uint32_t const i = c.i;
+    float const* p = pressures_cur(a, *S);
+    float const pi = p[i];
+    float const beta = iisph_beta<K, CH>(P, S->dt, pi, a.sdp[i], a.nf_cnt[i], a.ns_cnt[i],
+                                         ArenaIisph{a, p}, ArenaList{a, i},
+                                         ArenaBoundary{a, i, P.rho0});
+    bool counted;
+    pressures_next(a, *S)[i] =
+      iisph_new_pressure(P, S, pi, a.aii[i], a.rho_star[i], beta, err, counted);
+    return counted;
+}
+
+// compute_densities, integrate_velocities_in_place, zero pressures.
+template <bool K>
+__device__ __forceinline__ void ap_density_at(Arena const& a, Ctx const& c) {
+    SceneParams const& P = a.sp[c.s];
+    a.rho[c.i] = density_of<K>(a, P, c.i);
+    a.v[c.i] = integrate_external(a, P, c.i, a.v[c.i], a.ss[c.s].dt);
+    a.pbuf0[c.i] = 0.0f;
+    a.qdens[c.i] = 0.0f;
+}
+
+template <bool K>
+__device__ __forceinline__ void ap_diag_at(Arena const& a, Ctx const& c, int pseudo) {
+    SceneParams const& P = a.sp[c.s];
+    uint32_t const i = c.i;
+    float aii, star;
+    ap_diag<K>(P, a.ss[c.s].dt, a.rho[i], a.v[i], a.nf_cnt[i], a.ns_cnt[i], pseudo,
+               ArenaSource<float2>{a.v}, ArenaList{a, i}, ArenaBoundary{a, i, P.rho0}, aii, star);
+    a.aii[i] = aii;
+    a.rho_star[i] = star;
+}
+
+template <bool K>
+__device__ __forceinline__ bool ap_iterate_at(Arena const& a, Ctx const& c, int pseudo,
+                                              float& err) {
+    SceneParams const& P = a.sp[c.s];
+    uint32_t const i = c.i;
+    bool counted;
+    float const p = ap_iterate<K>(P, a.ss[c.s].dt, a.nf_cnt[i], a.ns_cnt[i], pseudo, a.aii[i],
+                                  a.rho_star[i], a.pbuf0[i], a.acc[i], ArenaSource<float2>{a.acc},
+                                  ArenaList{a, i}, ArenaBoundary{a, i, P.rho0}, err, counted);
+    a.pbuf0[i] = p;
+    a.qdens[i] = p_over_rho2(p, a.rho[i]);
+    return counted;
+}
+
+template <bool K>
+__device__ __forceinline__ void ap_finish_at(Arena const& a, Ctx const& c, int pseudo) {
+    SceneParams const& P = a.sp[c.s];
+    float2 const acc = pressure_accel_at<K>(a, P, c.i);
+    a.acc[c.i] = acc;
+    ap_integrate(a, P, c.i, a.ss[c.s].dt, a.v[c.i], acc, pseudo);
+}
+
+template <bool K>
+__device__ __forceinline__ float pc_density_at(Arena const& a, SceneParams const& P, uint32_t i) {
+    return pc_density_of<K>(a, P, i, a.xstar[i], a.nf_cnt[i], a.ns_cnt[i],
+                            ArenaSource<float2>{a.xstar}, ArenaList{a, i});
+}
+
+struct ArenaPc {
+    Arena const& a;
+    __device__ __forceinline__ PcNeighbor at(uint32_t j) const {
+        return PcNeighbor{a.xstar[j], a.vstar[j], a.rho[j], a.qdens[j]};
+    }
+};
+
+template <bool K>
+__device__ __forceinline__ void pc_forces_at(Arena const& a, Ctx const& c) {
+    uint32_t const i = c.i;
+    ArenaPc const src{a};
+    a.fp[i] = pc_forces<K>(a, a.sp[c.s], i, src.at(i), a.pbuf0[i], a.nf_cnt[i], a.ns_cnt[i], src,
+                           ArenaList{a, i});
+}
 
 // Each warp of a gather kernel may first ask L2 for its fluid list rows
 // (lane k: slot k's 128 index bytes and 256 gradient bytes), so that the
@@ -452,319 +592,7 @@ __device__ __forceinline__ void prefetch_fluid_lists(Arena const& a, int count) 
     }
 }
 
-// Neighbour values the IISPH beta sum gathers.
-struct IisphNeighbor {
-    float rho, p;
-    float2 sdp, dii;
-};
-
-template <int CH, class Gather, class Fold>
-__device__ __forceinline__ void fold_fluid_list(Arena const& a, uint32_t i, int c, Gather gather,
-                                                Fold fold) {
-    size_t const stride = a.stride;
-    using T = decltype(gather(0u));
-    for (int k0 = 0; k0 < c; k0 += CH) {
-        uint32_t jj[CH];
-        float2 gw[CH];
-        T val[CH];
-#pragma unroll
-        for (int u = 0; u < CH; ++u) {
-            if (k0 + u < c) {
-                size_t const e = static_cast<size_t>(k0 + u) * stride + i;
-                jj[u] = a.nf_idx[e];
-                gw[u] = a.nf_gw[e];
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < CH; ++u) {
-            if (k0 + u < c) val[u] = gather(jj[u]);
-        }
-#pragma unroll
-        for (int u = 0; u < CH; ++u) {
-            if (k0 + u < c) fold(val[u], gw[u]);
-        }
-    }
-}
-
-// compute_densities (emerald/sph_common/density.cpp:10-73); with K each
-// sum is Kahan-compensated.
-template <bool K = false>
-__device__ __forceinline__ float density_of(Arena const& a, SceneParams const& P, uint32_t i) {
-    size_t const stride = a.stride;
-    float const rho0 = P.rho0;
-    float const fmass = rho0 * P.fluid_volume;
-    SumF<K> d(P.fluid_volume * rho0 * P.w0);
-    int const c = a.nf_cnt[i];
-    #pragma unroll 4
-
-    for (int k = 0; k < c; ++k) d.add(a.nf_w[k * stride + i] * fmass);
-    float out = d.get();
-    int const cs = a.ns_cnt[i];
-    if (cs) {
-        SumF<K> db;
-        #pragma unroll 4
-
-        for (int k = 0; k < cs; ++k) {
-            size_t const e = k * stride + i;
-            db.add(a.ns_w[e] * (rho0 * a.vols[a.ns_idx[e]]));
-        }
-        out += db.get();
-    }
-    return out;
-}
-
-// compute_divergences (emerald/sph_common/divergence.cpp:5-74).
-// With K, the fluid and boundary terms go into one Kahan-compensated sum.
-template <bool K = false, int CH = kDivergenceChunk>
-__device__ __forceinline__ float divergence_of(Arena const& a, SceneParams const& P, uint32_t i) {
-    size_t const stride = a.stride;
-    float const rho0 = P.rho0;
-    float const fmass = rho0 * P.fluid_volume;
-    float2 const vi = a.v[i];
-    int const c = a.nf_cnt[i];
-    if (K) {
-        KahanF acc{0.0f, 0.0f};
-        for (int k = 0; k < c; ++k) {
-            size_t const e = k * stride + i;
-            kahan_add(acc, fmass * dot2(sub2(vi, a.v[a.nf_idx[e]]), a.nf_gw[e]));
-        }
-        int const cs = a.ns_cnt[i];
-        for (int k = 0; k < cs; ++k) {
-            size_t const e = k * stride + i;
-            uint32_t const j = a.ns_idx[e];
-            kahan_add(acc, (rho0 * a.vols[j]) * dot2(sub2(vi, a.vs[j]), a.ns_gw[e]));
-        }
-        return acc.s;
-    }
-    float d = 0.0f;
-    fold_fluid_list<CH>(
-      a, i, c, [&](uint32_t j) { return a.v[j]; },
-      [&](float2 vj, float2 g) { d += fmass * dot2(sub2(vi, vj), g); });
-    int const cs = a.ns_cnt[i];
-    if (cs) {
-        float db = 0.0f;
-        #pragma unroll 4
-
-        for (int k = 0; k < cs; ++k) {
-            size_t const e = k * stride + i;
-            uint32_t const j = a.ns_idx[e];
-            db += (rho0 * a.vols[j]) * dot2(sub2(vi, a.vs[j]), a.ns_gw[e]);
-        }
-        d += db;
-    }
-    return d;
-}
-
-// apply_pressures_in_place (emerald/sph_common/pressure.cpp:9-80) for one
-// particle, with q = safe_divide(p, rho^2) precomputed per particle. With K,
-// each sum is Kahan-compensated.
-template <bool K = false, int CH = kPressureChunk>
-__device__ __forceinline__ float2 apply_pressure_of(Arena const& a, SceneParams const& P, uint32_t i,
-                                                    float2 v, float const* q, float dt) {
-    size_t const stride = a.stride;
-    float const rho0 = P.rho0;
-    float const neg_fmass = -(rho0 * P.fluid_volume);
-    float const qi = q[i];
-    int const c = a.nf_cnt[i];
-    if (K) {
-        if (c) {
-            KahanF2 acc{{0.0f, 0.0f}, {0.0f, 0.0f}};
-            for (int k = 0; k < c; ++k) {
-                size_t const e = k * stride + i;
-                kahan_add(acc, scl2(neg_fmass * (qi + q[a.nf_idx[e]]), a.nf_gw[e]));
-            }
-            v = add2(v, scl2(dt, mk2(acc.x.s, acc.y.s)));
-        }
-        int const cs = a.ns_cnt[i];
-        if (cs) {
-            KahanF2 acc{{0.0f, 0.0f}, {0.0f, 0.0f}};
-            for (int k = 0; k < cs; ++k) {
-                size_t const e = k * stride + i;
-                kahan_add(acc, scl2(-(rho0 * a.vols[a.ns_idx[e]]) * qi, a.ns_gw[e]));
-            }
-            v = add2(v, scl2(dt, mk2(acc.x.s, acc.y.s)));
-        }
-        return v;
-    }
-    if (c) {
-        float2 acc = mk2(0.0f, 0.0f);
-        fold_fluid_list<CH>(
-          a, i, c, [&](uint32_t j) { return q[j]; },
-          [&](float qj, float2 g) { acc = add2(acc, scl2(neg_fmass * (qi + qj), g)); });
-        v = add2(v, scl2(dt, acc));
-    }
-    int const cs = a.ns_cnt[i];
-    if (cs) {
-        float2 acc = mk2(0.0f, 0.0f);
-        #pragma unroll 4
-
-        for (int k = 0; k < cs; ++k) {
-            size_t const e = k * stride + i;
-            acc = add2(acc, scl2(-(rho0 * a.vols[a.ns_idx[e]]) * qi, a.ns_gw[e]));
-        }
-        v = add2(v, scl2(dt, acc));
-    }
-    return v;
-}
-
-// compute_pressure_accelerations (emerald/sph_common/pressure.cpp:83-178);
-// with K each sum is Kahan-compensated.
-template <bool K = false>
-__device__ __forceinline__ float2 pressure_accel_of(Arena const& a, SceneParams const& P, uint32_t i,
-                                                    float const* q) {
-    size_t const stride = a.stride;
-    float const rho0 = P.rho0;
-    float const neg_fmass = -(rho0 * P.fluid_volume);
-    float const qi = q[i];
-    float2 out = mk2(0.0f, 0.0f);
-    int const c = a.nf_cnt[i];
-    if (c) {
-        SumF2<K> acc;
-        #pragma unroll 4
-
-        for (int k = 0; k < c; ++k) {
-            size_t const e = k * stride + i;
-            acc.add(scl2(neg_fmass * (qi + q[a.nf_idx[e]]), a.nf_gw[e]));
-        }
-        out = acc.get();
-    }
-    int const cs = a.ns_cnt[i];
-    if (cs) {
-        SumF2<K> acc;
-        #pragma unroll 4
-
-        for (int k = 0; k < cs; ++k) {
-            size_t const e = k * stride + i;
-            acc.add(scl2(-(rho0 * a.vols[a.ns_idx[e]]) * qi, a.ns_gw[e]));
-        }
-        out = add2(out, acc.get());
-    }
-    return out;
-}
-
-// compute_all_external_forces (emerald/sph2d_box/forces.cpp:11-33) for one
-// particle: the force starts at zero and takes the scene's terms in order,
-// each with the reference function's own arithmetic; a scene driven by a
-// host callback reads the callback's forces instead. v is the velocity at
-// the point of the sub-step where the solver computes the forces.
-__device__ __forceinline__ float2 external_force(Arena const& a, SceneParams const& P,
-                                                 uint32_t i, float2 v) {
-    if (P.force_array) return a.ext_f[i];
-    float2 f = mk2(0.0f, 0.0f);
-    for (int k = 0; k < P.force_count; ++k) {
-        ForceTerm const t = P.force_terms[k];
-        if (t.kind == kForceGravity) {
-            // accumulate_gravity_forces (forces.cpp:63-71)
-            f.y -= P.mass * t.a;
-        } else if (t.kind == kForcePole) {
-            // accumulate_constant_pole_attraction_forces (forces.cpp:85-101):
-            // pull along the unit vector to the pole (Imath normalized(),
-            // zero at the pole), plus the swirl (0, 0, magnitude / 8) x
-            // (rN, 0) written out component by component.
-            float2 const r = sub2(a.x[i], mk2(t.b, t.c));
-            float const l = length2f(r);
-            float2 const rn = (l == 0.0f) ? mk2(0.0f, 0.0f) : mk2(r.x / l, r.y / l);
-            f = sub2(f, mk2(t.a * rn.x, t.a * rn.y));
-            float const tz = 0.125f * t.a;
-            float const zero = 0.0f;
-            f = add2(f, mk2(zero * zero - tz * rn.y, tz * rn.x - zero * zero));
-        } else if (t.kind == kForceDrag) {
-            // accumulate_simple_drag_forces (forces.cpp:104-111)
-            float const m = -t.a * t.b;
-            f = add2(f, mk2(m * v.x, m * v.y));
-        }
-    }
-    return f;
-}
-
-// integrate_velocities_in_place (dynamics.cpp:24-37) with the scene's
-// external forces.
-__device__ __forceinline__ float2 integrate_external(Arena const& a, SceneParams const& P,
-                                                     uint32_t i, float2 v, float dt) {
-    float2 const f = external_force(a, P, i, v);
-    float const denom = P.rho0 * P.fluid_volume;
-    float2 const numer = scl2(dt, f);
-    if (safe_v(numer, denom)) v = add2(v, div2(numer, denom));
-    return v;
-}
-
 // ------------------------------------------------------------------- DFSPH
-
-// compute_densities + dfsph_p_compute_shared_coeffs (dfsph_p_ops.cpp:19-72),
-// the per-frame kappa reset, and the p/rho^2 caches of both warm starts.
-// With K, the density and the two alpha sums are Kahan-compensated.
-template <bool K>
-__device__ __forceinline__ void dfsph_density_alpha(Arena const& a, Ctx const& c) {
-    SceneParams const& P = a.sp[c.s];
-    uint32_t const i = c.i;
-    size_t const stride = a.stride;
-    float const rho0 = P.rho0;
-    float const fvol = P.fluid_volume;
-    float d = fvol * rho0 * P.w0;
-    float2 sum = mk2(0.0f, 0.0f);
-    float sdot = 0.0f;
-    KahanF kd{d, 0.0f}, ksdot{0.0f, 0.0f};
-    KahanF2 ksum{{0.0f, 0.0f}, {0.0f, 0.0f}};
-    int const cf = a.nf_cnt[i];
-    float const fmass = rho0 * fvol;
-    float const fmass_a = fvol * rho0;
-    #pragma unroll 4
-
-    for (int k = 0; k < cf; ++k) {
-        size_t const e = k * stride + i;
-        float2 const m = scl2(fmass_a, a.nf_gw[e]);
-        if (K) {
-            kahan_add(kd, a.nf_w[e] * fmass);
-            kahan_add(ksum, m);
-            kahan_add(ksdot, dot2(m, m));
-        } else {
-            d += a.nf_w[e] * fmass;
-            sum = add2(sum, m);
-            sdot += dot2(m, m);
-        }
-    }
-    int const cs = a.ns_cnt[i];
-    if (cs) {
-        float db = 0.0f;
-        #pragma unroll 4
-
-        for (int k = 0; k < cs; ++k) {
-            size_t const e = k * stride + i;
-            float const vs = a.vols[a.ns_idx[e]];
-            if (K) {
-                kahan_add(kd, a.ns_w[e] * (rho0 * vs));
-                kahan_add(ksum, scl2(vs * rho0, a.ns_gw[e]));
-            } else {
-                db += a.ns_w[e] * (rho0 * vs);
-                sum = add2(sum, scl2(vs * rho0, a.ns_gw[e]));
-            }
-        }
-        if (!K) d += db;
-    }
-    if (K) {
-        d = kd.s;
-        sum = mk2(ksum.x.s, ksum.y.s);
-        sdot = ksdot.s;
-    }
-    a.rho[i] = d;
-    float alpha = 0.0f;
-    if (cf + cs) {
-        float const numer = sqrf(d);
-        float const denom = dot2(sum, sum) + sdot;
-        alpha = safe_f(numer, denom) ? numer / denom : 0.0f;
-    }
-    a.alpha[i] = alpha;
-    float kd0 = a.kdiv[i];
-    float kn = a.kdens[i];
-    if (a.ss[c.s].new_frame) {
-        kd0 = 0.0f;
-        kn = 0.0f;
-        a.kdiv[i] = kd0;
-        a.kdens[i] = kn;
-    }
-    a.qdiv[i] = p_over_rho2(kd0, d);
-    a.qdens[i] = p_over_rho2(kn, d);
-}
 
 // MODE 0 launches carry only the reference arithmetic; MODE 1 launches
 // (when some resident scene is in compensated mode) choose per scene.
@@ -773,9 +601,9 @@ __global__ void k_dfsph_density_alpha(Arena a) {
     Ctx c;
     if (!enter(a, false, c) || !c.live) return;
     if (MODE && a.sp[c.s].precision) {
-        dfsph_density_alpha<true>(a, c);
+        dfsph_density_alpha_at<true>(a, c);
     } else {
-        dfsph_density_alpha<false>(a, c);
+        dfsph_density_alpha_at<false>(a, c);
     }
 }
 
@@ -793,8 +621,8 @@ __global__ void k_apply_pressures(Arena a, int which_q, int external, int skip_d
     float2 v = a.v[c.i];
     if (external) v = integrate_external(a, P, c.i, v, dt);
     float const* q = which_q ? a.qdens : a.qdiv;
-    a.v[c.i] = (MODE && P.precision) ? apply_pressure_of<true, CH>(a, P, c.i, v, q, dt)
-                                     : apply_pressure_of<false, CH>(a, P, c.i, v, q, dt);
+    a.v[c.i] = (MODE && P.precision) ? apply_pressure_at<true, CH>(a, P, c.i, v, q, dt)
+                                     : apply_pressure_at<false, CH>(a, P, c.i, v, q, dt);
 }
 
 // compute_divergences + dfsph_p_compute_divergence_pseudo_pressures
@@ -810,17 +638,9 @@ __global__ void k_dfsph_divergence(Arena a) {
     if (PF) prefetch_fluid_lists(a, c.live ? int(a.nf_cnt[c.i]) : 0);
     if (c.live) {
         uint32_t const i = c.i;
-        float const d = (MODE && P.precision) ? divergence_of<true, CH>(a, P, i)
-                                              : divergence_of<false, CH>(a, P, i);
-        a.rho_star[i] = d;
-        float kappa = 0.0f;
-        if (!(d <= 0.0f)) {
-            float const numer = d * a.alpha[i];
-            kappa = safe_f(numer, dt) ? numer / dt : 0.0f;
-        }
-        a.kdiv[i] = kappa;
-        a.qdiv[i] = p_over_rho2(kappa, a.rho[i]);
-        err = d <= 0.0f ? 0.0f : (dt * d / P.rho0);
+        float const d = (MODE && P.precision) ? divergence_at<true, CH>(a, P, i)
+                                              : divergence_at<false, CH>(a, P, i);
+        err = dfsph_divergence_step_at(a, P, i, dt, d);
     }
     accumulate_error(S, static_cast<unsigned long long>(static_cast<long long>(err * 1000.0f)),
                      err, c.live, true);
@@ -836,26 +656,14 @@ __global__ void k_dfsph_density(Arena a) {
     SceneParams const& P = a.sp[c.s];
     SceneState* S = &a.ss[c.s];
     float const dt = S->dt;
-    float const rho0 = P.rho0;
     float err = 0.0f;
     if (PF) prefetch_fluid_lists(a, c.live ? int(a.nf_cnt[c.i]) : 0);
     if (c.live) {
         uint32_t const i = c.i;
         float const rho = a.rho[i];
-        float const div = (MODE && P.precision) ? divergence_of<true, CH>(a, P, i)
-                                                : divergence_of<false, CH>(a, P, i);
-        float const star = max_0x(rho + (dt * div));
-        a.rho_star[i] = star;
-        float const delta = star - rho0;
-        float kappa = 0.0f;
-        if (!(delta <= 0.0f)) {
-            float const numer = delta * a.alpha[i];
-            float const dd = sqrf(dt);
-            kappa = safe_f(numer, dd) ? numer / dd : 0.0f;
-        }
-        a.kdens[i] = kappa;
-        a.qdens[i] = p_over_rho2(kappa, rho);
-        err = delta <= 0.0f ? 0.0f : (delta / rho0);
+        float const div = (MODE && P.precision) ? divergence_at<true, CH>(a, P, i)
+                                                : divergence_at<false, CH>(a, P, i);
+        err = dfsph_density_step_at(a, P, i, dt, rho, div);
     }
     accumulate_error(S, static_cast<unsigned long long>(static_cast<long long>(err * 1000.0f)),
                      err, c.live, true);
@@ -1099,9 +907,9 @@ __global__ void __launch_bounds__(256) k_dfsph_density_alpha_pw(Arena a, uint32_
           if (!live) return;
           Ctx const c{s, i, true};
           if (MODE && a.sp[s].precision) {
-              dfsph_density_alpha<true>(a, c);
+              dfsph_density_alpha_at<true>(a, c);
           } else {
-              dfsph_density_alpha<false>(a, c);
+              dfsph_density_alpha_at<false>(a, c);
           }
       });
 }
@@ -1123,8 +931,8 @@ __global__ void __launch_bounds__(256) k_apply_pressures_pw(Arena a, uint32_t wt
           float const dt = a.ss[s].dt;
           float2 v = a.v[i];
           if (external) v = integrate_external(a, P, i, v, dt);
-          a.v[i] = (MODE && P.precision) ? apply_pressure_of<true, CH>(a, P, i, v, q, dt)
-                                         : apply_pressure_of<false, CH>(a, P, i, v, q, dt);
+          a.v[i] = (MODE && P.precision) ? apply_pressure_at<true, CH>(a, P, i, v, q, dt)
+                                         : apply_pressure_at<false, CH>(a, P, i, v, q, dt);
       });
     fused_exit_test(a, lc, false);
 }
@@ -1143,17 +951,9 @@ __global__ void __launch_bounds__(256) k_dfsph_divergence_pw(Arena a, uint32_t w
           float const dt = a.ss[s].dt;
           float err = 0.0f;
           if (live) {
-              float const d = (MODE && P.precision) ? divergence_of<true, CH>(a, P, i)
-                                                    : divergence_of<false, CH>(a, P, i);
-              a.rho_star[i] = d;
-              float kappa = 0.0f;
-              if (!(d <= 0.0f)) {
-                  float const numer = d * a.alpha[i];
-                  kappa = safe_f(numer, dt) ? numer / dt : 0.0f;
-              }
-              a.kdiv[i] = kappa;
-              a.qdiv[i] = p_over_rho2(kappa, a.rho[i]);
-              err = d <= 0.0f ? 0.0f : (dt * d / P.rho0);
+              float const d = (MODE && P.precision) ? divergence_at<true, CH>(a, P, i)
+                                                    : divergence_at<false, CH>(a, P, i);
+              err = dfsph_divergence_step_at(a, P, i, dt, d);
           }
           add_err(a, e, s,
                   static_cast<unsigned long long>(static_cast<long long>(err * 1000.0f)), err,
@@ -1174,56 +974,18 @@ __global__ void __launch_bounds__(256, LIST ? 3 : 1) k_dfsph_density_pw(Arena a,
       [&](int32_t s, uint32_t i, bool live) {
           SceneParams const& P = a.sp[s];
           float const dt = a.ss[s].dt;
-          float const rho0 = P.rho0;
           float err = 0.0f;
           if (live) {
               float const rho = a.rho[i];
-              float const div = (MODE && P.precision) ? divergence_of<true, CH>(a, P, i)
-                                                      : divergence_of<false, CH>(a, P, i);
-              float const star = max_0x(rho + (dt * div));
-              a.rho_star[i] = star;
-              float const delta = star - rho0;
-              float kappa = 0.0f;
-              if (!(delta <= 0.0f)) {
-                  float const numer = delta * a.alpha[i];
-                  float const dd = sqrf(dt);
-                  kappa = safe_f(numer, dd) ? numer / dd : 0.0f;
-              }
-              a.kdens[i] = kappa;
-              a.qdens[i] = p_over_rho2(kappa, rho);
-              err = delta <= 0.0f ? 0.0f : (delta / rho0);
+              float const div = (MODE && P.precision) ? divergence_at<true, CH>(a, P, i)
+                                                      : divergence_at<false, CH>(a, P, i);
+              err = dfsph_density_step_at(a, P, i, dt, rho, div);
           }
           add_err(a, e, s,
                   static_cast<unsigned long long>(static_cast<long long>(err * 1000.0f)), err,
                   live, true);
       });
     flush_err_block(a, e);
-}
-
-// integrate_positions_in_place (dynamics.cpp:46-51). Compensated mode
-// accumulates the positions in double and stores their float rounding.
-// x_i += dt * v (+ shift): the reference's FP32 update, or for a
-// compensated scene the FP64 accumulator (the positions the neighbour search
-// takes its vectors from) rounded once into x_i. Every method's position
-// update goes through here, so a compensated scene's FP64 positions stay
-// current whichever method advances it.
-__device__ __forceinline__ void advance_position(Arena const& a, SceneParams const& P,
-                                                 uint32_t i, float dt, float2 v,
-                                                 float2 shift = {0.0f, 0.0f}, bool shifted = false) {
-    if (P.precision) {
-        double2 x = a.x64[i];
-        x.x += static_cast<double>(dt) * static_cast<double>(v.x);
-        x.y += static_cast<double>(dt) * static_cast<double>(v.y);
-        if (shifted) {
-            x.x += static_cast<double>(shift.x);
-            x.y += static_cast<double>(shift.y);
-        }
-        a.x64[i] = x;
-        a.x[i] = mk2(static_cast<float>(x.x), static_cast<float>(x.y));
-        return;
-    }
-    float2 const x = add2(a.x[i], scl2(dt, v));
-    a.x[i] = shifted ? add2(x, shift) : x;
 }
 
 template <int MODE>
@@ -1240,112 +1002,15 @@ __global__ void k_integrate_positions(Arena a) {
 
 // -------------------------------------------------------------------- IISPH
 
-// compute_densities, integrate_velocities_in_place and iisph_compute_diis
-// (iisph_ops.cpp:20-90), plus the zero initial pressures (iisph.cpp:76).
-// MODE 1 launches (some resident scene in compensated mode) Kahan-compensate
-// the sums of compensated scenes, here and in the kernels below.
-template <bool K>
-__device__ __forceinline__ void iisph_density_dii(Arena const& a, Ctx const& c) {
-    SceneParams const& P = a.sp[c.s];
-    uint32_t const i = c.i;
-    size_t const stride = a.stride;
-    float const dt = a.ss[c.s].dt;
-    float const rho0 = P.rho0;
-    float const d = density_of<K>(a, P, i);
-    a.rho[i] = d;
-    a.v[i] = integrate_external(a, P, i, a.v[i], dt);
-    float const neg_dt2 = -sqrf(dt);
-    float const denom = sqrf(d);
-    float2 dii = mk2(0.0f, 0.0f);
-    int const cf = a.nf_cnt[i];
-    if (cf) {
-        float const fmass = rho0 * P.fluid_volume;
-        SumF2<K> g;
-        #pragma unroll 4
-
-        for (int k = 0; k < cf; ++k) g.add(scl2(fmass, a.nf_gw[k * stride + i]));
-        float2 const numer = scl2(neg_dt2, g.get());
-        dii = safe_v(numer, denom) ? div2(numer, denom) : mk2(0.0f, 0.0f);
-    }
-    int const cs = a.ns_cnt[i];
-    if (cs) {
-        SumF2<K> g;
-        #pragma unroll 4
-
-        for (int k = 0; k < cs; ++k) {
-            size_t const e = k * stride + i;
-            g.add(scl2(rho0 * a.vols[a.ns_idx[e]], a.ns_gw[e]));
-        }
-        float2 const numer = scl2(neg_dt2, g.get());
-        dii = add2(dii, safe_v(numer, denom) ? div2(numer, denom) : mk2(0.0f, 0.0f));
-    }
-    a.dii[i] = dii;
-    a.pbuf0[i] = 0.0f;
-}
-
 template <int MODE>
 __global__ void k_iisph_density_dii(Arena a) {
     Ctx c;
     if (!enter(a, false, c) || !c.live) return;
     if (MODE && a.sp[c.s].precision) {
-        iisph_density_dii<true>(a, c);
+        iisph_density_dii_at<true>(a, c);
     } else {
-        iisph_density_dii<false>(a, c);
+        iisph_density_dii_at<false>(a, c);
     }
-}
-
-// iisph_compute_aiis_and_density_stars (iisph_ops.cpp:92-200).
-template <bool K>
-__device__ __forceinline__ void iisph_aii(Arena const& a, Ctx const& c) {
-    SceneParams const& P = a.sp[c.s];
-    uint32_t const i = c.i;
-    size_t const stride = a.stride;
-    float const dt = a.ss[c.s].dt;
-    float const rho0 = P.rho0;
-    float2 const dii = a.dii[i];
-    float2 const vi = a.v[i];
-    float const neg_dt2 = -sqrf(dt);
-    float aii = 0.0f;
-    float star = a.rho[i];
-    int const cf = a.nf_cnt[i];
-    if (cf) {
-        float const mass = P.fluid_volume * rho0;
-        SumF<K> af, dd;
-        #pragma unroll 4
-
-        for (int k = 0; k < cf; ++k) {
-            size_t const e = k * stride + i;
-            uint32_t const j = a.nf_idx[e];
-            float2 const gw = a.nf_gw[e];
-            float2 const numer = scl2(neg_dt2 * mass, gw);
-            float const denom = sqrf(a.rho[j]);
-            if (safe_v(numer, denom)) {
-                float2 const dji = neg2(div2(numer, denom));
-                af.add(mass * dot2(sub2(dii, dji), gw));
-            }
-            dd.add(dt * mass * dot2(sub2(vi, a.v[j]), gw));
-        }
-        aii = af.get();
-        star = a.rho[i] + dd.get();
-    }
-    int const cs = a.ns_cnt[i];
-    if (cs) {
-        SumF<K> ab, dd;
-        #pragma unroll 4
-
-        for (int k = 0; k < cs; ++k) {
-            size_t const e = k * stride + i;
-            uint32_t const j = a.ns_idx[e];
-            float2 const gw = a.ns_gw[e];
-            float const mass = a.vols[j] * rho0;
-            ab.add(mass * dot2(dii, gw));
-            dd.add(dt * mass * dot2(sub2(vi, a.vs[j]), gw));
-        }
-        aii += ab.get();
-        star += dd.get();
-    }
-    a.aii[i] = aii;
-    a.rho_star[i] = star;
 }
 
 template <int MODE>
@@ -1353,34 +1018,10 @@ __global__ void k_iisph_aii(Arena a) {
     Ctx c;
     if (!enter(a, false, c) || !c.live) return;
     if (MODE && a.sp[c.s].precision) {
-        iisph_aii<true>(a, c);
+        iisph_aii_at<true>(a, c);
     } else {
-        iisph_aii<false>(a, c);
+        iisph_aii_at<false>(a, c);
     }
-}
-
-// iisph_compute_sum_dij_pjs (iisph_ops.cpp:202-235).
-template <bool K, int CH>
-__device__ __forceinline__ void iisph_sum_dij(Arena const& a, Ctx const& c) {
-    SceneParams const& P = a.sp[c.s];
-    SceneState const& S = a.ss[c.s];
-    uint32_t const i = c.i;
-    size_t const stride = a.stride;
-    float const dt = S.dt;
-    float const* p = pressures_cur(a, S);
-    float const mass = P.fluid_volume * P.rho0;
-    float const neg_dt2 = -sqrf(dt);
-    SumF2<K> sum;
-    int const cf = a.nf_cnt[i];
-    (void)stride;
-    fold_fluid_list<CH>(
-      a, i, cf, [&](uint32_t j) { return mk2(p[j], a.rho[j]); },
-      [&](float2 prho, float2 g) {
-          float2 const numer = scl2(neg_dt2 * mass * prho.x, g);
-          float const denom = sqrf(prho.y);
-          if (safe_v(numer, denom)) sum.add(div2(numer, denom));
-      });
-    a.sdp[i] = sum.get();
 }
 
 template <int MODE, int CH, int PF>
@@ -1390,75 +1031,10 @@ __global__ void k_iisph_sum_dij(Arena a) {
     if (PF) prefetch_fluid_lists(a, c.live ? int(a.nf_cnt[c.i]) : 0);
     if (!c.live) return;
     if (MODE && a.sp[c.s].precision) {
-        iisph_sum_dij<true, CH>(a, c);
+        iisph_sum_dij_at<true, CH>(a, c);
     } else {
-        iisph_sum_dij<false, CH>(a, c);
+        iisph_sum_dij_at<false, CH>(a, c);
     }
-}
-
-// iisph_compute_betas (iisph_ops.cpp:237-330) followed by
-// iisph_compute_new_pressures for the same particle (iisph_ops.cpp:332-425).
-// Returns whether the particle's error counts (a_ii != 0).
-template <bool K, int CH>
-__device__ __forceinline__ bool iisph_beta_pressure(Arena const& a, Ctx const& c, SceneState* S,
-                                                    float& err) {
-    SceneParams const& P = a.sp[c.s];
-    bool counted = false;
-    {
-        uint32_t const i = c.i;
-        size_t const stride = a.stride;
-        float const dt = S->dt;
-        float const rho0 = P.rho0;
-        float const* p = pressures_cur(a, *S);
-        float* pn = pressures_next(a, *S);
-        float const pi = p[i];
-        float2 const si = a.sdp[i];
-        float const neg_dt2 = -sqrf(dt);
-        float beta = 0.0f;
-        int const cf = a.nf_cnt[i];
-        if (cf) {
-            float const mass = rho0 * P.fluid_volume;
-            SumF<K> bf;
-            fold_fluid_list<CH>(
-              a, i, cf,
-              [&](uint32_t j) { return IisphNeighbor{a.rho[j], p[j], a.sdp[j], a.dii[j]}; },
-              [&](IisphNeighbor const& nb, float2 gw) {
-                  float2 const numer = scl2(neg_dt2 * mass, gw);
-                  float const denom = sqrf(nb.rho);
-                  float2 const dij = safe_v(numer, denom) ? div2(numer, denom) : mk2(0.0f, 0.0f);
-                  float2 const dji = neg2(dij);
-                  float2 const skni = sub2(nb.sdp, scl2(pi, dji));
-                  float2 const t = sub2(sub2(si, scl2(nb.p, nb.dii)), skni);
-                  bf.add(mass * dot2(t, gw));
-              });
-            beta = bf.get();
-        }
-        int const cs = a.ns_cnt[i];
-        if (cs) {
-            SumF<K> bb;
-            #pragma unroll 4
-
-            for (int k = 0; k < cs; ++k) {
-                size_t const e = k * stride + i;
-                bb.add((rho0 * a.vols[a.ns_idx[e]]) * dot2(si, a.ns_gw[e]));
-            }
-            beta += bb.get();
-        }
-        float const alpha = a.aii[i];
-        float out = pi;
-        if (alpha != 0.0f) {
-            float const numer = rho0 - a.rho_star[i] - beta;
-            if (safe_f(numer, alpha)) {
-                err = max_0x(-(numer - (alpha * pi)) / rho0);
-                counted = true;
-                out = max_0x(mix1(pi, numer / alpha, P.iisph_omega));
-            } else {
-                atomicOr(&S->error, kErrNonFinite);
-            }
-        }
-        pn[i] = out;
-    }
-    return counted;
 }
 
 template <int MODE, int CH, int PF>
@@ -1470,8 +1046,8 @@ __global__ void k_iisph_beta_pressure(Arena a) {
     bool counted = false;
     if (PF) prefetch_fluid_lists(a, c.live ? int(a.nf_cnt[c.i]) : 0);
     if (c.live) {
-        counted = (MODE && a.sp[c.s].precision) ? iisph_beta_pressure<true, CH>(a, c, S, err)
-                                                : iisph_beta_pressure<false, CH>(a, c, S, err);
+        counted = (MODE && a.sp[c.s].precision) ? iisph_beta_pressure_at<true, CH>(a, c, S, err)
+                                                : iisph_beta_pressure_at<false, CH>(a, c, S, err);
     }
     accumulate_error(S, counted ? static_cast<unsigned long long>(err * 1000.0f) : 0ull, err,
                      c.live && counted);
@@ -1490,9 +1066,9 @@ __global__ void __launch_bounds__(256) k_iisph_sum_dij_pw(Arena a, uint32_t wtil
           if (!live) return;
           Ctx const c{s, i, true};
           if (MODE && a.sp[s].precision) {
-              iisph_sum_dij<true, CH>(a, c);
+              iisph_sum_dij_at<true, CH>(a, c);
           } else {
-              iisph_sum_dij<false, CH>(a, c);
+              iisph_sum_dij_at<false, CH>(a, c);
           }
       });
 }
@@ -1513,8 +1089,8 @@ __global__ void __launch_bounds__(256, LIST ? 3 : 1) k_iisph_beta_pressure_pw(Ar
           bool counted = false;
           if (live) {
               Ctx const c{s, i, true};
-              counted = (MODE && a.sp[s].precision) ? iisph_beta_pressure<true, CH>(a, c, S, err)
-                                                    : iisph_beta_pressure<false, CH>(a, c, S, err);
+              counted = (MODE && a.sp[s].precision) ? iisph_beta_pressure_at<true, CH>(a, c, S, err)
+                                                    : iisph_beta_pressure_at<false, CH>(a, c, S, err);
           }
           add_err(a, e, s, counted ? static_cast<unsigned long long>(err * 1000.0f) : 0ull, err,
                   live && counted, false);
@@ -1539,8 +1115,8 @@ __global__ void k_apply_integrate(Arena a) {
     if (!enter(a, false, c) || !c.live) return;
     SceneParams const& P = a.sp[c.s];
     float const dt = a.ss[c.s].dt;
-    float2 const v = (MODE && P.precision) ? apply_pressure_of<true>(a, P, c.i, a.v[c.i], a.qdens, dt)
-                                           : apply_pressure_of<false>(a, P, c.i, a.v[c.i], a.qdens, dt);
+    float2 const v = (MODE && P.precision) ? apply_pressure_at<true>(a, P, c.i, a.v[c.i], a.qdens, dt)
+                                           : apply_pressure_at<false>(a, P, c.i, a.v[c.i], a.qdens, dt);
     a.v[c.i] = v;
     advance_position(a, P, c.i, dt, v);
 }
@@ -1552,63 +1128,11 @@ template <int MODE>
 __global__ void k_ap_density(Arena a) {
     Ctx c;
     if (!enter(a, false, c) || !c.live) return;
-    SceneParams const& P = a.sp[c.s];
-    float const dt = a.ss[c.s].dt;
-    a.rho[c.i] = (MODE && P.precision) ? density_of<true>(a, P, c.i) : density_of<false>(a, P, c.i);
-    a.v[c.i] = integrate_external(a, P, c.i, a.v[c.i], dt);
-    a.pbuf0[c.i] = 0.0f;
-    a.qdens[c.i] = 0.0f;
-}
-
-// iisph_ap_density_stars_and_diagonals (iisph_ap_ops.cpp:19-103) and the
-// pseudo variant (iisph_pseudo_ap_ops.cpp:19-117).
-template <bool K>
-__device__ __forceinline__ void ap_diag(Arena const& a, Ctx const& c, int pseudo) {
-    SceneParams const& P = a.sp[c.s];
-    uint32_t const i = c.i;
-    size_t const stride = a.stride;
-    float const dt = a.ss[c.s].dt;
-    float const rho0 = P.rho0;
-    int const cf = a.nf_cnt[i];
-    int const cs = a.ns_cnt[i];
-    float const rho = a.rho[i];
-    if (!(cf + cs)) {
-        a.rho_star[i] = rho;
-        a.aii[i] = 0.0f;
-        return;
+    if (MODE && a.sp[c.s].precision) {
+        ap_density_at<true>(a, c);
+    } else {
+        ap_density_at<false>(a, c);
     }
-    float const self_mass = P.fluid_volume * rho0;
-    float2 const vi = a.v[i];
-    SumF2<K> sum_acc;
-    SumF<K> sdot_acc, div_acc;
-    float const fmass = P.fluid_volume * rho0;
-    #pragma unroll 4
-
-    for (int k = 0; k < cf; ++k) {
-        size_t const e = k * stride + i;
-        float2 const gw = a.nf_gw[e];
-        sum_acc.add(scl2(fmass, gw));
-        sdot_acc.add(fmass * dot2(gw, gw));
-        div_acc.add(fmass * dot2(sub2(vi, a.v[a.nf_idx[e]]), gw));
-    }
-    #pragma unroll 4
-
-    for (int k = 0; k < cs; ++k) {
-        size_t const e = k * stride + i;
-        uint32_t const j = a.ns_idx[e];
-        float2 const gw = a.ns_gw[e];
-        float const mass = a.vols[j] * rho0;
-        sum_acc.add(scl2(mass, gw));
-        div_acc.add(mass * dot2(sub2(vi, a.vs[j]), gw));
-    }
-    float2 const sum = sum_acc.get();
-    float const sdot = sdot_acc.get();
-    float const div = div_acc.get();
-    float const denom = sqrf(rho);
-    float const numer = pseudo ? -(dot2(sum, sum) + self_mass * sdot)
-                               : -sqrf(dt) * (dot2(sum, sum) + self_mass * sdot);
-    a.aii[i] = safe_f(numer, denom) ? numer / denom : 0.0f;
-    a.rho_star[i] = rho + dt * div;
 }
 
 template <int MODE>
@@ -1616,9 +1140,9 @@ __global__ void k_ap_diag(Arena a, int pseudo) {
     Ctx c;
     if (!enter(a, false, c) || !c.live) return;
     if (MODE && a.sp[c.s].precision) {
-        ap_diag<true>(a, c, pseudo);
+        ap_diag_at<true>(a, c, pseudo);
     } else {
-        ap_diag<false>(a, c, pseudo);
+        ap_diag_at<false>(a, c, pseudo);
     }
 }
 
@@ -1629,172 +1153,69 @@ __global__ void k_pressure_accel(Arena a) {
     Ctx c;
     if (!enter(a, true, c) || !c.live) return;
     SceneParams const& P = a.sp[c.s];
-    a.acc[c.i] = (MODE && P.precision) ? pressure_accel_of<true>(a, P, c.i, a.qdens)
-                                       : pressure_accel_of<false>(a, P, c.i, a.qdens);
-}
-
-// iisph_ap_iterate_pressures_in_place (iisph_ap_ops.cpp:105-194) and the
-// pseudo variant (iisph_pseudo_ap_ops.cpp:226-323).
-template <bool K>
-__device__ __forceinline__ float ap_neighbor_sum(Arena const& a, SceneParams const& P, uint32_t i,
-                                                 int cf, int cs) {
-    size_t const stride = a.stride;
-    float const rho0 = P.rho0;
-    SumF<K> api;
-    float2 const ai = a.acc[i];
-    float const fmass = rho0 * P.fluid_volume;
-    #pragma unroll 4
-
-    for (int k = 0; k < cf; ++k) {
-        size_t const e = k * stride + i;
-        api.add(fmass * dot2(sub2(ai, a.acc[a.nf_idx[e]]), a.nf_gw[e]));
-    }
-    #pragma unroll 4
-
-    for (int k = 0; k < cs; ++k) {
-        size_t const e = k * stride + i;
-        api.add((rho0 * a.vols[a.ns_idx[e]]) * dot2(ai, a.ns_gw[e]));
-    }
-    return api.get();
+    a.acc[c.i] = (MODE && P.precision) ? pressure_accel_at<true>(a, P, c.i)
+                                       : pressure_accel_at<false>(a, P, c.i);
 }
 
 template <int MODE>
 __global__ void k_ap_iterate(Arena a, int pseudo) {
     Ctx c;
     if (!enter(a, true, c)) return;
-    SceneParams const& P = a.sp[c.s];
     SceneState* S = &a.ss[c.s];
     float err = 0.0f;
     bool counted = false;
     if (c.live) {
-        uint32_t const i = c.i;
-        float const rho0 = P.rho0;
-        int const cf = a.nf_cnt[i];
-        int const cs = a.ns_cnt[i];
-        float const diag = a.aii[i];
-        float pnew;
-        if (!cf && !cs) {
-            pnew = 0.0f;
-        } else if (pseudo && diag == 0.0f) {
-            pnew = 0.0f;
-        } else {
-            float api = (MODE && P.precision) ? ap_neighbor_sum<true>(a, P, i, cf, cs)
-                                              : ap_neighbor_sum<false>(a, P, i, cf, cs);
-            if (!pseudo) api *= sqrf(S->dt);
-            float const source = rho0 - a.rho_star[i];
-            float const r = api - source;
-            err = max_0x(safe_f(r, rho0) ? r / rho0 : 0.0f);
-            counted = true;
-            float const old = a.pbuf0[i];
-            float const numer = P.iisph_omega * (source - api);
-            pnew = max_0x(old + (safe_f(numer, diag) ? numer / diag : 0.0f));
-        }
-        a.pbuf0[i] = pnew;
-        a.qdens[i] = p_over_rho2(pnew, a.rho[i]);
+        counted = (MODE && a.sp[c.s].precision)
+                    ? ap_iterate_at<true>(a, c, pseudo, err)
+                    : ap_iterate_at<false>(a, c, pseudo, err);
     }
     accumulate_error(S, counted ? static_cast<unsigned long long>(err * 1000.0f) : 0ull, err,
                      c.live && counted);
 }
 
-// Final pressure accelerations and the integration of iisph_ap.cpp:138-153
-// (integrate_velocities_and_positions_in_place, dynamics.cpp:53-63) or
-// iisph_pseudo_ap_integrate_velocities_and_positions_in_place
-// (iisph_pseudo_ap_ops.cpp:325-343).
 template <int MODE>
 __global__ void k_ap_finish(Arena a, int pseudo) {
     Ctx c;
     if (!enter(a, false, c) || !c.live) return;
-    SceneParams const& P = a.sp[c.s];
-    float const dt = a.ss[c.s].dt;
-    uint32_t const i = c.i;
-    float2 const acc = (MODE && P.precision) ? pressure_accel_of<true>(a, P, i, a.qdens)
-                                             : pressure_accel_of<false>(a, P, i, a.qdens);
-    a.acc[i] = acc;
-    if (!pseudo) {
-        float2 const v = add2(a.v[i], scl2(dt, acc));
-        a.v[i] = v;
-        advance_position(a, P, i, dt, v);
+    if (MODE && a.sp[c.s].precision) {
+        ap_finish_at<true>(a, c, pseudo);
     } else {
-        float2 const vstar = a.v[i];
-        advance_position(a, P, i, dt, vstar, acc, true);
-        if (safe_v(vstar, dt)) a.v[i] = add2(vstar, div2(acc, dt));
+        ap_finish_at<false>(a, c, pseudo);
     }
 }
 
 // ------------------------------------------------------------------- PCISPH
 
-// Velocity from external forces only (pcisph.cpp:54-65).
 __global__ void k_pc_init(Arena a) {
     Ctx c;
     if (!enter(a, false, c) || !c.live) return;
-    SceneParams const& P = a.sp[c.s];
-    float const dt = a.ss[c.s].dt;
-    float const mult = dt / P.mass;
-    float2 const v = a.v[c.i];
-    float2 const f = external_force(a, P, c.i, v);
-    a.vext[c.i] = add2(v, scl2(mult, f));
+    a.vext[c.i] = pc_external_velocity(a, a.sp[c.s], c.i, a.ss[c.s].dt, a.v[c.i]);
     a.pbuf0[c.i] = 0.0f;
 }
 
-// Predicted velocity and position of one predictor pass (pcisph.cpp:72-88).
+// Predicted velocity and position of one predictor pass.
 __global__ void k_pc_predict(Arena a) {
     Ctx c;
     if (!enter(a, true, c) || !c.live) return;
-    SceneParams const& P = a.sp[c.s];
     SceneState const& S = a.ss[c.s];
-    float const dt = S.dt;
-    float2 vs = a.vext[c.i];
-    if (S.iter > 0) vs = add2(vs, scl2(dt / P.mass, a.fp[c.i]));
+    float2 const vs = pc_predicted_velocity(a.sp[c.s], S.dt, S.iter, a.vext[c.i], a.fp[c.i]);
     a.vstar[c.i] = vs;
-    a.xstar[c.i] = add2(a.x[c.i], scl2(dt, vs));
-}
-
-// Densities at the predicted positions with the kernel values recomputed
-// (compute_neighbor_distances_and_vectors_to + compute_neighbor_kernels,
-// neighborhoods_from_state.cpp:103-128), pcisph_compute_densities,
-// pcisph_accumulate_density_from_solids and pcisph_update_pressures
-// (pcisph_ops.cpp:18-76), plus the max density error (common.cpp:78-85).
-template <bool K>
-__device__ __forceinline__ float pc_density_of(Arena const& a, SceneParams const& P, uint32_t i) {
-    size_t const stride = a.stride;
-    float const h = P.support;
-    float2 const pos = a.xstar[i];
-    int const cf = a.nf_cnt[i];
-    SumF<K> ws(P.w0);
-    #pragma unroll 4
-
-    for (int k = 0; k < cf; ++k) {
-        uint32_t const j = a.nf_idx[k * stride + i];
-        ws.add(kernel_w(length2f(sub2(a.xstar[j], pos)), h));
-    }
-    float d = P.mass * ws.get();
-    int const cs = a.ns_cnt[i];
-    if (cs) {
-        SumF<K> vf;
-        #pragma unroll 4
-
-        for (int k = 0; k < cs; ++k) {
-            uint32_t const j = a.ns_idx[k * stride + i];
-            vf.add(a.vols[j] * kernel_w(length2f(sub2(a.xs[j], pos)), h));
-        }
-        d += P.rho0 * vf.get();
-    }
-    return d;
+    a.xstar[c.i] = add2(a.x[c.i], scl2(S.dt, vs));
 }
 
 template <int MODE>
 __global__ void k_pc_density(Arena a) {
     Ctx c;
     if (!enter(a, true, c)) return;
-    SceneParams const& P = a.sp[c.s];
     SceneState* S = &a.ss[c.s];
     float err = 0.0f;
     if (c.live) {
         uint32_t const i = c.i;
-        float const d = (MODE && P.precision) ? pc_density_of<true>(a, P, i)
-                                              : pc_density_of<false>(a, P, i);
+        SceneParams const& P = a.sp[c.s];
+        float const d = (MODE && P.precision) ? pc_density_at<true>(a, P, i)
+                                              : pc_density_at<false>(a, P, i);
+        float const p = pc_pressure(P, a.pbuf0[i], d);
         a.rho[i] = d;
-        float const p = a.pbuf0[i] + max_x0(d - P.rho0) / P.pcisph_denom;
         a.pbuf0[i] = p;
         a.qdens[i] = p / sqrf(d);
         err = max_0x(d - P.rho0);
@@ -1802,67 +1223,14 @@ __global__ void k_pc_density(Arena a) {
     accumulate_error(S, 0ull, err, c.live);
 }
 
-// pcisph_accumulate_pressure_forces and ..._from_solids (pcisph_ops.cpp:78-178)
-// on the fixed neighbour lists at the predicted positions.
-template <bool K>
-__device__ __forceinline__ void pc_forces(Arena const& a, Ctx const& c) {
-    SceneParams const& P = a.sp[c.s];
-    uint32_t const i = c.i;
-    size_t const stride = a.stride;
-    float const h = P.support;
-    float const m = P.mass;
-    float const N2 = 0.01f * h * h;
-    float2 const pos = a.xstar[i];
-    float2 f = mk2(0.0f, 0.0f);
-    int const cf = a.nf_cnt[i];
-    if (cf) {
-        float2 const vi = a.vstar[i];
-        float const rho = a.rho[i];
-        float const pors = a.qdens[i];
-        SumF2<K> pf;
-        #pragma unroll 4
-
-        for (int k = 0; k < cf; ++k) {
-            uint32_t const j = a.nf_idx[k * stride + i];
-            float2 const vto = sub2(a.xstar[j], pos);
-            float const dist = length2f(vto);
-            float2 const gw = kernel_grad_w(neg2(vto), h);
-            float const rho_j = a.rho[j];
-            pf.add(scl2(pors + a.qdens[j], gw));
-            float2 const dv = sub2(a.vstar[j], vi);
-            float const dvr = dot2(vto, dv);
-            if (dvr < 0.0f) {
-                float const mu = h * dvr / (dist + N2);
-                float const den = (rho + rho_j) / 2.0f;
-                pf.add(scl2(((-1.0f * P.viscosity * mu) + (2.0f * sqrf(mu))) / den, gw));
-            }
-        }
-        f = add2(f, scl2(-(m * m), pf.get()));
-    }
-    int const cs = a.ns_cnt[i];
-    if (cs) {
-        float const pors = a.pbuf0[i] / sqrf(a.rho[i]);
-        SumF2<K> vg;
-        #pragma unroll 4
-
-        for (int k = 0; k < cs; ++k) {
-            uint32_t const j = a.ns_idx[k * stride + i];
-            float2 const gw = kernel_grad_w(neg2(sub2(a.xs[j], pos)), h);
-            vg.add(scl2(a.vols[j], gw));
-        }
-        f = add2(f, scl2(-m * P.rho0 * pors, vg.get()));
-    }
-    a.fp[i] = f;
-}
-
 template <int MODE>
 __global__ void k_pc_forces(Arena a) {
     Ctx c;
     if (!enter(a, true, c) || !c.live) return;
     if (MODE && a.sp[c.s].precision) {
-        pc_forces<true>(a, c);
+        pc_forces_at<true>(a, c);
     } else {
-        pc_forces<false>(a, c);
+        pc_forces_at<false>(a, c);
     }
 }
 

@@ -20,6 +20,35 @@ namespace emerald {
 EMLD_HD float2 mk2(float x, float y) { return make_float2(x, y); }
 EMLD_HD float2 add2(float2 a, float2 b) { return mk2(a.x + b.x, a.y + b.y); }
 EMLD_HD float2 sub2(float2 a, float2 b) { return mk2(a.x - b.x, a.y - b.y); }
+EMLD_HD float2 mul2(float2 a, float2 b) { return mk2(a.x * b.x, a.y * b.y); }
+
+#ifdef __CUDACC__
+// The same three on both halves in one instruction (sm_100's packed
+// single-precision arithmetic: each half rounds as the scalar operation does),
+// for the inner loops of the neighbour sums.
+__device__ __forceinline__ unsigned long long pair_bits(float2 a) {
+    return (static_cast<unsigned long long>(__float_as_uint(a.y)) << 32) | __float_as_uint(a.x);
+}
+__device__ __forceinline__ float2 pair_of(unsigned long long w) {
+    return make_float2(__uint_as_float(static_cast<uint32_t>(w)),
+                       __uint_as_float(static_cast<uint32_t>(w >> 32)));
+}
+__device__ __forceinline__ float2 add2p(float2 a, float2 b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair_bits(a)), "l"(pair_bits(b)));
+    return pair_of(r);
+}
+__device__ __forceinline__ float2 sub2p(float2 a, float2 b) {
+    unsigned long long r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair_bits(a)), "l"(pair_bits(b)));
+    return pair_of(r);
+}
+__device__ __forceinline__ float2 mul2p(float2 a, float2 b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair_bits(a)), "l"(pair_bits(b)));
+    return pair_of(r);
+}
+#endif
 EMLD_HD float2 neg2(float2 a) { return mk2(-a.x, -a.y); }
 EMLD_HD float2 scl2(float s, float2 a) { return mk2(s * a.x, s * a.y); }
 EMLD_HD float2 div2(float2 a, float s) { return mk2(a.x / s, a.y / s); }
@@ -92,12 +121,17 @@ EMLD_HD void kahan_add(KahanF2& k, float2 v) {
 }
 
 // A running sum of float (SumF) or float2 (SumF2) terms: with K = false
-// exactly the reference's s += t, with K = true Kahan-compensated.
+// exactly the reference's s += t, with K = true Kahan-compensated. add(t, on)
+// takes the term only where `on` (a term past a list's end is formed and
+// dropped: one predicated addition instead of a branch around the term).
 template <bool K>
 struct SumF {
     float s;
     EMLD_HD explicit SumF(float init = 0.0f) : s(init) {}
     EMLD_HD void add(float v) { s += v; }
+    EMLD_HD void add(float v, bool on) {
+        if (on) s += v;
+    }
     EMLD_HD float get() const { return s; }
 };
 template <>
@@ -105,6 +139,9 @@ struct SumF<true> {
     KahanF k;
     EMLD_HD explicit SumF(float init = 0.0f) : k{init, 0.0f} {}
     EMLD_HD void add(float v) { kahan_add(k, v); }
+    EMLD_HD void add(float v, bool on) {
+        if (on) kahan_add(k, v);
+    }
     EMLD_HD float get() const { return k.s; }
 };
 template <bool K>
@@ -115,6 +152,12 @@ struct SumF2 {
         s.x += v.x;
         s.y += v.y;
     }
+    EMLD_HD void add(float2 v, bool on) {
+        if (on) {
+            s.x += v.x;
+            s.y += v.y;
+        }
+    }
     EMLD_HD float2 get() const { return s; }
 };
 template <>
@@ -122,6 +165,9 @@ struct SumF2<true> {
     KahanF2 k;
     EMLD_HD SumF2() : k{{0.0f, 0.0f}, {0.0f, 0.0f}} {}
     EMLD_HD void add(float2 v) { kahan_add(k, v); }
+    EMLD_HD void add(float2 v, bool on) {
+        if (on) kahan_add(k, v);
+    }
     EMLD_HD float2 get() const { return float2{k.x.s, k.y.s}; }
 };
 

@@ -110,7 +110,7 @@ def test_server_footprint_matches_allocation(E):
 def test_bursts_on_several_lanes_equal_alone(E):
     """Requests that several lanes admit and step at the same time: the copies
     of one lane's admission are ordered before its own sub-steps."""
-    srv = E.Server(64 << 20, "dfsph_p", max_scenes=16, lanes=4)
+    srv = E.Server(256 << 20, "dfsph_p", max_scenes=16, lanes=4)
     scenes = [scene(E, 40 + 9 * k, 20 + k) for k in range(6)]
     want = [alone(E, sc, 4) for sc in scenes]
     for burst in range(12):
