@@ -957,24 +957,29 @@ void Engine::emit_substep(int32_t method, bool reorder) {
         launch("reorder", [&] { launch_reorder(a_, order_sort_, tiles * kTile, bits, st); },
                3 + 3 * (bits / 8));
     }
-    launch("max_v2", [&] { launch_max_v2(a_, tiles, st); });
-    launch("begin_substep", [&] { launch_begin_substep(a_, max_scenes_, st); });
-    // binning, cell ranges, scatter, per-cell ordering
+    auto begin = [&](cudaStream_t s) {
+        launch("max_v2", [&] { launch_max_v2(a_, tiles, s); });
+        launch("begin_substep", [&] { launch_begin_substep(a_, max_scenes_, s); });
+    };
     Arena const ext = extent_arena();
     bool const kernels = method != kPcisph;
     bool const resident = use_resident(method);
-    // The boundary lists read only positions and the static boundary tables,
-    // so they are built on a side stream (a parallel branch of the graph)
-    // while the fluid cells and fluid lists are built; the per-kernel timing
-    // mode keeps everything on one stream.
+    // The sub-step's dt and the boundary lists need neither the fluid cells nor
+    // the fluid lists, so they are made on a side stream (a parallel branch of
+    // the graph) beside them; the per-kernel timing mode keeps everything on
+    // one stream.
     bool const fork = !timing_;
     if (fork) {
         cudaEventRecord(ev_fork_, st);
         cudaStreamWaitEvent(side_st_, ev_fork_, 0);
+        begin(side_st_);
         launch("neighbors_solid",
                [&] { launch_neighbors(a_, tiles, true, kernels, side_st_, compensated_); });
         cudaEventRecord(ev_join_, side_st_);
+    } else {
+        begin(st);
     }
+    // binning, cell ranges, scatter, per-cell ordering
     launch("build_cells", [&] { launch_build_cells(ext, false, tiles, d_scan_, st); }, 4);
     launch("neighbors_fluid", [&] { launch_neighbors(a_, tiles, false, kernels, st, compensated_); });
     if (fork) {

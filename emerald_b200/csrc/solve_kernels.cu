@@ -130,7 +130,8 @@ __global__ void k_begin_substep(Arena a, int nscenes) {
     SceneParams const& P = a.sp[s];
     SceneState& S = a.ss[s];
     if (!S.active) return;
-    S.error &= ~kErrNonFinite;
+    // (the cell build may report a full table meanwhile)
+    atomicAnd(&S.error, ~kErrNonFinite);
     if (P.mode == kFixedDt) {
         S.dt = P.fixed_dt;
         S.t = P.fixed_t;
