@@ -4,12 +4,14 @@
 // The reference sorts (z, index) pairs and keeps a hash map from z to the
 // [begin, end) range of each cell (neighborhood.cpp:10-124). Here each scene
 // has an open-addressing table keyed by z; binning counts the members of
-// every cell, an exclusive scan turns the counts into ranges, and each
-// cell's member list is ordered by index, which is exactly the order the
-// sorted pairs give inside a cell. The neighbour search then walks the 3x3
-// cells in the reference's row-major order, keeps the first 64 accepted
-// candidates and orders them by (distance, index) (neighborhood.h:199-282),
-// so the lists are bit-identical.
+// every cell, and an exclusive scan turns the counts into ranges. The
+// neighbour search then walks the 3x3 cells in the reference's row-major
+// order, keeps the first 64 accepted candidates and orders them by (distance,
+// index) (neighborhood.h:199-282), so the lists are bit-identical. Inside a
+// cell the reference's sorted pairs are in index order; here a fluid cell's
+// members are in no order, which shows only where the cap cuts a cell (and
+// there the search takes them by index) and in the exported cell maps (which
+// order them first).
 #include "engine_types.cuh"
 #include "kernels.cuh"
 #include "sph_math.cuh"
@@ -66,6 +68,7 @@ struct OtherSet {
     uint32_t const* count;
     uint32_t const* start;
     uint32_t const* members;
+    float2 const* member_x;  // positions in member order (nullptr: by x[members])
     uint32_t log2cap;
     uint32_t begin;
     uint32_t const* oid;      // original index of a stored slot (nullptr: slot - begin)
@@ -79,17 +82,38 @@ __device__ __forceinline__ uint32_t stored_slot(OtherSet const& o, uint32_t oid)
     return o.slot_of ? o.slot_of[o.begin + oid] : o.begin + oid;
 }
 
+// The member of [b, e) that comes next by original index after `after`.
+__device__ __noinline__ uint32_t next_by_index(uint32_t const* members, uint32_t const* oid,
+                                               uint32_t first, uint32_t b, uint32_t e,
+                                               int64_t after) {
+    uint32_t best = 0;
+    int64_t best_index = INT64_MAX;
+#pragma unroll 1
+    for (uint32_t m = b; m != e; ++m) {
+        uint32_t const other = members[m];
+        int64_t const index = oid ? oid[other] : other - first;
+        if (index > after && index < best_index) {
+            best = other;
+            best_index = index;
+        }
+    }
+    return best;
+}
+
 // The neighbour search of create_neighborhoods
 // (emerald/sph_common/neighborhood.h:199-282). Accepted candidates are kept
 // in `list` as (distance bits << 32 | scene-local index), sorted ascending,
 // which is the reference's (distance, index) order for non-negative
-// distances. Returns the count.
-__device__ int find_neighbors(float2 pos,
+// distances. Returns the count. by_index takes each cell's members by index
+// from lists that are in no order, which matters only where the 64-entry cap
+// cuts the candidates.
+__device__ __forceinline__ int find_neighbors(float2 pos,
                               uint32_t self,
                               bool same_set,
                               float cell,
                               float max_distance,
                               OtherSet const& o,
+                              bool by_index,
                               uint64_t (&list)[kMaxNeighbors]) {
     int32_t gx, gy;
     grid_coord(pos, cell, gx, gy);
@@ -101,8 +125,11 @@ __device__ int find_neighbors(float2 pos,
             if (!table_find(o.keys, o.log2cap, z, slot)) continue;
             uint32_t const b = o.start[slot];
             uint32_t const e = b + o.count[slot];
+            int64_t last = -1;
             for (uint32_t m = b; cnt < kMaxNeighbors && m != e; ++m) {
-                uint32_t const other = o.members[m];
+                uint32_t const other =
+                  by_index ? next_by_index(o.members, o.oid, o.begin, b, e, last) : o.members[m];
+                if (by_index) last = original_index(o, other);
                 if (same_set && other == self) continue;
                 float2 const vec = sub2(o.x[other], pos);
                 float const dist = length2f(vec);
@@ -165,6 +192,12 @@ __global__ void k_scatter(Arena a) {
     if (slot == UINT32_MAX) return;
     uint32_t const pos = (SOLID ? a.sstart : a.fstart)[slot] + (SOLID ? a.srank : a.rank)[i];
     (SOLID ? a.smembers : a.members)[pos] = i;
+    if (!SOLID) {
+        // for the search: the cells' positions side by side, and where the
+        // particle itself stands among them
+        a.member_x[pos] = a.x[i];
+        a.rank[i] = pos;
+    }
 }
 
 // Orders every cell's members by original index (the within-cell order of
@@ -192,196 +225,193 @@ __global__ void k_sort_cells(uint32_t const* count,
     }
 }
 
-// Registers that hold a particle's sorted list on the common path.
-constexpr int kRegList = 16;
+// The fast path of the search: a particle with at most kShortList accepted
+// candidates, kSearchBatch of a row's candidates in flight together (a row
+// holds about twelve at one particle per support squared).
+constexpr int kShortList = 16;
+constexpr int kSearchBatch = 6;
 
-// The search of find_neighbors with the sorted list in registers: every
-// accepted key bubbles through kRegList registers (min/max exchange, static
-// indices, so nothing spills). A candidate is rejected before its square root
-// when x*x + y*y >= reject_l2: sqrtf is correctly rounded and monotone, so
-// that test equals the reference's length() >= max_distance for every
-// non-tiny vector, and tiny vectors (dot < 2*FLT_MIN) are far below it.
-// Returns the accepted count; above kRegList the registers overflowed and the
-// caller redoes the particle with the 64-entry list.
-__device__ __forceinline__ int find_neighbors_reg(float2 pos, uint32_t self, bool same_set,
-                                                  float cell, float max_distance, float reject_l2,
-                                                  OtherSet const& o, uint64_t (&r)[kRegList]) {
-#pragma unroll
-    for (int q = 0; q < kRegList; ++q) r[q] = ~0ull;
-    int32_t gx, gy;
-    grid_coord(pos, cell, gx, gy);
-    uint64_t const sx0 = spread_bits(static_cast<uint32_t>(gx - 1));
-    uint64_t const sx1 = spread_bits(static_cast<uint32_t>(gx));
-    uint64_t const sx2 = spread_bits(static_cast<uint32_t>(gx + 1));
-    uint64_t const sy0 = spread_bits(static_cast<uint32_t>(gy - 1)) << 1;
-    uint64_t const sy1 = spread_bits(static_cast<uint32_t>(gy)) << 1;
-    uint64_t const sy2 = spread_bits(static_cast<uint32_t>(gy + 1)) << 1;
-    int cnt = 0;
-#pragma unroll 1
-    for (int jj = 0; jj < 3 && cnt < kMaxNeighbors; ++jj) {
-        uint64_t const zy = jj == 0 ? sy0 : (jj == 1 ? sy1 : sy2);
-#pragma unroll 1
-        for (int kk = 0; kk < 3 && cnt < kMaxNeighbors; ++kk) {
-            uint64_t const zx = kk == 0 ? sx0 : (kk == 1 ? sx1 : sx2);
-            uint32_t slot;
-            if (!table_find(o.keys, o.log2cap, zx | zy, slot)) continue;
-            uint32_t const b = o.start[slot];
-            uint32_t const e = b + o.count[slot];
-#pragma unroll 1
-            for (uint32_t m = b; cnt < kMaxNeighbors && m != e; ++m) {
-                uint32_t const other = o.members[m];
-                if (same_set && other == self) continue;
-                float2 const vec = sub2(o.x[other], pos);
-                if (vec.x * vec.x + vec.y * vec.y >= reject_l2) continue;
-                float const dist = length2f(vec);
-                if (dist >= max_distance) continue;
-                uint64_t key = (static_cast<uint64_t>(__float_as_uint(dist)) << 32) |
-                               static_cast<uint64_t>(original_index(o, other));
-#pragma unroll
-                for (int q = 0; q < kRegList; ++q) {
-                    uint64_t const lo = r[q] < key ? r[q] : key;
-                    key = r[q] < key ? key : r[q];
-                    r[q] = lo;
-                }
-                ++cnt;
-            }
-        }
-    }
-    return cnt;
-}
-
-// Candidates whose member indices, then positions, the shared-memory search
-// loads together before it tests them in order.
-constexpr int kNeighborBatch = 4;
-
-// The [begin, end) member ranges of the three cells (zx_k | zy) of one row:
-// the three first probes are loaded together, then each is resolved (linear
-// probing from there, bounded by the capacity), as table_find does.
-__device__ __forceinline__ void row_ranges(OtherSet const& o, uint64_t zx0, uint64_t zx1,
-                                           uint64_t zx2, uint64_t zy, uint32_t (&b)[3],
-                                           uint32_t (&e)[3]) {
+// The first members and the counts of the nine cells around (gx, gy), in the
+// reference's row-major order: nine first probes in flight together, then
+// nine ranges. Linear probing from the first probe is bounded by the
+// capacity, as in table_find.
+__device__ __forceinline__ void cell_ranges(OtherSet const& o, int32_t gx, int32_t gy,
+                                            uint32_t (&b)[9], uint32_t (&n)[9]) {
     uint32_t const cap = 1u << o.log2cap;
-    uint64_t const z[3] = {zx0 | zy, zx1 | zy, zx2 | zy};
-    uint32_t h[3];
-    uint64_t k[3];
-#pragma unroll
-    for (int q = 0; q < 3; ++q) h[q] = cell_hash(z[q], o.log2cap);
-#pragma unroll
-    for (int q = 0; q < 3; ++q) k[q] = (z[q] == kEmptyKey) ? kEmptyKey : o.keys[h[q]];
-    uint32_t slot[3] = {0u, 0u, 0u};
-    bool found[3];
+    uint64_t zx[3], zy[3];
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-        if (z[q] == kEmptyKey) {
-            slot[q] = cap;
-            found[q] = true;
-        } else if (k[q] == z[q]) {
-            slot[q] = h[q];
-            found[q] = true;
-        } else if (k[q] == kEmptyKey) {
-            found[q] = false;
-        } else {
-            uint32_t hh = h[q];
-            found[q] = false;
-            for (uint32_t probe = 1; probe < cap; ++probe) {
-                hh = (hh + 1u) & (cap - 1u);
-                uint64_t const kk = o.keys[hh];
-                if (kk == z[q]) {
-                    slot[q] = hh;
-                    found[q] = true;
-                    break;
-                }
-                if (kk == kEmptyKey) break;
-            }
-        }
+        zx[q] = spread_bits(static_cast<uint32_t>(gx - 1 + q));
+        zy[q] = spread_bits(static_cast<uint32_t>(gy - 1 + q)) << 1;
+    }
+    uint32_t slot[9];
+    uint64_t k[9];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+        // the reserved slot of cell (-1, -1) is read through the same load
+        uint64_t const z = zx[q % 3] | zy[q / 3];
+        slot[q] = z == kEmptyKey ? cap : cell_hash(z, o.log2cap);
+        k[q] = z == kEmptyKey ? z : o.keys[slot[q]];
     }
 #pragma unroll
-    for (int q = 0; q < 3; ++q) {
-        b[q] = found[q] ? o.start[slot[q]] : 0u;
-        e[q] = found[q] ? b[q] + o.count[slot[q]] : 0u;
+    for (int q = 0; q < 9; ++q) {
+        uint64_t const z = zx[q % 3] | zy[q / 3];
+#pragma unroll 1
+        for (uint32_t probe = 1; k[q] != z && k[q] != kEmptyKey && probe < cap; ++probe) {
+            slot[q] = (slot[q] + 1u) & (cap - 1u);
+            k[q] = o.keys[slot[q]];
+        }
+        bool const found = k[q] == z;
+        b[q] = found ? o.start[slot[q]] : 0u;
+        n[q] = found ? o.count[slot[q]] : 0u;
     }
 }
 
-// The search of find_neighbors_reg with the sorted list in shared memory:
-// entry k of this thread at list[k * kTile]; an accepted key shifts only the
-// entries above it (fewer instructions than the register bubble). The three
-// cells of a row are looked up together, and each cell's members are taken
-// kNeighborBatch at a time (their indices, then their positions, then the
-// tests in member order): the candidates and their order are those of the
-// one-at-a-time walk, with fewer dependent loads in a row (measured 20%
-// faster on B200). Above kRegList entries the caller redoes the particle
-// with the 64-entry list.
-__device__ __forceinline__ int find_neighbors_smem(float2 pos, uint32_t self, bool same_set,
-                                                   float cell, float max_distance, float reject_l2,
-                                                   OtherSet const& o, uint64_t* list) {
-    int32_t gx, gy;
-    grid_coord(pos, cell, gx, gy);
-    uint64_t const sx0 = spread_bits(static_cast<uint32_t>(gx - 1));
-    uint64_t const sx1 = spread_bits(static_cast<uint32_t>(gx));
-    uint64_t const sx2 = spread_bits(static_cast<uint32_t>(gx + 1));
-    int cnt = 0;
+// One thread's column of the block's short lists.
+struct ShortList {
+    float* x;       // vector to the candidate
+    float* y;
+    uint32_t* who;  // its place among the members, then its slot
+};
+
+// Appends the candidates of row r's three cells (first members b, counts n)
+// that are closer than the search distance to the list and returns the new
+// count; what is past kShortList is counted only, and past the cap not even
+// that. The three cells are one run of candidates, so that lanes with
+// differently filled cells stay together. low: the smallest squared distance
+// listed.
+template <bool BY_PLACE>
+__device__ __forceinline__ int search_row(OtherSet const& o, float2 pos, uint32_t self,
+                                          float reject_l2, uint32_t const (&b)[9],
+                                          uint32_t const (&n)[9], int r, ShortList const& list,
+                                          int cnt, float& low) {
+    uint32_t const n0 = n[3 * r];
+    uint32_t const n01 = n0 + n[3 * r + 1];
+    uint32_t const all = n01 + n[3 * r + 2];
+    uint32_t const off0 = b[3 * r];
+    uint32_t const off1 = b[3 * r + 1] - n0;
+    uint32_t const off2 = b[3 * r + 2] - n01;
 #pragma unroll 1
-    for (int jj = 0; jj < 3 && cnt < kMaxNeighbors; ++jj) {
-        uint64_t const zy = spread_bits(static_cast<uint32_t>(gy - 1 + jj)) << 1;
-        uint32_t rb[3], re[3];
-        row_ranges(o, sx0, sx1, sx2, zy, rb, re);
-#pragma unroll 1
-        for (int kk = 0; kk < 3 && cnt < kMaxNeighbors; ++kk) {
-            uint32_t const e = re[kk];
-#pragma unroll 1
-            for (uint32_t m0 = rb[kk]; m0 < e && cnt < kMaxNeighbors; m0 += kNeighborBatch) {
-                uint32_t oth[kNeighborBatch];
-                float2 xo[kNeighborBatch];
+    for (uint32_t m0 = 0; m0 < all && cnt <= kMaxNeighbors; m0 += kSearchBatch) {
+        uint32_t at[kSearchBatch];
+        float2 xo[kSearchBatch];
 #pragma unroll
-                for (int u = 0; u < kNeighborBatch; ++u) {
-                    if (m0 + u < e) oth[u] = o.members[m0 + u];
-                }
+        for (int u = 0; u < kSearchBatch; ++u) {
+            uint32_t const m = m0 + u;
+            at[u] = m + (m < n0 ? off0 : (m < n01 ? off1 : off2));
+            // past the end of the row: the particle's own place, not taken
+            if (m >= all) at[u] = self;
+        }
+        if (!BY_PLACE) {
 #pragma unroll
-                for (int u = 0; u < kNeighborBatch; ++u) {
-                    if (m0 + u < e) xo[u] = o.x[oth[u]];
-                }
-#pragma unroll
-                for (int u = 0; u < kNeighborBatch; ++u) {
-                    if (m0 + u >= e || cnt >= kMaxNeighbors) break;
-                    uint32_t const other = oth[u];
-                    if (same_set && other == self) continue;
-                    float2 const vec = sub2(xo[u], pos);
-                    if (vec.x * vec.x + vec.y * vec.y >= reject_l2) continue;
-                    float const dist = length2f(vec);
-                    if (dist >= max_distance) continue;
-                    uint64_t const key = (static_cast<uint64_t>(__float_as_uint(dist)) << 32) |
-                                         static_cast<uint64_t>(original_index(o, other));
-                    if (cnt < kRegList) {
-                        int p = cnt;
-                        while (p > 0) {
-                            uint64_t const prev = list[(p - 1) * kTile];
-                            if (prev < key) break;
-                            list[p * kTile] = prev;
-                            --p;
-                        }
-                        list[p * kTile] = key;
-                    }
-                    ++cnt;
-                }
+            for (int u = 0; u < kSearchBatch; ++u) {
+                if (at[u] != self) at[u] = o.members[at[u]];
             }
+        }
+#pragma unroll
+        for (int u = 0; u < kSearchBatch; ++u) {
+            if (BY_PLACE) {
+                xo[u] = o.member_x[at[u]];
+            } else {
+                xo[u] = pos;
+                if (at[u] != self) xo[u] = o.x[at[u]];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kSearchBatch; ++u) {
+            float2 const vec = sub2(xo[u], pos);
+            float const l2 = vec.x * vec.x + vec.y * vec.y;
+            bool const take = at[u] != self && !(l2 >= reject_l2);
+            if (take && cnt < kShortList) {
+                list.x[cnt * kTile] = vec.x;
+                list.y[cnt * kTile] = vec.y;
+                list.who[cnt * kTile] = at[u];
+            }
+            low = take ? fminf(low, l2) : low;
+            cnt += take ? 1 : 0;
         }
     }
     return cnt;
+}
+
+// The order of the cnt <= kShortList listed candidates by (distance, index):
+// list position of the k-th in bits 4k..4k+3. Batcher's odd-even merge sort
+// (K. Batcher, "Sorting networks and their applications", 1968) in registers,
+// the same instructions in every lane whatever the counts, where an insertion
+// sort costs a warp the longest of its lanes' moves at every candidate. The
+// keys are the distances with their last four bits replaced by the list
+// position; where two keys differ in nothing else, the exact distances and the
+// indices decide afterwards.
+template <bool BY_PLACE>
+__device__ __forceinline__ uint64_t sort_short_list(OtherSet const& o, ShortList const& list,
+                                                    int cnt) {
+    uint32_t d[kShortList];
+#pragma unroll
+    for (int q = 0; q < kShortList; ++q) {
+        // no distance has these bits, and no two of them the same upper ones
+        d[q] = 0xffffff00u + 17u * q;
+        if (q < cnt) {
+            float const vx = list.x[q * kTile], vy = list.y[q * kTile];
+            d[q] = (__float_as_uint(sqrtf(vx * vx + vy * vy)) & ~15u) | q;
+            if (BY_PLACE) list.who[q * kTile] = o.members[list.who[q * kTile]];
+        }
+    }
+    constexpr int kSpan[10] = {1, 2, 2, 4, 4, 4, 8, 8, 8, 8};
+    constexpr int kStep[10] = {1, 2, 1, 4, 2, 1, 8, 4, 2, 1};
+#pragma unroll
+    for (int t = 0; t < 10; ++t) {
+        int const span = kSpan[t], k = kStep[t];
+#pragma unroll
+        for (int lo = 0; lo < kShortList; ++lo) {
+            int const hi = lo + k;
+            bool const pair = hi < kShortList && lo >= k % span &&
+                              (lo - k % span) % (2 * k) < k && lo / (2 * span) == hi / (2 * span);
+            if (pair) {
+                uint32_t const dl = min(d[lo], d[hi]);
+                d[hi] = max(d[lo], d[hi]);
+                d[lo] = dl;
+            }
+        }
+    }
+    bool tie = false;
+#pragma unroll
+    for (int q = 1; q < kShortList; ++q) tie = tie || (d[q] ^ d[q - 1]) < 16u;
+    uint32_t half[2] = {0u, 0u};
+#pragma unroll
+    for (int q = 0; q < kShortList; ++q) half[q / 8] |= (d[q] & 15u) << (4 * (q % 8));
+    uint64_t order = (static_cast<uint64_t>(half[1]) << 32) | half[0];
+    if (tie) {
+        auto key = [&](int k) {
+            uint32_t const at = (static_cast<uint32_t>(order >> (4 * k)) & 15u) * kTile;
+            float const dist = sqrtf(list.x[at] * list.x[at] + list.y[at] * list.y[at]);
+            return (static_cast<uint64_t>(__float_as_uint(dist)) << 32) |
+                   original_index(o, list.who[at]);
+        };
+#pragma unroll 1
+        for (int k = 1; k < cnt; ++k) {
+#pragma unroll 1
+            for (int q = k; q > 0 && key(q) < key(q - 1); --q) {
+                uint64_t const diff = ((order >> (4 * q)) ^ (order >> (4 * q - 4))) & 15u;
+                order ^= (diff << (4 * q)) | (diff << (4 * q - 4));
+            }
+        }
+    }
+    return order;
 }
 
 // Writes list entry k of particle i: index, W and GradW(-vector_to)
 // (compute_neighbor_kernels / compute_neighbor_kernel_gradients,
-// emerald/sph_common/neighborhood.cpp:178-210), the vector recomputed from
-// positions bit for bit and its length taken from the search.
+// emerald/sph_common/neighborhood.cpp:178-210) from the vector to the
+// neighbour and its length.
 __device__ __forceinline__ void write_entry(uint32_t* idx_out, float* w_out, float2* gw_out,
-                                            size_t e, uint32_t j, float dist, float2 pos,
-                                            float2 const* xo, float h, bool kernels) {
+                                            size_t e, uint32_t j, float dist, float2 vec,
+                                            float h, bool kernels) {
     idx_out[e] = j;
     if (!kernels) return;
     float w, dw;
     kernel_w_dw(dist, h, w, dw);
     w_out[e] = w;
-    float2 const dp = neg2(sub2(xo[j], pos));
+    float2 const dp = neg2(vec);
     float2 g = mk2(0.0f, 0.0f);
     if (safe_v(dp, dist)) {
         float2 const u = div2(dp, dist);
@@ -413,8 +443,199 @@ __device__ __noinline__ void write_entry_precise(uint32_t* idx_out, float* w_out
     gw_out[e] = g;
 }
 
+// What the search of a particle without a short list needs.
+struct LongSearch {
+    OtherSet o;
+    float2 pos;
+    uint32_t i, self;
+    int cnt;      // accepted candidates, or any number past the cap
+    bool normal;  // every vector's length is the root of its dot product
+    float cell, reject_l2, h;
+    uint8_t* cnt_out;
+    uint32_t* idx_out;
+    float* w_out;
+    float2* gw_out;
+    size_t stride;
+    bool kernels, precise;
+    double2 pos64;
+    double2 const* x64o;
+    ShortList list;
+};
+
+// Particles with 17 to 64 neighbours: runs of sixteen are sorted by the network
+// and merged as they are written. Where a vector is too short for its dot
+// product the one-at-a-time search decides.
+// Out of line, so that k_neighbors keeps its registers. A 256 x 256 frame at a
+// support of two spacings (45 neighbours) took 5.3 ms with PCISPH when every
+// long list was made by insertion, 2.1 ms now; 1.5 spacings (26 neighbours)
+// with IISPH 3.5 and 1.9 ms.
+template <bool SOLID_OTHER>
+__device__ __noinline__ void neighbors_long(LongSearch s) {
+    OtherSet const& o = s.o;
+    ShortList const& list = s.list;
+    float2 const pos = s.pos;
+    int cnt = s.cnt;
+    uint64_t full[kMaxNeighbors];
+    int ends[4];  // of the sorted runs of `full`
+    // the places of the first kMaxNeighbors accepted, in any order
+    int found = 0;
+    float low = s.normal ? 1.0f : 0.0f;
+    if (s.normal) {
+        uint32_t b[9], n[9];
+        int32_t gx, gy;
+        grid_coord(pos, s.cell, gx, gy);
+        cell_ranges(o, gx, gy, b, n);
+#pragma unroll 1
+        for (int q = 0; q < 9 && found < kMaxNeighbors; ++q) {
+            uint32_t const e = b[q] + n[q];
+            int const before = found;
+            auto test = [&](uint32_t m, uint32_t& place, float& l2) {
+                place = SOLID_OTHER ? o.members[m] : m;
+                float2 const vec = sub2(SOLID_OTHER ? o.x[place] : o.member_x[place], pos);
+                l2 = vec.x * vec.x + vec.y * vec.y;
+                return place != s.self && !(l2 >= s.reject_l2);
+            };
+            uint32_t place;
+            float l2;
+#pragma unroll 1
+            for (uint32_t m = b[q]; m != e; ++m) {
+                if (!test(m, place, l2)) continue;
+                low = fminf(low, l2);
+                if (found < kMaxNeighbors) full[found] = place;
+                ++found;
+            }
+            if (found <= kMaxNeighbors) continue;
+            found = kMaxNeighbors;
+            if (SOLID_OTHER) continue;
+            // the cap cuts this cell, whose members are in no order: those of
+            // the lowest indices stay
+            int c = before;
+#pragma unroll 1
+            for (uint32_t m = b[q]; m != e; ++m) {
+                if (!test(m, place, l2)) continue;
+                uint64_t const key =
+                  (static_cast<uint64_t>(original_index(o, o.members[place])) << 32) | place;
+                if (c == kMaxNeighbors && key >= full[c - 1]) continue;
+                int p = c < kMaxNeighbors ? c++ : c - 1;
+                for (; p > before && full[p - 1] > key; --p) full[p] = full[p - 1];
+                full[p] = key;
+            }
+        }
+    }
+    if (low >= 2.0f * kFltMin) {
+        // sixteen at a time through the short list, then merged
+        cnt = found;
+#pragma unroll
+        for (int run = 0; run < 4; ++run) {
+            int const first = run * kShortList;
+            int const c = max(0, min(cnt - first, kShortList));
+            ends[run] = first + c;
+            if (c == 0) continue;
+#pragma unroll
+            for (int q = 0; q < kShortList; ++q) {
+                if (q < c) {
+                    uint32_t const place = static_cast<uint32_t>(full[first + q]);
+                    float2 const vec =
+                      sub2(SOLID_OTHER ? o.x[place] : o.member_x[place], pos);
+                    list.x[q * kTile] = vec.x;
+                    list.y[q * kTile] = vec.y;
+                    list.who[q * kTile] = place;
+                }
+            }
+            uint64_t order = sort_short_list<!SOLID_OTHER>(o, list, c);
+#pragma unroll 1
+            for (int q = 0; q < c; ++q, order >>= 4) {
+                uint32_t const at = (static_cast<uint32_t>(order) & 15u) * kTile;
+                float const dist = sqrtf(list.x[at] * list.x[at] + list.y[at] * list.y[at]);
+                full[first + q] = (static_cast<uint64_t>(__float_as_uint(dist)) << 32) |
+                                  original_index(o, list.who[at]);
+            }
+        }
+    } else {
+        cnt = find_neighbors(pos, s.i, !SOLID_OTHER, s.cell, s.cell, o,
+                             !SOLID_OTHER && cnt > kMaxNeighbors, full);
+        ends[0] = cnt;
+        ends[1] = kShortList;
+        ends[2] = 2 * kShortList;
+        ends[3] = 3 * kShortList;
+    }
+    s.cnt_out[s.i] = static_cast<uint8_t>(cnt);
+    int at[4] = {0, kShortList, 2 * kShortList, 3 * kShortList};
+    uint64_t head[4];
+#pragma unroll
+    for (int run = 0; run < 4; ++run) head[run] = at[run] < ends[run] ? full[at[run]] : ~0ull;
+#pragma unroll 1
+    for (int k = 0; k < cnt; ++k) {
+        uint64_t const lo = head[0] < head[1] ? head[0] : head[1];
+        uint64_t const hi = head[2] < head[3] ? head[2] : head[3];
+        uint64_t const key = lo < hi ? lo : hi;
+#pragma unroll
+        for (int run = 0; run < 4; ++run) {
+            if (head[run] == key) {
+                ++at[run];
+                head[run] = at[run] < ends[run] ? full[at[run]] : ~0ull;
+            }
+        }
+        size_t const e = static_cast<size_t>(k) * s.stride + s.i;
+        uint32_t const j = stored_slot(o, static_cast<uint32_t>(key & 0xffffffffu));
+        if (s.precise) {
+            write_entry_precise(s.idx_out, s.w_out, s.gw_out, e, j, s.pos64, s.x64o, o.x, s.h);
+        } else {
+            write_entry(s.idx_out, s.w_out, s.gw_out, e, j,
+                        __uint_as_float(static_cast<uint32_t>(key >> 32)), sub2(o.x[j], pos), s.h,
+                        s.kernels);
+        }
+    }
+}
+
+// kernel_w_dw's quotients by what depends on the support alone, with the same
+// bits from five multiply-adds each: for y = RN(1 / b) and a q within one ulp
+// of a / b whose remainder r = a - b q is exact, RN(q + r y) is the correctly
+// rounded quotient (P. Markstein, "Computation of elementary functions on the
+// IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990). The first
+// correction makes q that close. Supports in [2^-16, 2^10] keep every
+// quotient and remainder in the normal range for 2^-62 <= r < 2 h (what the
+// short lists hold): the smallest numerators are 2^-71 (W), 2^-46 and 2^-61
+// (GradW), the divisors lie in 2^-46..2^32, and no numerator is zero because
+// r / h cannot round to 2 for r < 2 h.
+struct KernelDivisors {
+    float h, hh, h4, hhh, k;
+    float y_h, y_hh, y_h4, y_hhh, y_k;
+    bool quick;
+    __device__ __forceinline__ explicit KernelDivisors(float support)
+        : h(support), hh(h * h), h4(4.0f * h), hhh(h * h * h), k(h * h * h * kPi),
+          y_h(1.0f / h), y_hh(1.0f / hh), y_h4(1.0f / h4), y_hhh(1.0f / hhh), y_k(1.0f / k),
+          quick(h >= 0x1p-16f && h <= 0x1p10f) {}
+    static __device__ __forceinline__ float quotient(float a, float b, float y) {
+        float q = a * y;
+        q = __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+        return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+    }
+    __device__ __forceinline__ void kernel_w_dw(float r, float& w, float& dw) const {
+        float const q = quotient(r, h, y_h);
+        bool const inner = q <= 1.0f;
+        float const t = 2.0f - q;
+        float d = quotient(inner ? -3.0f * r : -3.0f * sqrf(t), inner ? hh : h4,
+                           inner ? y_hh : y_h4);
+        if (inner) d = d + quotient(2.25f * r * r, hhh, y_hhh);
+        w = quotient(inner ? 1.0f + q * q * (q * 0.75f - 1.5f) : (t * t * t) / 4.0f, k, y_k);
+        dw = quotient(d, k, y_k);
+    }
+};
+
+// One thread a particle, 62 registers (eight blocks an SM; left alone the
+// compiler takes 56 and spills). What bounds it is instruction issue and, below
+// a wave of blocks, one warp's chain of dependent reads: cell keys, cell
+// ranges, then per row two batches of positions that the cell build has laid
+// side by side (an index in between would double the chain and the loads).
+// Kernel time on one B200 with cold caches, before -> after the short lists
+// moved from an insertion sort to the fixed network, the positions to member
+// order and W's divisions to multiply-adds: 2k particles 28 -> 15.7 us, 37k
+// 30 -> 17.8 us, 262k 70 -> 50 us, 1M 232 -> 171 us. Batches of four measured
+// 16.8 / 18.6 / 50.6 / 173 us, with the next batch in flight 17.3 / 19.2 /
+// 51.8 / 178 us; four lanes a particle 17.6 / 38 / 158 / 629 us.
 template <bool SOLID_OTHER, bool COMP>
-__global__ void __launch_bounds__(kTile) k_neighbors(Arena a, int write_kernels) {
+__global__ void __launch_bounds__(kTile, 8) k_neighbors(Arena a, int write_kernels) {
     int32_t const s = a.tile_scene[blockIdx.x];
     if (s < 0) return;
     SceneParams const& P = a.sp[s];
@@ -426,10 +647,10 @@ __global__ void __launch_bounds__(kTile) k_neighbors(Arena a, int write_kernels)
     OtherSet o;
     if (SOLID_OTHER) {
         o = OtherSet{a.xs, a.skeys + P.stab_begin, a.scount + P.stab_begin, a.sstart + P.stab_begin,
-                     a.smembers, P.stab_log2, P.solid_begin, nullptr, nullptr};
+                     a.smembers, nullptr, P.stab_log2, P.solid_begin, nullptr, nullptr};
     } else {
         o = OtherSet{a.x, a.fkeys + P.ftab_begin, a.fcount + P.ftab_begin, a.fstart + P.ftab_begin,
-                     a.members, P.ftab_log2, P.fluid_begin, a.oid, a.slot_of};
+                     a.members, a.member_x, P.ftab_log2, P.fluid_begin, a.oid, a.slot_of};
     }
     uint8_t* cnt_out = SOLID_OTHER ? a.ns_cnt : a.nf_cnt;
     uint32_t* idx_out = SOLID_OTHER ? a.ns_idx : a.nf_idx;
@@ -442,9 +663,9 @@ __global__ void __launch_bounds__(kTile) k_neighbors(Arena a, int write_kernels)
     }
     bool const kernels = write_kernels != 0;
     float2 const pos = a.x[i];
+    int32_t gx, gy;
+    grid_coord(pos, cell, gx, gy);
     if (SOLID_OTHER && P.near_w) {
-        int32_t gx, gy;
-        grid_coord(pos, cell, gx, gy);
         int64_t const ix = int64_t(gx) - P.near_x0;
         int64_t const iy = int64_t(gy) - P.near_y0;
         bool near = false;
@@ -457,81 +678,62 @@ __global__ void __launch_bounds__(kTile) k_neighbors(Arena a, int write_kernels)
             return;
         }
     }
-    if (!(COMP && P.precision && kernels)) {
-        __shared__ uint64_t s_list[kRegList * kTile];
-        uint64_t* const list = s_list + threadIdx.x;
-        int const cnt = find_neighbors_smem(pos, i, !SOLID_OTHER, cell, cell, P.reject_l2, o, list);
+    __shared__ uint32_t s_list[3 * kShortList * kTile];
+    ShortList const list{reinterpret_cast<float*>(s_list) + threadIdx.x,
+                         reinterpret_cast<float*>(s_list) + kShortList * kTile + threadIdx.x,
+                         s_list + 2 * kShortList * kTile + threadIdx.x};
+    int cnt = 0;
+    float low = 1.0f;
+    uint32_t const self = SOLID_OTHER ? UINT32_MAX : a.rank[i];
+    {
+        uint32_t b[9], n[9];
+        cell_ranges(o, gx, gy, b, n);
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            cnt = search_row<!SOLID_OTHER>(o, pos, self, P.reject_l2, b, n, r, list, cnt, low);
+        }
+    }
+    bool const precise = COMP && P.precision && kernels;
+    double2 const pos64 = precise ? a.x64[i] : make_double2(0.0, 0.0);
+    double2 const* const x64o = SOLID_OTHER ? nullptr : a.x64;
+    KernelDivisors const div(h);
+    // From 2*FLT_MIN on a vector's length is the root of its dot product, which
+    // is below max_distance exactly when the product is below reject_l2.
+    if (cnt <= kShortList && low >= 2.0f * kFltMin) {
+        uint64_t order = sort_short_list<!SOLID_OTHER>(o, list, cnt);
         cnt_out[i] = static_cast<uint8_t>(cnt);
-        if (cnt <= kRegList) {
 #pragma unroll 1
-            for (int k = 0; k < cnt; ++k) {
-                uint64_t const key = list[k * kTile];
-                write_entry(idx_out, w_out, gw_out, static_cast<size_t>(k) * stride + i,
-                            stored_slot(o, static_cast<uint32_t>(key & 0xffffffffu)),
-                            __uint_as_float(static_cast<uint32_t>(key >> 32)), pos, o.x, h,
-                            kernels);
+        for (int k = 0; k < cnt; ++k, order >>= 4) {
+            uint32_t const at = (static_cast<uint32_t>(order) & 15u) * kTile;
+            size_t const e = static_cast<size_t>(k) * stride + i;
+            if (precise) {
+                write_entry_precise(idx_out, w_out, gw_out, e, list.who[at], pos64, x64o, o.x, h);
+                continue;
             }
-            return;
-        }
-        uint64_t full[kMaxNeighbors];
-        int const n64 = find_neighbors(pos, i, !SOLID_OTHER, cell, cell, o, full);
-#pragma unroll 1
-        for (int k = 0; k < n64; ++k) {
-            write_entry(idx_out, w_out, gw_out, static_cast<size_t>(k) * stride + i,
-                        stored_slot(o, static_cast<uint32_t>(full[k] & 0xffffffffu)),
-                        __uint_as_float(static_cast<uint32_t>(full[k] >> 32)), pos, o.x, h,
-                        kernels);
-        }
-        return;
-    }
-    // compensated scenes: the register list, with entries from double positions
-    uint64_t r[kRegList];
-    int const cnt = find_neighbors_reg(pos, i, !SOLID_OTHER, cell, cell, P.reject_l2, o, r);
-    cnt_out[i] = static_cast<uint8_t>(cnt);
-    if (COMP && P.precision && kernels) {
-        double2 const pos64 = a.x64[i];
-        double2 const* x64o = SOLID_OTHER ? nullptr : a.x64;
-        uint64_t full[kMaxNeighbors];
-        int const n64 = cnt <= kRegList ? cnt : find_neighbors(pos, i, !SOLID_OTHER, cell, cell, o, full);
-#pragma unroll 1
-        for (int k = 0; k < n64; ++k) {
-            uint64_t key;
-            if (cnt <= kRegList) {
-                key = r[0];
-#pragma unroll
-                for (int q = 0; q + 1 < kRegList; ++q) r[q] = r[q + 1];
+            idx_out[e] = list.who[at];
+            if (!kernels) continue;
+            float2 const dp = mk2(-list.x[at], -list.y[at]);
+            float const dist = sqrtf(dp.x * dp.x + dp.y * dp.y);
+            float w, dw;
+            if (div.quick) {
+                div.kernel_w_dw(dist, w, dw);
             } else {
-                key = full[k];
+                kernel_w_dw(dist, h, w, dw);
             }
-            write_entry_precise(idx_out, w_out, gw_out, static_cast<size_t>(k) * stride + i,
-                                stored_slot(o, static_cast<uint32_t>(key & 0xffffffffu)), pos64,
-                                x64o, o.x, h);
+            w_out[e] = w;
+            // safe_v: dist is not zero, so only a NaN fails it
+            float2 g = mk2(0.0f, 0.0f);
+            if (dist > 0.0f) {
+                float2 const u = div2(dp, dist);
+                g = mk2(u.x * dw, u.y * dw);
+            }
+            gw_out[e] = g;
         }
         return;
     }
-    if (cnt <= kRegList) {
-        // drain the sorted registers from the front: one copy of the entry
-        // code, register moves instead of dynamic indexing
-#pragma unroll 1
-        for (int k = 0; k < cnt; ++k) {
-            uint64_t const key = r[0];
-#pragma unroll
-            for (int q = 0; q + 1 < kRegList; ++q) r[q] = r[q + 1];
-            write_entry(idx_out, w_out, gw_out, static_cast<size_t>(k) * stride + i,
-                        stored_slot(o, static_cast<uint32_t>(key & 0xffffffffu)),
-                        __uint_as_float(static_cast<uint32_t>(key >> 32)), pos, o.x, h, kernels);
-        }
-        return;
-    }
-    // more than kRegList neighbours: the full 64-entry list
-    uint64_t full[kMaxNeighbors];
-    int const n64 = find_neighbors(pos, i, !SOLID_OTHER, cell, cell, o, full);
-#pragma unroll 1
-    for (int k = 0; k < n64; ++k) {
-        write_entry(idx_out, w_out, gw_out, static_cast<size_t>(k) * stride + i,
-                    stored_slot(o, static_cast<uint32_t>(full[k] & 0xffffffffu)),
-                    __uint_as_float(static_cast<uint32_t>(full[k] >> 32)), pos, o.x, h, kernels);
-    }
+    neighbors_long<SOLID_OTHER>(LongSearch{o, pos, i, self, cnt, low >= 2.0f * kFltMin, cell,
+                                           P.reject_l2, h, cnt_out, idx_out, w_out, gw_out, stride,
+                                           kernels, precise, pos64, x64o, list});
 }
 
 // compute_volumes (emerald/sph2d_box/solids.cpp:52-74) over the solid-solid
@@ -544,9 +746,9 @@ __global__ void k_solid_volumes(Arena a, float numer, int only_scene) {
     uint32_t const i = blockIdx.x * kTile + threadIdx.x;
     if (i - P.solid_begin >= P.solid_count) return;
     OtherSet const o{a.xs, a.skeys + P.stab_begin, a.scount + P.stab_begin, a.sstart + P.stab_begin,
-                     a.smembers, P.stab_log2, P.solid_begin, nullptr, nullptr};
+                     a.smembers, nullptr, P.stab_log2, P.solid_begin, nullptr, nullptr};
     uint64_t list[kMaxNeighbors];
-    int const cnt = find_neighbors(a.xs[i], i, true, P.cell_size, P.cell_size, o, list);
+    int const cnt = find_neighbors(a.xs[i], i, true, P.cell_size, P.cell_size, o, false, list);
     float const w0 = kernel_w(0.0f, P.support);
     if (!cnt) {
         a.vols[i] = 1.0f / w0;
@@ -701,9 +903,12 @@ void launch_build_cells(Arena const& a, bool solid, uint32_t tiles, uint32_t* sc
         k_cell_ranges<<<(a.ftab_total + kScanBlock - 1) / kScanBlock, kScanThreads, 0, st>>>(
           a.fcount, a.ftab_total, a.fstart);
         k_scatter<false><<<tiles, kTile, 0, st>>>(a);
-        k_sort_cells<<<(a.ftab_total + 255) / 256, 256, 0, st>>>(a.fcount, a.fstart, a.members,
-                                                                 a.oid, a.ftab_total);
     }
+}
+
+void launch_order_members(Arena const& a, uint32_t tab_begin, uint32_t tab_size, cudaStream_t st) {
+    k_sort_cells<<<(tab_size + 255) / 256, 256, 0, st>>>(a.fcount + tab_begin, a.fstart + tab_begin,
+                                                         a.members, a.oid, tab_size);
 }
 
 void launch_neighbors(Arena const& a, uint32_t tiles, bool solid_other, bool write_kernels,

@@ -276,6 +276,7 @@ Engine::Engine(uint32_t fluid_capacity, uint32_t solid_capacity, int max_scenes)
     a_.slot = reinterpret_cast<uint32_t*>(a_.tkdiv);
     a_.rank = reinterpret_cast<uint32_t*>(a_.tkdens);
     a_.members = static_cast<uint32_t*>(dev(4 * N));
+    a_.member_x = a_.tx;  // the re-sort is over before the cells are built
     a_.zkey = static_cast<uint64_t*>(dev(8 * N));
     a_.ftab_total = ftab_.capacity();
     a_.fkeys = static_cast<uint64_t*>(dev(8ull * a_.ftab_total));
@@ -979,8 +980,8 @@ void Engine::emit_substep(int32_t method, bool reorder) {
     } else {
         begin(st);
     }
-    // binning, cell ranges, scatter, per-cell ordering
-    launch("build_cells", [&] { launch_build_cells(ext, false, tiles, d_scan_, st); }, 4);
+    // binning, cell ranges, scatter
+    launch("build_cells", [&] { launch_build_cells(ext, false, tiles, d_scan_, st); }, 3);
     launch("neighbors_fluid", [&] { launch_neighbors(a_, tiles, false, kernels, st, compensated_); });
     if (fork) {
         cudaStreamWaitEvent(st, ev_join_, 0);
@@ -1912,6 +1913,7 @@ size_t Engine::get_sort(int id, bool solid, int32_t* gc, uint64_t* z, uint64_t* 
     p += 8 * words;
     uint32_t* d_nb = reinterpret_cast<uint32_t*>(p);
     launch("sort_products", [&] {
+        if (!solid) launch_order_members(a_, P.ftab_begin, sc.ftab_size, st_);
         launch_sort_products(a_, solid, id, solid ? P.solid_begin : P.fluid_begin, n,
                              solid ? P.stab_begin : P.ftab_begin, solid ? sc.stab_size : sc.ftab_size,
                              P.cell_size, sort_, d_gc, d_z, d_pz, d_pi, d_bi, d_bl, d_nb, st_);

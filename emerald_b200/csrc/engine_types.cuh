@@ -214,6 +214,7 @@ struct Arena {
     uint32_t* rank;
     uint64_t* zkey;   // z key of each particle at the last build
     uint32_t* members;
+    float2* member_x;  // positions in member order, from the cell build to the search
     uint64_t* fkeys;
     uint32_t* fcount;
     uint32_t* fstart;

@@ -14,6 +14,10 @@ void launch_exclusive_scan(uint32_t const* in, uint32_t n, uint32_t* out, uint32
                            cudaStream_t st);
 void launch_build_cells(Arena const& a, bool solid, uint32_t tiles, uint32_t* scan_scratch,
                         cudaStream_t st);
+// Orders the members of the fluid cells in [tab_begin, tab_begin + tab_size) by
+// original index, as the exported cell maps list them (the build leaves them in
+// no order: the search needs none).
+void launch_order_members(Arena const& a, uint32_t tab_begin, uint32_t tab_size, cudaStream_t st);
 void launch_neighbors(Arena const& a, uint32_t tiles, bool solid_other, bool write_kernels,
                       cudaStream_t st, bool comp = false);
 void launch_solid_volumes(Arena const& a, uint32_t solid_tiles, float numer, int scene,

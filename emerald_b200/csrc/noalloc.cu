@@ -44,7 +44,8 @@ constexpr size_t kOffStart = align256(kOffCount + size_t(kTableSize) * 4);
 constexpr size_t kOffSlot = align256(kOffStart + size_t(kTableSize) * 4);
 constexpr size_t kOffRank = align256(kOffSlot + size_t(kMaxPoints) * 4);
 constexpr size_t kOffMembers = align256(kOffRank + size_t(kMaxPoints) * 4);
-constexpr size_t kOffZkey = align256(kOffMembers + size_t(kMaxPoints) * 4);
+constexpr size_t kOffMemberX = align256(kOffMembers + size_t(kMaxPoints) * 4);
+constexpr size_t kOffZkey = align256(kOffMemberX + size_t(kMaxPoints) * 8);
 constexpr size_t kOffScan = align256(kOffZkey + size_t(kMaxPoints) * 8);
 constexpr size_t kScratchBytes = align256(kOffScan + size_t(kScanWords) * 4);
 
@@ -137,6 +138,7 @@ extern "C" int emerald_neighbors_static(void const* d_xy, uint32_t n, float supp
     a.slot = reinterpret_cast<uint32_t*>(base + kOffSlot);
     a.rank = reinterpret_cast<uint32_t*>(base + kOffRank);
     a.members = reinterpret_cast<uint32_t*>(base + kOffMembers);
+    a.member_x = reinterpret_cast<float2*>(base + kOffMemberX);
     a.zkey = reinterpret_cast<uint64_t*>(base + kOffZkey);
     a.ftab_total = kTableSize;
     uint32_t const tiles = (n + kTile - 1) / kTile;

@@ -197,16 +197,16 @@ EMLD_HD float kernel_dw(float r, float h) {
 // W and dW of the same r, sharing q = r / h (the same value either function
 // computes on its own).
 EMLD_HD void kernel_w_dw(float r, float h, float& w, float& dw) {
+    // one division for both branches of each quotient
     float const q = r / h;
     float const k = h * h * h * kPi;
-    if (q <= 1.0f) {
-        w = (1.0f + q * q * (q * 0.75f - 1.5f)) / k;
-        dw = (-3.0f * r / (h * h) + 2.25f * r * r / (h * h * h)) / k;
-    } else if (q <= 2.0f) {
-        float const t = 2.0f - q;
-        w = ((t * t * t) / 4.0f) / k;
-        dw = (-3.0f * sqrf(2.0f - q) / (4.0f * h)) / k;
-    } else {
+    bool const inner = q <= 1.0f;
+    float const t = 2.0f - q;
+    float d = (inner ? -3.0f * r : -3.0f * sqrf(t)) / (inner ? h * h : 4.0f * h);
+    if (inner) d = d + 2.25f * r * r / (h * h * h);
+    w = (inner ? 1.0f + q * q * (q * 0.75f - 1.5f) : (t * t * t) / 4.0f) / k;
+    dw = d / k;
+    if (!(q <= 2.0f)) {
         w = 0.0f;
         dw = 0.0f;
     }
