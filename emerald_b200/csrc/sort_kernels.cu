@@ -10,6 +10,8 @@
 #include "kernels.cuh"
 #include "sph_math.cuh"
 
+#include <algorithm>
+
 namespace emerald {
 
 namespace {
@@ -67,6 +69,166 @@ __global__ void k_rank_scatter(uint64_t const* kin, uint32_t const* vin, uint64_
             vout[pos] = vin[e];
         }
         __syncthreads();
+    }
+}
+
+// Words of the resident sort at the start of the scan scratch, zero at launch.
+struct SortControl {
+    unsigned long long any;      // OR of the keys
+    unsigned long long any_not;  // OR of their complements
+    uint32_t arrived;            // blocks at the grid barriers so far
+    uint32_t stalled;            // a barrier ran out of polls: every block returns
+};
+
+constexpr int kSortThreads = 1024;
+constexpr int kSortWarps = kSortThreads / 32;
+constexpr uint32_t kSortPolls = 1u << 22;
+
+// False when a block did not come: the launch is cooperative, so all are
+// resident and this only bounds the wait.
+__device__ __forceinline__ bool sort_barrier(SortControl* c, uint32_t target) {
+    __syncthreads();
+    uint32_t bad = 0;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(&c->arrived, 1u);
+        uint32_t polls = 0;
+        while (*reinterpret_cast<uint32_t volatile*>(&c->arrived) < target) {
+            bad = *reinterpret_cast<uint32_t volatile*>(&c->stalled);
+            if (bad) break;
+            if (++polls == kSortPolls) {
+                atomicExch(&c->stalled, 1u);
+                bad = 1;
+                break;
+            }
+        }
+        __threadfence();
+    }
+    return __syncthreads_or(static_cast<int>(bad)) == 0;
+}
+
+// All passes of the sort in one cooperative launch, block b on a contiguous
+// run of the kItems-key tiles. What bounds these sizes is not the keys' traffic
+// but the chain of launches (histogram, three of a scan, scatter: 30 us a pass
+// at 100k keys), and most passes move nothing: a sweep first finds the bits in
+// which the keys differ, and a digit that is the same in all of them is left
+// out. Each block adds up the other blocks' histograms itself, so a pass has
+// two barriers. The result is put in buffer `out`.
+__global__ void __launch_bounds__(kSortThreads, 1)
+  k_sort_resident(uint64_t* k0, uint64_t* k1, uint32_t* v0, uint32_t* v1, uint32_t n, int bits,
+                  uint32_t tiles, uint32_t* hist, SortControl* ctl, int out) {
+    __shared__ uint32_t wcnt[kSortWarps][kDigits];  // also the partial sums of the offsets
+    __shared__ uint32_t base[kDigits];
+    __shared__ uint32_t wsum[kDigits / 32];
+    uint32_t const t = threadIdx.x, lane = t & 31u, warp = t >> 5, b = blockIdx.x, nb = gridDim.x;
+    size_t const lo = static_cast<size_t>(static_cast<uint64_t>(tiles) * b / nb) * kItems;
+    size_t const end = static_cast<size_t>(static_cast<uint64_t>(tiles) * (b + 1) / nb) * kItems;
+    size_t const hi = end < n ? end : n;
+    uint64_t any = 0, any_not = 0;
+    for (size_t e = lo + t; e < hi; e += kSortThreads) {
+        uint64_t const k = __ldcg(k0 + e);
+        any |= k;
+        any_not |= ~k;
+    }
+    for (int d = 16; d; d >>= 1) {
+        any |= __shfl_xor_sync(0xffffffffu, any, d);
+        any_not |= __shfl_xor_sync(0xffffffffu, any_not, d);
+    }
+    if (lane == 0) {
+        if (any) atomicOr(&ctl->any, static_cast<unsigned long long>(any));
+        if (any_not) atomicOr(&ctl->any_not, static_cast<unsigned long long>(any_not));
+    }
+    uint32_t target = nb;
+    if (!sort_barrier(ctl, target)) return;
+    uint64_t const differ = __ldcg(&ctl->any) & __ldcg(&ctl->any_not);
+    int cur = 0;
+    for (int shift = 0; shift < bits; shift += 8) {
+        if (((differ >> shift) & 0xffu) == 0) continue;
+        uint64_t const* const kin = cur ? k1 : k0;
+        uint32_t const* const vin = cur ? v1 : v0;
+        uint64_t* const kout = cur ? k0 : k1;
+        uint32_t* const vout = cur ? v0 : v1;
+        if (t < kDigits) base[t] = 0;
+        __syncthreads();
+        for (size_t e = lo + t; e < hi; e += kSortThreads) {
+            atomicAdd(&base[(__ldcg(kin + e) >> shift) & 0xffu], 1u);
+        }
+        __syncthreads();
+        if (t < kDigits) __stcg(hist + static_cast<size_t>(b) * kDigits + t, base[t]);
+        target += nb;
+        if (!sort_barrier(ctl, target)) return;
+        // digit d over all blocks, and over the blocks before this one
+        {
+            uint32_t const d = t % kDigits, part = t / kDigits, parts = kSortThreads / kDigits;
+            uint32_t total = 0, before = 0;
+#pragma unroll 8
+            for (uint32_t q = part; q < nb; q += parts) {
+                uint32_t const c = __ldcg(hist + static_cast<size_t>(q) * kDigits + d);
+                total += c;
+                before += q < b ? c : 0u;
+            }
+            wcnt[2 * part][d] = total;
+            wcnt[2 * part + 1][d] = before;
+        }
+        __syncthreads();
+        uint32_t total = 0, before = 0, run = 0;
+        if (t < kDigits) {
+            for (int part = 0; part < kSortThreads / kDigits; ++part) {
+                total += wcnt[2 * part][t];
+                before += wcnt[2 * part + 1][t];
+            }
+            run = total;
+            for (uint32_t d = 1; d < 32; d <<= 1) {
+                uint32_t const o = __shfl_up_sync(0xffffffffu, run, d);
+                if (lane >= d) run += o;
+            }
+            if (lane == 31) wsum[warp] = run;
+        }
+        __syncthreads();
+        if (t < kDigits) {
+            uint32_t first = run - total + before;
+            for (uint32_t w = 0; w < warp; ++w) first += wsum[w];
+            base[t] = first;
+        }
+        for (size_t e0 = lo; e0 < hi; e0 += kSortThreads) {
+            __syncthreads();
+            for (uint32_t q = t; q < kSortWarps * kDigits; q += kSortThreads) (&wcnt[0][0])[q] = 0;
+            __syncthreads();
+            size_t const e = e0 + t;
+            bool const live = e < hi;
+            uint64_t const key = live ? __ldcg(kin + e) : 0ull;
+            uint32_t const val = live ? __ldcg(vin + e) : 0u;
+            uint32_t const dg = live ? static_cast<uint32_t>((key >> shift) & 0xffu) : 0xffffffffu;
+            uint32_t const peers = __match_any_sync(0xffffffffu, dg);
+            uint32_t const rank = __popc(peers & ((1u << lane) - 1u));
+            if (live && rank == 0) wcnt[warp][dg] = __popc(peers);
+            __syncthreads();
+            if (t < kDigits) {
+                uint32_t at = base[t];
+#pragma unroll 8
+                for (int w = 0; w < kSortWarps; ++w) {
+                    uint32_t const c = wcnt[w][t];
+                    wcnt[w][t] = at;
+                    at += c;
+                }
+                base[t] = at;
+            }
+            __syncthreads();
+            if (live) {
+                uint32_t const pos = wcnt[warp][dg] + rank;
+                __stcg(kout + pos, key);
+                __stcg(vout + pos, val);
+            }
+        }
+        target += nb;
+        if (!sort_barrier(ctl, target)) return;
+        cur ^= 1;
+    }
+    if (cur != out) {
+        for (size_t e = lo + t; e < hi; e += kSortThreads) {
+            __stcg((out ? k1 : k0) + e, __ldcg((cur ? k1 : k0) + e));
+            __stcg((out ? v1 : v0) + e, __ldcg((cur ? v1 : v0) + e));
+        }
     }
 }
 
@@ -186,9 +348,51 @@ void sort_scratch_carve(void* base, uint32_t n, SortScratch& s) {
     carve(static_cast<char*>(base), n, &s);
 }
 
+// Keys up to which the passes run in one launch. A pass of a few hundred tiles
+// costs the chain of launches about 30 us whatever its size, the resident sort
+// 17 us at 100k keys and 23 us at 300k, but 43 us to 35 us at 1M, where the
+// chain has more warps in flight: keys of few digits, which all differ, change
+// over at 2^19. Of 64-bit keys some digits are the same in all keys as a rule,
+// and those passes are left out: a pair sort (index, then z) takes 450 -> 114
+// us at 100k, 527 -> 261 us at 1M and 1232 -> 754 us at 4M pairs. At 2^22 it
+// still breaks even when all of z's digits differ.
+constexpr uint32_t kResidentKeysShort = 1u << 19;
+constexpr uint32_t kResidentKeysLong = 1u << 22;
+
+static bool launch_sort_resident(SortScratch& s, uint32_t n, int bits, int out, cudaStream_t st) {
+    int dev = 0, coop = 0, sms = 0;
+    if (n > (bits > 40 ? kResidentKeysLong : kResidentKeysShort) ||
+        cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    uint32_t const tiles = (n + kItems - 1) / kItems;
+    uint32_t const blocks = std::min<uint32_t>(tiles, static_cast<uint32_t>(sms));
+    SortControl* const ctl = reinterpret_cast<SortControl*>(s.scan);
+    cudaMemsetAsync(ctl, 0, sizeof(SortControl), st);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(kSortThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeCooperative;
+    at.val.cooperative = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, k_sort_resident, s.keys[0], s.keys[1], s.vals[0], s.vals[1], n,
+                           bits, tiles, s.hist, ctl, out) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return true;
+}
+
 int launch_radix_sort(SortScratch& s, uint32_t n, int bits, cudaStream_t st) {
     int cur = 0;
     if (n <= 1) return cur;
+    if (launch_sort_resident(s, n, bits, ((bits + 7) / 8) & 1, st)) return ((bits + 7) / 8) & 1;
     uint32_t const nb = (n + kItems - 1) / kItems;
     uint32_t* offsets = s.hist + static_cast<size_t>(kDigits) * nb;
     for (int shift = 0; shift < bits; shift += 8) {
