@@ -14,6 +14,7 @@
 // order them first).
 #include "engine_types.cuh"
 #include "kernels.cuh"
+#include "short_list.cuh"
 #include "sph_math.cuh"
 
 namespace emerald {
@@ -225,10 +226,8 @@ __global__ void k_sort_cells(uint32_t const* count,
     }
 }
 
-// The fast path of the search: a particle with at most kShortList accepted
-// candidates, kSearchBatch of a row's candidates in flight together (a row
+// kSearchBatch of a row's candidates in flight together (a row
 // holds about twelve at one particle per support squared).
-constexpr int kShortList = 16;
 constexpr int kSearchBatch = 6;
 
 // The first members and the counts of the nine cells around (gx, gy), in the
@@ -334,69 +333,25 @@ __device__ __forceinline__ int search_row(OtherSet const& o, float2 pos, uint32_
     return cnt;
 }
 
-// The order of the cnt <= kShortList listed candidates by (distance, index):
-// list position of the k-th in bits 4k..4k+3. Batcher's odd-even merge sort
-// (K. Batcher, "Sorting networks and their applications", 1968) in registers,
-// the same instructions in every lane whatever the counts, where an insertion
-// sort costs a warp the longest of its lanes' moves at every candidate. The
-// keys are the distances with their last four bits replaced by the list
-// position; where two keys differ in nothing else, the exact distances and the
-// indices decide afterwards.
+// The order of the cnt <= kShortList listed candidates by (distance, index).
 template <bool BY_PLACE>
 __device__ __forceinline__ uint64_t sort_short_list(OtherSet const& o, ShortList const& list,
                                                     int cnt) {
     uint32_t d[kShortList];
 #pragma unroll
     for (int q = 0; q < kShortList; ++q) {
-        // no distance has these bits, and no two of them the same upper ones
-        d[q] = 0xffffff00u + 17u * q;
+        d[q] = unused_key(q);
         if (q < cnt) {
             float const vx = list.x[q * kTile], vy = list.y[q * kTile];
             d[q] = (__float_as_uint(sqrtf(vx * vx + vy * vy)) & ~15u) | q;
             if (BY_PLACE) list.who[q * kTile] = o.members[list.who[q * kTile]];
         }
     }
-    constexpr int kSpan[10] = {1, 2, 2, 4, 4, 4, 8, 8, 8, 8};
-    constexpr int kStep[10] = {1, 2, 1, 4, 2, 1, 8, 4, 2, 1};
-#pragma unroll
-    for (int t = 0; t < 10; ++t) {
-        int const span = kSpan[t], k = kStep[t];
-#pragma unroll
-        for (int lo = 0; lo < kShortList; ++lo) {
-            int const hi = lo + k;
-            bool const pair = hi < kShortList && lo >= k % span &&
-                              (lo - k % span) % (2 * k) < k && lo / (2 * span) == hi / (2 * span);
-            if (pair) {
-                uint32_t const dl = min(d[lo], d[hi]);
-                d[hi] = max(d[lo], d[hi]);
-                d[lo] = dl;
-            }
-        }
-    }
-    bool tie = false;
-#pragma unroll
-    for (int q = 1; q < kShortList; ++q) tie = tie || (d[q] ^ d[q - 1]) < 16u;
-    uint32_t half[2] = {0u, 0u};
-#pragma unroll
-    for (int q = 0; q < kShortList; ++q) half[q / 8] |= (d[q] & 15u) << (4 * (q % 8));
-    uint64_t order = (static_cast<uint64_t>(half[1]) << 32) | half[0];
-    if (tie) {
-        auto key = [&](int k) {
-            uint32_t const at = (static_cast<uint32_t>(order >> (4 * k)) & 15u) * kTile;
-            float const dist = sqrtf(list.x[at] * list.x[at] + list.y[at] * list.y[at]);
-            return (static_cast<uint64_t>(__float_as_uint(dist)) << 32) |
-                   original_index(o, list.who[at]);
-        };
-#pragma unroll 1
-        for (int k = 1; k < cnt; ++k) {
-#pragma unroll 1
-            for (int q = k; q > 0 && key(q) < key(q - 1); --q) {
-                uint64_t const diff = ((order >> (4 * q)) ^ (order >> (4 * q - 4))) & 15u;
-                order ^= (diff << (4 * q)) | (diff << (4 * q - 4));
-            }
-        }
-    }
-    return order;
+    return order_short_list(d, cnt, [&](int q) {
+        uint32_t const at = static_cast<uint32_t>(q) * kTile;
+        float const dist = sqrtf(list.x[at] * list.x[at] + list.y[at] * list.y[at]);
+        return ShortKey{__float_as_uint(dist), original_index(o, list.who[at])};
+    });
 }
 
 // Writes list entry k of particle i: index, W and GradW(-vector_to)
