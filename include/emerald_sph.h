@@ -306,7 +306,8 @@ int emerald_sim_kernel_times(emerald_sim* sim, char* names, size_t names_len, do
 /* Execution mode: graphs != 0 (default) runs each sub-step as one CUDA graph
  * launch with the solver loops as conditional nodes; graphs == 0 launches
  * kernels one by one and tests the loop exit on the host after every
- * iteration, as the reference does. */
+ * iteration, as the reference does. Where a scene's solve fits on the chip it
+ * is one kernel, its loops included, in both modes. */
 int emerald_sim_set_graphs(emerald_sim* sim, int32_t graphs);
 
 /* Kernels this simulation has launched (graph nodes included, loop bodies
@@ -404,7 +405,8 @@ int emerald_sim_autotune(emerald_sim* sim, int32_t method, emerald_tuning* out);
 int emerald_batch_autotune(emerald_batch* batch, int32_t method, emerald_tuning* out);
 /* Pins the settings of *tuning (its chunks and prefetch modes; the candidate
  * fields are ignored) until the next call; NULL returns to the tuned or
- * default settings. */
+ * default settings. Pinned settings are those of the kernel-per-phase solve,
+ * which then runs whatever the scene's size. */
 int emerald_sim_set_tuning(emerald_sim* sim, emerald_tuning const* tuning);
 int emerald_batch_set_tuning(emerald_batch* batch, emerald_tuning const* tuning);
 
