@@ -31,6 +31,17 @@ constexpr uint32_t kMinShare = 4;
 // holds the lists of: 12.5 rows of 320 bytes a tile (11 neighbours a particle,
 // the longest list of 32).
 constexpr uint32_t kHeldTiles = 56;
+// Between re-sorts of the storage a violent flow mixes the particles, and a
+// share's halo grows: the exchanges with it, and in the end it has no room. The
+// lists of a share above kTightShare tiles leave little of it, so those scenes
+// report the largest halo of their shares (256ths of the share, 0xffff when a
+// gang took the plain form), and above kDrifted they take the kernels per phase
+// until the storage is in order again. 262k DFSPH particles, a sub-step
+// resident against per phase: halo 63-67 (calm) 0.56-0.62 against 0.62-0.89 ms,
+// 78 1.08 and 0.92-0.98, 93-104 0.97-1.18 and 0.96-1.05, plain form 1.2-2.2 and
+// 1.0-1.3. At 8 tiles a share the resident solve stays ahead throughout.
+constexpr uint32_t kTightShare = 24;
+constexpr uint32_t kDrifted = 84;
 // Batches of fewer warp tiles (2,048 particles) keep the launch-per-phase
 // kernels. The resident solve is the faster one there too (48 requests of 128
 // to 512 particles through one lane: 17.5 against 20.4 ms on B200), but a
@@ -310,7 +321,7 @@ Engine::Engine(uint32_t fluid_capacity, uint32_t solid_capacity, int max_scenes)
     cudaMemset(a_.loop_wt0, 0, 4);
     a_.batch = max_scenes_ > 1 ? 1 : 0;
     a_.gangs = static_cast<GangState*>(dev(sizeof(GangState) * max_scenes_));
-    a_.gang_ticket = static_cast<uint32_t*>(dev(4));
+    a_.gang_ticket = static_cast<uint32_t*>(dev(8));
     d_nparts_ = static_cast<uint32_t*>(dev(4));
     parts_cap_ = max_parts(fluid_cap_, max_scenes_);
     d_parts_ = static_cast<GangPart*>(dev(sizeof(GangPart) * parts_cap_));
@@ -1184,8 +1195,9 @@ int Engine::frame(int id, int32_t method, SceneState& out) {
         } while (out.remaining > 0 && n < 100000);
         return n;
     }
-    prepare_substep(method);
     bool const reorder = reorder_every_ > 0 && (frames_launched_ % 2) == 0;
+    if (reorder) storage_in_order();
+    prepare_substep(method);
     ++frames_launched_;
     int const key = graph_key(method, reorder);
     auto it = frame_graphs_.find(key);
@@ -1281,7 +1293,7 @@ bool Engine::use_resident(int32_t method) {
     ResidentLimits const& lim = limits_of(method);
     if (!lim.blocks) return false;
     if (!parts_valid_) divide_scenes(lim.blocks);
-    if (max_scenes_ == 1) return largest_share_ <= lim.share;
+    if (max_scenes_ == 1) return largest_share_ <= lim.share && !(drifted_ && watch_drift_);
     return total_tiles_ >= kMinBatchTiles && largest_share_ <= std::min(kHeldTiles, lim.share);
 }
 
@@ -1320,6 +1332,7 @@ void Engine::divide_scenes(uint32_t blocks) {
             largest_share_ = std::max(largest_share_, e - b);
         }
     }
+    watch_drift_ = max_scenes_ == 1 && largest_share_ > kTightShare;
     if (parts_.size() > parts_cap_) throw std::runtime_error("resident solve: too many shares");
     uint32_t const n = uint32_t(parts_.size());
     cudaMemcpyAsync(d_parts_, parts_.data(), sizeof(GangPart) * n, cudaMemcpyHostToDevice, st_);
@@ -1348,10 +1361,21 @@ void Engine::plan_resident(int32_t method) {
     now = p;
 }
 
+// The storage is about to be put in order: a scene that had drifted gets
+// another chance, the later the more often it has drifted in a row.
+void Engine::storage_in_order() {
+    if (!drifted_) {
+        retry_wait_ = 0;
+    } else if (retry_in_-- <= 0) {
+        drifted_ = false;
+    }
+}
+
 void Engine::substep(int32_t method) {
     if (active_scenes() == 0) return;
-    prepare_substep(method);
     bool const reorder = reorder_every_ > 0 && (substeps_launched_ % reorder_every_) == 0;
+    if (reorder) storage_in_order();
+    prepare_substep(method);
     ++substeps_launched_;
     if (use_graphs_ && !timing_ && !has_force_callbacks()) {
         int const key = graph_key(method, reorder);
@@ -1550,9 +1574,19 @@ void Engine::set_tuning(Tuning const* t) {
 
 SceneState Engine::scene_state(int id) {
     SceneState s{};
+    uint32_t drift = 0;
     cudaMemcpyAsync(&s, d_ss_ + id, sizeof(SceneState), cudaMemcpyDeviceToHost, st_);
+    if (watch_drift_) {
+        cudaMemcpyAsync(&drift, a_.gang_ticket + 1, 4, cudaMemcpyDeviceToHost, st_);
+        cudaMemsetAsync(a_.gang_ticket + 1, 0, 4, st_);
+    }
     host_wait(st_);
     check("scene_state");
+    if (watch_drift_ && drift > kDrifted) {
+        drifted_ = true;
+        retry_wait_ = std::min(2 * retry_wait_ + 1, 31);
+        retry_in_ = retry_wait_;
+    }
     if (s.error & kErrStalled) throw std::runtime_error("resident solve: a barrier gave up");
     return s;
 }

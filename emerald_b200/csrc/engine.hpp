@@ -266,6 +266,11 @@ private:
     std::vector<GangPart> parts_;
     bool parts_valid_ = false;  // false: the scenes changed since parts_ was made
     uint32_t largest_share_ = 1;
+    void storage_in_order();
+    bool watch_drift_ = false;  // the share is large enough for drift to matter
+    bool drifted_ = false;      // kernels per phase until storage is in order again
+    int retry_wait_ = 0;        // re-sorts to let pass after the next drift
+    int retry_in_ = 0;
     uint64_t total_tiles_ = 0;
     GangPart* d_parts_ = nullptr;
     uint32_t* d_nparts_ = nullptr;

@@ -155,7 +155,7 @@ struct Arena {
     // resident solve: per-scene gang states, the next share to take, and the
     // shares' error records (two each)
     GangState* gangs;
-    uint32_t* gang_ticket;
+    uint32_t* gang_ticket;  // and, after it, the largest drift reported since the host last looked
     GangRecord* records;
     int32_t batch;  // the arena holds more than one scene slot (loop kernels walk the work list)
     int32_t const* tile_scene;   // fluid tile -> scene (-1: free)

@@ -549,7 +549,12 @@ __device__ __forceinline__ void stage_lists(Arena const& a, Layout const& l, Sha
         }
     });
     block_sync();
-    if (threadIdx.x == 0) s.halo_n = min(s.halo_n, l.halo_max);
+    if (threadIdx.x == 0) {
+        s.halo_n = min(s.halo_n, l.halo_max);
+        // how far the storage order has drifted, for the host's choice of path
+        uint32_t const drift = s.plain ? 0xffffu : s.halo_n * 256u / max(sh.own(), 1u);
+        atomicMax(a.gang_ticket + 1, drift);
+    }
 }
 
 // ---------------------------------------------------------------- barriers
