@@ -575,6 +575,12 @@ struct KernelDivisors {
         if (inner) d = d + quotient(2.25f * r * r, hhh, y_hhh);
         w = quotient(inner ? 1.0f + q * q * (q * 0.75f - 1.5f) : (t * t * t) / 4.0f, k, y_k);
         dw = quotient(d, k, y_k);
+        // past the support; a distance in a list is below 2 h or a NaN, which
+        // counts as outside, as in kernel_w_dw
+        if (!(q <= 2.0f)) {
+            w = 0.0f;
+            dw = 0.0f;
+        }
     }
 };
 
