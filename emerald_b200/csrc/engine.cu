@@ -94,7 +94,7 @@ cudaError_t launch_resident_solve(Arena const& a, ResidentPlan const& p, int met
 }
 #undef EMLD_RESIDENT
 
-// Shares a plan of the resident solve has at most: a scene's last share may
+// Shares a plan of the resident solve has at most: one share of a scene may
 // be smaller than kMinShare tiles.
 uint32_t max_parts(uint32_t fluid_capacity, int max_scenes) {
     return fluid_capacity / 32 / kMinShare + uint32_t(max_scenes);
@@ -1311,7 +1311,7 @@ void Engine::divide_scenes(uint32_t blocks) {
     uint64_t total = 0;
     for (int id = 0; id < max_scenes_; ++id) {
         Scene const& sc = scenes_[id];
-        if (!sc.used || !sc.active || sc.p.fluid_count == 0) continue;
+        if (!sc.used || !sc.active) continue;
         items.push_back({(sc.p.fluid_count + 31u) / 32u, id});
         total += items.back().tiles;
     }
@@ -1323,7 +1323,9 @@ void Engine::divide_scenes(uint32_t blocks) {
     parts_.clear();
     largest_share_ = 1;
     for (Item const& it : items) {
-        uint32_t const size = std::min(blocks, (it.tiles + quota - 1) / quota);
+        // (a scene without particles still has loops, and their statistics)
+        uint32_t const size =
+          std::max<uint32_t>(1, std::min(blocks, (it.tiles + quota - 1) / quota));
         uint32_t const base = uint32_t(parts_.size());
         for (uint32_t r = 0; r < size; ++r) {
             uint32_t const b = uint32_t(uint64_t(it.tiles) * r / size);

@@ -1,0 +1,65 @@
+"""The resident solve where a scene or a call is out of the ordinary, against
+the launch-per-phase kernels, which a pinned tuning selects: the same bits and
+the same statistics."""
+import numpy as np
+import pytest
+
+from conftest import assert_bitwise
+from scenes import F
+from test_gpu_resident import ARRAYS, METHODS, PINNED, scene
+
+pytestmark = pytest.mark.gpu
+
+STATS = ("pressure_iterations", "divergence_iterations", "error_average", "error_max",
+         "divergence_error_average", "divergence_error_max", "error_average_exact",
+         "divergence_error_average_exact", "dt", "error_flags")
+
+
+@pytest.fixture(scope="module")
+def E():
+    import emerald_b200
+    return emerald_b200
+
+
+def empty(E):
+    sc = scene(E, 8, 4)
+    return sc, np.zeros((0, 2), np.float32)
+
+
+@pytest.mark.parametrize("method", METHODS)
+def test_scene_without_particles_reports_its_loops(E, method):
+    """A loop over no particles runs until its exit test passes, and the
+    statistics say so."""
+    sc, none = empty(E)
+    a = E.Simulation(sc.params, sc.solid, none, None, sc.solid_volumes)
+    b = E.Simulation(sc.params, sc.solid, none, None, sc.solid_volumes)
+    b.set_tuning(PINNED)
+    sa, sb = a.advance(method, 2), b.advance(method, 2)
+    assert sb["pressure_iterations"] > 0
+    for key in STATS:
+        assert sa[key] == sb[key], (key, sa[key], sb[key])
+
+
+@pytest.mark.parametrize("method", ("dfsph_p", "iisph"))
+def test_batch_with_a_scene_without_particles(E, method):
+    sc, none = empty(E)
+    big = scene(E, 70, 60)
+    got = []
+    for pinned in (False, True):
+        b = E.Batch(8192, 4096, 4)
+        if pinned:
+            b.set_tuning(PINNED)
+        ids = [b.add_scene(sc.params, sc.solid, none, None, sc.solid_volumes),
+               b.add_block_scene(big)]
+        b.step(method, 2)
+        got.append(([b.stats(k) for k in ids], b.state(ids[1])))
+        b.close()
+    for sa, sb in zip(got[0][0], got[1][0]):
+        for key in STATS:
+            if key.endswith("exact"):
+                # summed in double, in another order
+                assert abs(sa[key] - sb[key]) <= 1e-12 * max(1.0, abs(sb[key])), key
+            else:
+                assert sa[key] == sb[key], (key, sa[key], sb[key])
+    for x, y in zip(got[0][1], got[1][1]):
+        assert_bitwise(x, y, method)
