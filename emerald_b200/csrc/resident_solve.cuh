@@ -902,6 +902,16 @@ __device__ __forceinline__ void report_exact(Arena const& a, Share& sh, Shared& 
     }
 }
 
+// Before a pressure loop whose coefficients read neighbours' velocities from
+// the arena: the loop's first exchange comes after those reads in every block,
+// and the velocities are overwritten after the loop. A loop that runs no
+// iteration has no exchange, so the gang waits here instead.
+__device__ __forceinline__ bool start_loop(Arena const& a, Shared& s) {
+    if (iteration_cap(s.P, 0) <= 0) return gang_sync(a, s);
+    block_sync();
+    return true;
+}
+
 // One solver loop of the reference: body(iter) runs an iteration, during which
 // the exit test's warp sets s.ends, and ends in a block barrier. Returns the
 // iterations run, or -1 when a wait gave up.
@@ -1159,7 +1169,7 @@ __device__ __forceinline__ bool solve_iisph(Arena const& a, Layout const& l, Sha
         a.aii[i] = aii;
         a.rho_star[i] = star;
     });
-    block_sync();
+    if (!start_loop(a, s)) return false;
     if (keeps_exit()) {
         uint32_t slot = 0u;
         if (attend_loop(a, sh, s, 0, false, slot) < 0) return false;
@@ -1304,7 +1314,7 @@ __device__ __forceinline__ bool solve_iisph_ap(Arena const& a, Layout const& l, 
         a.aii[i] = aii;
         a.rho_star[i] = star;
     });
-    block_sync();
+    if (!start_loop(a, s)) return false;
     if (keeps_exit()) {
         uint32_t slot = 0u;
         return attend_loop(a, sh, s, 0, false, slot) >= 0;

@@ -63,3 +63,30 @@ def test_batch_with_a_scene_without_particles(E, method):
                 assert sa[key] == sb[key], (key, sa[key], sb[key])
     for x, y in zip(got[0][1], got[1][1]):
         assert_bitwise(x, y, method)
+
+
+@pytest.mark.parametrize("method", METHODS)
+@pytest.mark.parametrize("nx,ny,ratio", [(300, 241, 1.0), (60, 50, 2.0), (60, 50, 2.6),
+                                         (150, 130, 2.6)])
+def test_no_iterations_at_all(E, method, nx, ny, ratio):
+    """Loops capped at none, with many blocks and in the barrier form (lists
+    cut at 64): no exchange orders the blocks, so what a block reads of its
+    neighbours' velocities has to come before they integrate."""
+    sc = scene(E, nx, ny, support_ratio=ratio, dfsph_max_correction_iterations=0,
+               iisph_max_pressure_iterations=0)
+    # (what only an iteration writes is left out)
+    arrays = [name for name in ARRAYS[method]
+              if (method, name) not in (("dfsph_p", "density_stars"), ("iisph", "sum_dij_pjs"))]
+    b = E.Simulation.from_block_scene(sc)
+    b.set_tuning(PINNED)
+    b.advance(method, 2)
+    want = [b.array(name) for name in arrays], b.state()
+    for _ in range(4):
+        a = E.Simulation.from_block_scene(sc)
+        a.advance(method, 2)
+        for name, x, y in zip("xv", a.state(), want[1]):
+            assert_bitwise(x, y, "%s %s" % (method, name))
+        for name, y in zip(arrays, want[0]):
+            assert_bitwise(a.array(name), y, "%s %s" % (method, name))
+        a.close()
+    b.close()
