@@ -344,6 +344,14 @@ Engine::Engine(uint32_t fluid_capacity, uint32_t solid_capacity, int max_scenes)
     cudaMemset(a_.ns_cnt, 0, N);
     cudaMemset(a_.kdiv, 0, 4 * N);
     cudaMemset(a_.kdens, 0, 4 * N);
+    // what the accessors may be asked for before a sub-step has written it (a
+    // loop of no iterations writes no error density, say)
+    for (float* p : {a_.rho, a_.rho_star, a_.pbuf0, a_.pbuf1, a_.alpha, a_.aii}) {
+        cudaMemset(p, 0, 4 * N);
+    }
+    for (float2* p : {a_.dii, a_.sdp, a_.acc, a_.vext, a_.xstar, a_.vstar, a_.fp}) {
+        cudaMemset(p, 0, 8 * N);
+    }
     scenes_.resize(max_scenes_);
     tile_scene_.assign(N / kTile, -1);
     stile_scene_.assign(S / kTile, -1);

@@ -90,3 +90,25 @@ def test_no_iterations_at_all(E, method, nx, ny, ratio):
             assert_bitwise(a.array(name), y, "%s %s" % (method, name))
         a.close()
     b.close()
+
+
+@pytest.mark.parametrize("method", METHODS)
+def test_arrays_nothing_has_written_are_zero(E, method):
+    """Also where the device memory held something else before."""
+    used = [E.Simulation.from_block_scene(scene(E, 60 + d, 50)) for d in range(8)]
+    for sim in used:
+        for m in METHODS:
+            sim.advance(m, 1, stats=False)
+    for sim in used[::2]:
+        sim.close()
+    sc = scene(E, 60, 50, dfsph_max_correction_iterations=0, iisph_max_pressure_iterations=0)
+    sim = E.Simulation.from_block_scene(sc)
+    fresh = E.Simulation.from_block_scene(sc)
+    for name in ARRAYS[method]:
+        if name != "pressures":                    # of the method the scene runs
+            assert not fresh.array(name).any(), name
+    sim.advance(method, 1)
+    if method == "iisph":
+        assert not sim.array("sum_dij_pjs").any()
+    if method == "dfsph_p":
+        assert not sim.array("density_stars").any()
