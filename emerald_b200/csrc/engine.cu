@@ -322,6 +322,7 @@ Engine::Engine(uint32_t fluid_capacity, uint32_t solid_capacity, int max_scenes)
     a_.batch = max_scenes_ > 1 ? 1 : 0;
     a_.gangs = static_cast<GangState*>(dev(sizeof(GangState) * max_scenes_));
     a_.gang_ticket = static_cast<uint32_t*>(dev(8));
+    cudaMemset(a_.gang_ticket, 0, 8);
     d_nparts_ = static_cast<uint32_t*>(dev(4));
     parts_cap_ = max_parts(fluid_cap_, max_scenes_);
     d_parts_ = static_cast<GangPart*>(dev(sizeof(GangPart) * parts_cap_));
@@ -483,6 +484,14 @@ void Engine::upload_params(int id) {
     cudaMemcpyAsync(d_sp_ + id, &scenes_[id].p, sizeof(SceneParams), cudaMemcpyHostToDevice, st_);
 }
 
+// The scenes or their positions are new: what was known of the storage order's
+// drift is not theirs.
+void Engine::forget_drift() {
+    cudaMemsetAsync(a_.gang_ticket + 1, 0, 4, st_);
+    drifted_ = false;
+    retry_wait_ = retry_in_ = 0;
+}
+
 int Engine::add_scene(SceneSpec const& spec) {
     int id = -1;
     for (int k = 0; k < max_scenes_; ++k) {
@@ -603,6 +612,7 @@ int Engine::add_scene(SceneSpec const& spec) {
     }
     update_sort_bases();
     update_extent();
+    forget_drift();
     rebuild_solids();
     if (spec.n_solid) {
         if (spec.solid_volumes) {
@@ -736,6 +746,7 @@ void Engine::remove_scene(int id) {
     parts_valid_ = false;
     update_sort_bases();
     update_extent();
+    forget_drift();
     rebuild_solids();
 }
 
@@ -1648,6 +1659,7 @@ bool Engine::set_state(int id, float const* x, float const* v, bool sync) {
     if (x) {
         launch_scatter_f2(a_, b, n, a_.tx + b, a_.x, st_);
         launch_positions_to_double(a_, b, n, st_);
+        if (watch_drift_) forget_drift();
     }
     if (v) launch_scatter_f2(a_, b, n, a_.tv + b, a_.v, st_);
     if (sync) host_wait(st_);

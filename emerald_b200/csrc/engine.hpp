@@ -267,6 +267,7 @@ private:
     bool parts_valid_ = false;  // false: the scenes changed since parts_ was made
     uint32_t largest_share_ = 1;
     void storage_in_order();
+    void forget_drift();
     bool watch_drift_ = false;  // the share is large enough for drift to matter
     bool drifted_ = false;      // kernels per phase until storage is in order again
     int retry_wait_ = 0;        // re-sorts to let pass after the next drift
