@@ -17,6 +17,8 @@ LIB_PATH = os.path.join(_HERE, "libemerald_b200.so")
 METHODS = {"pcisph": 0, "iisph": 1, "iisph_ap": 2, "iisph_pseudo_ap": 3, "dfsph_p": 4}
 PRECISION_REFERENCE = 0
 PRECISION_COMPENSATED = 1
+INJECT_BARRIER_POLLS = 0
+INJECT_VALUE_POLLS = 1
 FLICKS_PER_SECOND = 705600000
 
 c_f = ctypes.c_float
@@ -296,6 +298,8 @@ EXPORTS = {
     "emerald_iisph_pseudo_ap_integrate_velocities_and_positions_in_place": (
         c_i32, [c_sz, c_f, c_vp, c_vp, c_vp, c_vp]),
     "emerald_neighbors_static": (c_i32, [c_vp, c_u32, c_f, c_vp, c_vp, c_vp, c_vp, c_u32, c_vp]),
+    "emerald_sim_inject": (c_i32, [c_vp, c_i32, c_u32]),
+    "emerald_batch_inject": (c_i32, [c_vp, c_i32, c_u32]),
     "emerald_kernel_launches": (c_i64, []),
     "emerald_last_error": (ctypes.c_char_p, []),
 }
@@ -645,6 +649,10 @@ class Simulation:
         _check(lib.emerald_sim_set_tuning(self._h, None if t is None else ctypes.byref(t)),
                "set_tuning")
 
+    def inject(self, what, value):
+        """Fault injection for tests (INJECT_*)."""
+        _check(lib.emerald_sim_inject(self._h, what, value), "inject")
+
     def enable_timing(self, on=True):
         _check(lib.emerald_sim_enable_timing(self._h, int(on)), "enable_timing")
 
@@ -760,6 +768,10 @@ class Batch:
         n = c_i64()
         _check(lib.emerald_batch_kernel_launches(self._h, ctypes.byref(n)), "kernel_launches")
         return n.value
+
+    def inject(self, what, value):
+        """Fault injection for tests (INJECT_*)."""
+        _check(lib.emerald_batch_inject(self._h, what, value), "inject")
 
     def autotune(self, method):
         t = Tuning()

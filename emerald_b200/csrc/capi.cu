@@ -600,6 +600,7 @@ int emerald_batch_synchronize(emerald_batch* batch) {
     return guarded([&] {
         cudaStreamSynchronize(batch->engine.stream());
         batch->engine.check("synchronize");
+        batch->engine.check_solved(-1);
         return EMERALD_OK;
     });
 }
@@ -785,6 +786,29 @@ int emerald_sim_set_graphs(emerald_sim* sim, int32_t graphs) {
     if (!sim) return fail(EMERALD_EINVAL, "sim is NULL");
     sim->engine.set_graphs(graphs != 0);
     return EMERALD_OK;
+}
+
+namespace {
+int inject_into(Engine& engine, int32_t what, uint32_t value) {
+    return guarded([&] {
+        try {
+            engine.inject(what, value);
+        } catch (std::invalid_argument const& e) {
+            return fail(EMERALD_EINVAL, e.what());
+        }
+        return EMERALD_OK;
+    });
+}
+}  // namespace
+
+int emerald_sim_inject(emerald_sim* sim, int32_t what, uint32_t value) {
+    if (!sim) return fail(EMERALD_EINVAL, "sim is NULL");
+    return inject_into(sim->engine, what, value);
+}
+
+int emerald_batch_inject(emerald_batch* batch, int32_t what, uint32_t value) {
+    if (!batch) return fail(EMERALD_EINVAL, "batch is NULL");
+    return inject_into(batch->engine, what, value);
 }
 
 int emerald_sim_host_waits(emerald_sim* sim, int64_t* count) {

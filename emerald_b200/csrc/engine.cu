@@ -51,6 +51,11 @@ constexpr uint32_t kDrifted = 84;
 // tests require.
 constexpr uint32_t kMinBatchTiles = 64;
 
+// Polls of a wait of the resident solve before it gives up (seconds; a phase
+// takes microseconds).
+constexpr uint32_t kMaxPolls = 1u << 22;
+constexpr int kStallBits = kErrStalled | kErrUnsolved;
+
 // How many error sums s = 0, 1, ... pass the solvers' average test
 // float(double(s) / (1000 n)) <= threshold (a scene without particles has
 // average 0).
@@ -336,9 +341,13 @@ Engine::Engine(uint32_t fluid_capacity, uint32_t solid_capacity, int max_scenes)
         throw std::runtime_error("stream creation failed");
     }
     if (cudaMallocHost(reinterpret_cast<void**>(&h_running_), sizeof(int)) != cudaSuccess ||
-        cudaMallocHost(reinterpret_cast<void**>(&h_flag_), sizeof(uint32_t)) != cudaSuccess) {
+        cudaMallocHost(reinterpret_cast<void**>(&h_flag_), sizeof(uint32_t)) != cudaSuccess ||
+        cudaMallocHost(reinterpret_cast<void**>(&h_gave_up_), sizeof(uint32_t)) != cudaSuccess) {
         throw std::bad_alloc();
     }
+    *h_gave_up_ = 0u;
+    a_.gave_up = h_gave_up_;
+    a_.barrier_polls = a_.value_polls = kMaxPolls;
     cudaMemset(d_ss_, 0, sizeof(SceneState) * max_scenes_);
     cudaMemset(a_.vs, 0, 8 * S);
     cudaMemset(a_.nf_cnt, 0, N);
@@ -390,6 +399,7 @@ Engine::~Engine() {
     for (void* p : allocations_) cudaFree(p);
     if (h_running_) cudaFreeHost(h_running_);
     if (h_flag_) cudaFreeHost(h_flag_);
+    if (h_gave_up_) cudaFreeHost(h_gave_up_);
 }
 
 template <class F>
@@ -750,6 +760,31 @@ void Engine::remove_scene(int id) {
     rebuild_solids();
 }
 
+void Engine::inject(int what, uint32_t value) {
+    switch (what) {
+    case EMERALD_INJECT_BARRIER_POLLS: a_.barrier_polls = value; break;
+    case EMERALD_INJECT_VALUE_POLLS: a_.value_polls = value; break;
+    default: throw std::invalid_argument("unknown injection");
+    }
+    destroy_graphs();  // they hold the arena's values
+}
+
+// After a wait of a resident solve has given up (which the kernel tells the
+// host): throws where scene `id`, or with id < 0 an active scene, was not
+// solved to the end in some sub-step. Such a scene's particles are in no
+// defined state until it gets a new one.
+void Engine::check_solved(int id) {
+    if (!gave_up()) return;
+    std::vector<SceneState> const states = all_states();
+    bool bad = false;
+    for (int k = 0; k < max_scenes_; ++k) {
+        Scene const& sc = scenes_[k];
+        if (!sc.used || !(states[k].error & kStallBits)) continue;
+        bad = bad || (id < 0 ? sc.active : k == id);
+    }
+    if (bad) throw std::runtime_error("resident solve: a wait gave up; the scene needs a new state");
+}
+
 void Engine::set_active(int id, bool active) {
     if (!scene_used(id)) return;
     scenes_[id].active = active;
@@ -988,13 +1023,13 @@ void Engine::emit_substep(int32_t method, bool reorder) {
         launch("reorder", [&] { launch_reorder(a_, order_sort_, tiles * kTile, bits, st); },
                3 + 3 * (bits / 8));
     }
+    bool const resident = use_resident(method);
     auto begin = [&](cudaStream_t s) {
         launch("max_v2", [&] { launch_max_v2(a_, tiles, s); });
-        launch("begin_substep", [&] { launch_begin_substep(a_, max_scenes_, s); });
+        launch("begin_substep", [&] { launch_begin_substep(a_, max_scenes_, resident, s); });
     };
     Arena const ext = extent_arena();
     bool const kernels = method != kPcisph;
-    bool const resident = use_resident(method);
     // The sub-step's dt and the boundary lists need neither the fluid cells nor
     // the fluid lists, so they are made on a side stream (a parallel branch of
     // the graph) beside them; the per-kernel timing mode keeps everything on
@@ -1214,6 +1249,7 @@ int Engine::frame(int id, int32_t method, SceneState& out) {
         } while (out.remaining > 0 && n < 100000);
         return n;
     }
+    check_solved(-1);
     bool const reorder = reorder_every_ > 0 && (frames_launched_ % 2) == 0;
     if (reorder) storage_in_order();
     prepare_substep(method);
@@ -1394,6 +1430,7 @@ void Engine::storage_in_order() {
 
 void Engine::substep(int32_t method) {
     if (active_scenes() == 0) return;
+    check_solved(-1);
     bool const reorder = reorder_every_ > 0 && (substeps_launched_ % reorder_every_) == 0;
     if (reorder) storage_in_order();
     prepare_substep(method);
@@ -1608,7 +1645,7 @@ SceneState Engine::scene_state(int id) {
         retry_wait_ = std::min(2 * retry_wait_ + 1, 31);
         retry_in_ = retry_wait_;
     }
-    if (s.error & kErrStalled) throw std::runtime_error("resident solve: a barrier gave up");
+    check_solved(id);
     return s;
 }
 
@@ -1633,8 +1670,10 @@ void Engine::get_state(int id, float* x, float* v, bool sync) {
         launch_gather_f2(a_, b, n, a_.v, a_.tv + b, st_);
         cudaMemcpyAsync(v, a_.tv + b, 8ull * n, cudaMemcpyDeviceToHost, st_);
     }
-    if (sync) host_wait(st_);
+    if (!sync) return check("get_state");
+    host_wait(st_);
     check("get_state");
+    check_solved(id);
 }
 
 bool Engine::set_state(int id, float const* x, float const* v, bool sync) {
@@ -1662,6 +1701,7 @@ bool Engine::set_state(int id, float const* x, float const* v, bool sync) {
         if (watch_drift_) forget_drift();
     }
     if (v) launch_scatter_f2(a_, b, n, a_.tv + b, a_.v, st_);
+    if (x && v && gave_up()) launch_clear_stall(a_, id, st_);
     if (sync) host_wait(st_);
     check("set_state");
     return true;
@@ -1872,6 +1912,7 @@ bool Engine::get_array(int id, std::string const& name, float* out, int& width) 
         }
         host_wait(st_);
         check("get_array");
+        check_solved(id);
     }
     return true;
 }
@@ -1907,6 +1948,7 @@ void Engine::get_neighbors(int id, bool solid, uint8_t* counts, uint32_t* idx, f
     cudaMemcpyAsync(slot_of.data(), a_.slot_of + P.fluid_begin, 4ull * n, cudaMemcpyDeviceToHost, st_);
     host_wait(st_);
     check("get_neighbors");
+    check_solved(id);
     uint32_t const base = solid ? P.solid_begin : P.fluid_begin;
     for (uint32_t i = 0; i < n; ++i) {
         uint32_t const row = slot_of[i] - P.fluid_begin;  // storage column of particle i

@@ -153,7 +153,11 @@ public:
     void get_neighbors(int id, bool solid, uint8_t* counts, uint32_t* idx, float* w, float* gw);
     size_t get_sort(int id, bool solid, int32_t* gc, uint64_t* z, uint64_t* pair_z,
                     uint64_t* pair_index, uint32_t* block_indices, uint64_t* blocks);
+    // Throws where a sub-step of the scene was not solved to the end, as
+    // get_state (sync), get_array and get_neighbors do.
     SceneState scene_state(int id);
+    // Fault injection for tests (EMERALD_INJECT_*).
+    void inject(int what, uint32_t value);
     SceneParams const& scene_params(int id) const { return scenes_[id].p; }
     std::vector<SceneState> all_states();
     uint32_t fluid_count(int id) const { return scenes_[id].p.fluid_count; }
@@ -161,6 +165,7 @@ public:
     float2* device_x(int id) { return a_.x + scenes_[id].p.fluid_begin; }
     float2* device_v(int id) { return a_.v + scenes_[id].p.fluid_begin; }
     int active_scenes() const;
+    void check_solved(int id);
     size_t free_fluid() const { return size_t(fluid_tiles_.largest_free()) * kTile; }
     // Largest free runs of each arena region, for admission decisions made
     // away from the thread that owns the engine.
@@ -308,6 +313,8 @@ private:
     int* h_running_ = nullptr;
     uint32_t* d_flag_ = nullptr;
     uint32_t* h_flag_ = nullptr;
+    uint32_t* h_gave_up_ = nullptr;  // written by the resident solve
+    bool gave_up() const { return *reinterpret_cast<uint32_t volatile*>(h_gave_up_) != 0u; }
     unsigned int* d_check_counter_ = nullptr;  // finished blocks of a fused exit test
     int loop_kernels_[4] = {3, 3, 3, 4};        // kernels per iteration of each loop kind
     std::vector<Scene> scenes_;

@@ -29,8 +29,11 @@ enum Method : int { kPcisph = 0, kIisph = 1, kIisphAp = 2, kIisphPseudoAp = 3, k
 
 enum StepMode : int { kFixedDt = 0, kFrame = 1 };
 
-// Error bits reported through SceneState::error.
-enum ErrorBits : int { kErrTableFull = 1, kErrNonFinite = 2, kErrStalled = 4 };
+// Error bits reported through SceneState::error. kErrUnsolved is set while a
+// resident solve of the scene is due and cleared when all its shares are done;
+// what is left of it says that a wait gave up, and becomes kErrStalled at the
+// next sub-step. Either stays until the scene is given a new state.
+enum ErrorBits : int { kErrTableFull = 1, kErrNonFinite = 2, kErrStalled = 4, kErrUnsolved = 8 };
 
 // External force terms, the reference's force functions
 // (emerald/sph2d_box/forces.cpp): gravity (accumulate_gravity_forces,
@@ -114,11 +117,12 @@ struct SceneState {
 };
 
 // What the blocks that solve one scene together (its gang, see
-// resident_solve.cuh) share: arrivals at their barriers, and whether some
-// block needs the barrier form. Cleared by k_begin_substep.
+// resident_solve.cuh) share: arrivals at their barriers, whether some block
+// needs the barrier form, and the shares done. Cleared by k_begin_substep.
 struct alignas(64) GangState {
     uint32_t arrive;
     uint32_t plain;
+    uint32_t done;  // shares solved to the end
 };
 
 // A block's error sums of one solver iteration: 32 bits of value and the tag
@@ -157,6 +161,9 @@ struct Arena {
     GangState* gangs;
     uint32_t* gang_ticket;  // and, after it, the largest drift reported since the host last looked
     GangRecord* records;
+    uint32_t* gave_up;       // host memory: some wait of a resident solve has given up
+    uint32_t barrier_polls;  // polls of a barrier, and of a value, before it gives up
+    uint32_t value_polls;
     int32_t batch;  // the arena holds more than one scene slot (loop kernels walk the work list)
     int32_t const* tile_scene;   // fluid tile -> scene (-1: free)
     int32_t const* stile_scene;  // solid tile -> scene

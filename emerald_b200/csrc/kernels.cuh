@@ -64,6 +64,8 @@ void launch_scatter_d2(Arena const& a, uint32_t begin, uint32_t count, double2 c
                        double2* dst, cudaStream_t st);
 // *flag |= 1 when p[0, n) holds an infinity or a NaN.
 void launch_flag_nonfinite(float const* p, size_t n, uint32_t* flag, cudaStream_t st);
+// Clears a scene's stall bits (its state has been replaced).
+void launch_clear_stall(Arena const& a, int scene, cudaStream_t st);
 void launch_positions_to_double(Arena const& a, uint32_t begin, uint32_t count, cudaStream_t st);
 void launch_identity_order(Arena const& a, uint32_t begin, uint32_t count, cudaStream_t st);
 
@@ -74,7 +76,7 @@ void launch_max_v2(Arena const& a, uint32_t tiles, cudaStream_t st);
 void launch_frame_begin(Arena const& a, int nscenes, cudaStream_t st);
 void launch_frame_check(Arena const& a, int nscenes, int method, cudaGraphConditionalHandle cond,
                         cudaStream_t st);
-void launch_begin_substep(Arena const& a, int nscenes, cudaStream_t st);
+void launch_begin_substep(Arena const& a, int nscenes, bool resident, cudaStream_t st);
 void launch_zero_kappas(Arena const& a, uint32_t tiles, cudaStream_t st);
 // use_cond: also set `cond` (the loop's while condition) to 1
 void launch_iter_reset(Arena const& a, int nscenes, int kind, cudaStream_t st,

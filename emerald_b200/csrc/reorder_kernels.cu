@@ -124,6 +124,10 @@ __global__ void k_positions_to_double(Arena a, uint32_t begin, uint32_t count) {
     a.x64[begin + k] = make_double2(double(p.x), double(p.y));
 }
 
+__global__ void k_clear_stall(Arena a, int scene) {
+    atomicAnd(&a.ss[scene].error, ~(kErrStalled | kErrUnsolved));
+}
+
 __global__ void k_identity_order(Arena a, uint32_t begin, uint32_t count) {
     uint32_t const k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
@@ -169,6 +173,9 @@ void launch_flag_nonfinite(float const* p, size_t n, uint32_t* flag, cudaStream_
 }
 void launch_positions_to_double(Arena const& a, uint32_t begin, uint32_t count, cudaStream_t st) {
     if (count) k_positions_to_double<<<(count + 255) / 256, 256, 0, st>>>(a, begin, count);
+}
+void launch_clear_stall(Arena const& a, int scene, cudaStream_t st) {
+    k_clear_stall<<<1, 1, 0, st>>>(a, scene);
 }
 void launch_identity_order(Arena const& a, uint32_t begin, uint32_t count, cudaStream_t st) {
     if (count) k_identity_order<<<(count + 255) / 256, 256, 0, st>>>(a, begin, count);

@@ -60,8 +60,6 @@ constexpr uint32_t kBoundaryUnits = 2;   // rows of space per boundary row: 32 m
 constexpr uint32_t kMaxTiles = 256;      // warp tiles of a share at most
 constexpr uint32_t kNoKey = 0xffffffffu;
 constexpr uint32_t kFar = 0xffffu;       // a neighbour without a code
-// Barrier polls before a block gives up (seconds; a phase takes microseconds).
-constexpr uint32_t kMaxPolls = 1u << 22;
 
 // A particle's published values and the codes of its list that do not fit in
 // shared memory live in the upper half of its own column of the boundary lists
@@ -561,7 +559,7 @@ __device__ __forceinline__ void stage_lists(Arena const& a, Layout const& l, Sha
 
 // Waits until every block of the gang has arrived, making their writes before
 // it visible after it. Returns false when the others did not arrive within the
-// poll limit: the scene is flagged and the caller leaves.
+// poll limit (Arena::barrier_polls): the caller leaves.
 __device__ __forceinline__ bool gang_sync(Arena const& a, Shared& s) {
     block_sync();
     if (threadIdx.x == 0 && s.part.size > 1) {
@@ -574,7 +572,7 @@ __device__ __forceinline__ bool gang_sync(Arena const& a, Shared& s) {
         for (;;) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(arrive) : "memory");
             if (seen >= target) break;
-            if (++polls > kMaxPolls) {
+            if (++polls > a.barrier_polls) {
                 s.ok = 0;
                 break;
             }
@@ -689,9 +687,9 @@ __device__ __forceinline__ void receive(Arena const& a, Layout const& l, Share c
         T v;
         uint32_t polls = 0;
         while (!get_value(a, f, halo[h], sh.epoch, v)) {
-            if (++polls > kMaxPolls) {
+            if (++polls > a.value_polls) {
                 s.ok = 0;
-                break;
+                return;
             }
         }
         store(own + h, v);
@@ -788,8 +786,9 @@ __device__ __forceinline__ void post_errors(Arena const& a, Shared const& s, uin
 }
 
 // The two words from word k of a record, waited for until they carry the tag.
-__device__ __forceinline__ void record_words(GangRecord const* r, int k, uint32_t tag, Shared& s,
-                                             uint32_t& lo, uint32_t& hi) {
+__device__ __forceinline__ void record_words(Arena const& a, GangRecord const* r, int k,
+                                             uint32_t tag, Shared& s, uint32_t& lo,
+                                             uint32_t& hi) {
     unsigned long long w0, w1;
     uint32_t polls = 0;
     for (;;) {
@@ -798,7 +797,7 @@ __device__ __forceinline__ void record_words(GangRecord const* r, int k, uint32_
                      : "l"(r->w + k)
                      : "memory");
         if (word_tag(w0) == tag && word_tag(w1) == tag) break;
-        if (++polls > kMaxPolls) {
+        if (++polls > a.value_polls) {
             s.ok = 0;
             break;
         }
@@ -837,7 +836,7 @@ __device__ __forceinline__ void decide_exit(Arena const& a, Shared& s, int kind,
                 ready = ready && (k0 + u * 32u + lane >= size ||
                                   (word_tag(w0[u]) == tag && word_tag(w1[u]) == tag));
             }
-            if (++polls > kMaxPolls) {
+            if (++polls > a.value_polls) {
                 s.ok = 0;
                 break;
             }
@@ -850,7 +849,7 @@ __device__ __forceinline__ void decide_exit(Arena const& a, Shared& s, int kind,
             t.max = hi > t.max ? hi : t.max;
             unsigned long long sum = lo;
             if (lo == 0xffffffffu) {
-                record_words(record_of(a, s, k, slot), 2, tag, s, lo, hi);
+                record_words(a, record_of(a, s, k, slot), 2, tag, s, lo, hi);
                 sum = (static_cast<unsigned long long>(hi) << 32) | lo;
             }
             t.sum += sum;
@@ -890,9 +889,9 @@ __device__ __forceinline__ void report_exact(Arena const& a, Share& sh, Shared& 
     if (s.part.rank != 0) return;
     t = 0.0;
 #pragma unroll 1
-    for (uint32_t k = lane; k < s.part.size; k += 32u) {
+    for (uint32_t k = lane; k < s.part.size && s.ok; k += 32u) {
         uint32_t lo, hi;
-        record_words(record_of(a, s, k, slot), 4, sh.epoch, s, lo, hi);
+        record_words(a, record_of(a, s, k, slot), 4, sh.epoch, s, lo, hi);
         t += __longlong_as_double(
           static_cast<long long>((static_cast<unsigned long long>(hi) << 32) | lo));
     }
@@ -1525,7 +1524,10 @@ __device__ __forceinline__ bool solve(Arena const& a, Layout const& l, Share& sh
 // Every block takes shares in order until none is left. A gang's blocks wait
 // for each other only: shares are taken in order, so when a block waits, every
 // earlier gang is fully staffed and finishes, and its blocks go on to staff
-// this one. The launch is cooperative: all its blocks are resident.
+// this one. The launch is cooperative: all its blocks are resident. A block
+// whose wait gives up leaves the launch; every scene that is not solved to the
+// end, of that gang or of one that found no blocks any more, keeps the
+// kErrUnsolved that k_begin_substep gave it.
 template <int METHOD, int MODE, int FORM>
 __global__ void __launch_bounds__(Form<METHOD, MODE, FORM>::kThreads, 1)
   k_resident_solve(Arena a, GangPart const* parts, uint32_t const* nparts, Layout l) {
@@ -1565,9 +1567,19 @@ __global__ void __launch_bounds__(Form<METHOD, MODE, FORM>::kThreads, 1)
         constexpr int R = Form<METHOD, MODE, FORM>::kTiles, CH = Form<METHOD, MODE, FORM>::kRows;
         bool const ok = (MODE && s.P.precision) ? solve<METHOD, true, R, CH>(a, l, sh, s)
                                                 : solve<METHOD, false, R, CH>(a, l, sh, s);
-        if (!ok) {
-            if (threadIdx.x == 0) atomicOr(&a.ss[s.part.scene].error, kErrStalled);
+        // A thread whose wait gave up, or that saw another's give up, leaves (the
+        // block's barriers then count the threads that are left); the rest
+        // follow at the next of its checks, the last of which is here: the exit
+        // test's warp may have given up after the others' last look.
+        if (ok) block_sync();
+        if (!ok || !s.ok) {
+            *reinterpret_cast<uint32_t volatile*>(a.gave_up) = 1u;
             return;
+        }
+        // the scene is solved when its last share is
+        if (threadIdx.x == 0 &&
+            atomicAdd(&a.gangs[s.part.scene].done, 1u) + 1u == s.part.size) {
+            atomicAnd(&a.ss[s.part.scene].error, ~kErrUnsolved);
         }
     }
 }

@@ -122,7 +122,8 @@ __device__ int to_int_x86(double d) {
 // std_adaptive_time_step (emerald/sph2d_box/adaptive_time_step.h:63-103) with
 // cfl_maximum_time_step (emerald/sph_common/cfl.cpp:12-21), or the fixed
 // PCISPH sub-step (emerald/sph2d_box/pcisph.cpp:166-204), or the caller's dt.
-__global__ void k_begin_substep(Arena a, int nscenes) {
+// `resident`: a resident solve follows, which clears kErrUnsolved.
+__global__ void k_begin_substep(Arena a, int nscenes, int resident) {
     int const s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nscenes) return;
     if (s == 0) *a.gang_ticket = 0u;
@@ -131,7 +132,9 @@ __global__ void k_begin_substep(Arena a, int nscenes) {
     SceneState& S = a.ss[s];
     if (!S.active) return;
     // (the cell build may report a full table meanwhile)
-    atomicAnd(&S.error, ~kErrNonFinite);
+    int const before = atomicAnd(&S.error, ~(kErrNonFinite | kErrUnsolved));
+    int const now = ((before & kErrUnsolved) ? kErrStalled : 0) | (resident ? kErrUnsolved : 0);
+    if (now) atomicOr(&S.error, now);
     if (P.mode == kFixedDt) {
         S.dt = P.fixed_dt;
         S.t = P.fixed_t;
@@ -1306,8 +1309,8 @@ void launch_frame_check(Arena const& a, int nscenes, int method, cudaGraphCondit
 void launch_max_v2(Arena const& a, uint32_t tiles, cudaStream_t st) {
     k_max_v2<<<tiles, kTile, 0, st>>>(a);
 }
-void launch_begin_substep(Arena const& a, int nscenes, cudaStream_t st) {
-    k_begin_substep<<<(nscenes + 127) / 128, 128, 0, st>>>(a, nscenes);
+void launch_begin_substep(Arena const& a, int nscenes, bool resident, cudaStream_t st) {
+    k_begin_substep<<<(nscenes + 127) / 128, 128, 0, st>>>(a, nscenes, resident ? 1 : 0);
 }
 void launch_zero_kappas(Arena const& a, uint32_t tiles, cudaStream_t st) {
     k_zero_kappas<<<tiles, kTile, 0, st>>>(a);

@@ -83,6 +83,15 @@ typedef struct emerald_params {
 #define EMERALD_PRECISION_REFERENCE 0
 #define EMERALD_PRECISION_COMPENSATED 1
 
+/* Bits of error_flags. TABLE_FULL: a cell table had no room. NONFINITE: a
+ * division of the last sub-step was not safe (the reference asserts there).
+ * A sub-step that was not solved to the end, because a wait inside a kernel
+ * gave up, is no flag: the calls that return the scene's results, and those
+ * that would advance it, fail with EMERALD_ECUDA until the scene is given a
+ * new state (positions and velocities, or a snapshot). */
+#define EMERALD_ERROR_TABLE_FULL 1
+#define EMERALD_ERROR_NONFINITE 2
+
 /* Statistics of the last sub-step (or of the last sub-step of a frame). The
  * reference keeps these in local variables; they are returned here. */
 typedef struct emerald_step_stats {
@@ -95,7 +104,7 @@ typedef struct emerald_step_stats {
     float divergence_error_max;
     float dt;
     double time_seconds;
-    int32_t error_flags;
+    int32_t error_flags; /* EMERALD_ERROR_* */
     /* DFSPH_P: the exact mean of the per-particle errors (FP64 sum), beside
      * the reference's metric above, sum(int64(err * 1000)) / (1000 n), which
      * drops every particle's error below 0.1%. */
@@ -303,6 +312,12 @@ int emerald_sim_enable_timing(emerald_sim* sim, int32_t enable);
 int emerald_sim_kernel_times(emerald_sim* sim, char* names, size_t names_len, double* ms,
                              int32_t* launches, int32_t* count);
 
+/* Fault injection for tests: `what` set to `value` for this simulation.
+ * BARRIER_POLLS and VALUE_POLLS: how often a wait of the resident
+ * solve's blocks for one another looks before it gives up (2^22). */
+#define EMERALD_INJECT_BARRIER_POLLS 0
+#define EMERALD_INJECT_VALUE_POLLS 1
+int emerald_sim_inject(emerald_sim* sim, int32_t what, uint32_t value);
 /* Execution mode: graphs != 0 (default) runs each sub-step as one CUDA graph
  * launch with the solver loops as conditional nodes; graphs == 0 launches
  * kernels one by one and tests the loop exit on the host after every
@@ -358,6 +373,8 @@ int emerald_batch_set_forces(emerald_batch* batch, int32_t scene, emerald_force_
 int emerald_batch_free(emerald_batch* batch, size_t* fluid, int32_t* scenes);
 int emerald_batch_set_stream(emerald_batch* batch, void* cuda_stream);
 int emerald_batch_synchronize(emerald_batch* batch);
+/* As emerald_sim_inject. */
+int emerald_batch_inject(emerald_batch* batch, int32_t what, uint32_t value);
 int emerald_batch_kernel_launches(emerald_batch* batch, int64_t* count);
 
 /* -------------------------------------------------------------- autotuning */

@@ -1,0 +1,101 @@
+"""Waits inside kernels that give up (their poll limits set to none, so that
+healthy kernels run out of them): the calls that return results say so, the
+context stays usable, and a scene goes on from a new state with the bits it
+would have had."""
+import numpy as np
+import pytest
+
+from conftest import assert_bitwise
+from test_gpu_resident import METHODS, scene
+
+pytestmark = pytest.mark.gpu
+
+POLLS = 1 << 22
+# barrier and value polls: the gang's first barrier gives up; or the exchanges
+# do (and the barriers that then miss blocks, after a while)
+GIVE_UP = {"barrier": (0, 100), "value": (20000, 0)}
+
+
+def inject(E, target, barrier=POLLS, value=POLLS):
+    target.inject(E.INJECT_BARRIER_POLLS, barrier)
+    target.inject(E.INJECT_VALUE_POLLS, value)
+
+
+@pytest.fixture(scope="module")
+def E():
+    import emerald_b200
+    return emerald_b200
+
+
+@pytest.mark.parametrize("method", METHODS)
+@pytest.mark.parametrize("which", sorted(GIVE_UP))
+def test_solve_that_gives_up(E, method, which):
+    sc = scene(E, 97, 61)
+    sim = E.Simulation.from_block_scene(sc)
+    sim.advance(method, 2)
+    snap = sim.snapshot()
+    inject(E, sim, *GIVE_UP[which])
+    sim.advance(method, 1, stats=False)
+    for call in (sim.state, sim.time, sim.snapshot, sim.neighbors, lambda: sim.array("densities"),
+                 lambda: sim.advance(method, 1), lambda: sim.frame(method), sim.state):
+        with pytest.raises(E.EmeraldError):
+            call()
+    inject(E, sim)
+    with pytest.raises(E.EmeraldError):
+        sim.advance(method, 1)
+    sim.restore(snap)
+    sim.advance(method, 2)
+    want = E.Simulation.from_block_scene(sc)
+    want.advance(method, 4)
+    for name, x, y in zip("xv", sim.state(), want.state()):
+        assert_bitwise(x, y, "%s %s" % (method, name))
+    # positions and velocities are a new state too
+    inject(E, sim, *GIVE_UP[which])
+    with pytest.raises(E.EmeraldError):
+        sim.advance(method, 1)
+    inject(E, sim)
+    sim.set_state(sc.fluid, np.zeros_like(sc.fluid))
+    assert sim.advance(method, 1)["error_flags"] == 0
+
+
+@pytest.mark.parametrize("method", ("dfsph_p", "iisph_ap"))
+@pytest.mark.parametrize("which", sorted(GIVE_UP))
+def test_batch_that_gives_up(E, method, which):
+    """More shares than blocks: a scene whose blocks gave up, or that found no
+    blocks any more, reports it; one that was solved has its results."""
+    scenes = [scene(E, 40 + 13 * (k % 9), 30 + 17 * (k % 5)) for k in range(24)]
+    scenes += [scene(E, 330, 301), scene(E, 5, 4)]
+    sizes = [sum(-(-len(p) // 128) * 128 for p in ps)
+             for ps in ([s.fluid for s in scenes], [s.solid for s in scenes])]
+    b = E.Batch(sizes[0], sizes[1], len(scenes))
+    ids = [b.add_block_scene(s) for s in scenes]
+    b.step(method, 1)
+    b.synchronize()
+    inject(E, b, *GIVE_UP[which])
+    b.step(method, 1)
+    with pytest.raises(E.EmeraldError):
+        b.synchronize()
+    with pytest.raises(E.EmeraldError):
+        b.step(method, 1)
+    inject(E, b)
+    failed = []
+    for k, sc in enumerate(scenes):
+        want = E.Simulation.from_block_scene(sc)
+        want.advance(method, 2)
+        try:
+            got = b.state(ids[k])
+        except E.EmeraldError:
+            failed.append(k)
+            with pytest.raises(E.EmeraldError):
+                b.stats(ids[k])
+        else:
+            for name, x, y in zip("xv", got, want.state()):
+                assert_bitwise(x, y, "scene %d %s" % (k, name))
+        want.close()
+    assert 24 in failed
+    for k in failed:
+        b.remove_scene(ids[k])
+    if len(failed) < len(scenes):
+        b.step(method, 1)
+        b.synchronize()
+    b.close()
