@@ -19,6 +19,7 @@ PRECISION_REFERENCE = 0
 PRECISION_COMPENSATED = 1
 INJECT_BARRIER_POLLS = 0
 INJECT_VALUE_POLLS = 1
+INJECT_SORT_POLLS = 2
 FLICKS_PER_SECOND = 705600000
 
 c_f = ctypes.c_float
@@ -227,6 +228,7 @@ EXPORTS = {
     "emerald_compute_z_indices": (c_i32, [c_sz, c_vp, c_vp, c_vp]),
     "emerald_compute_index_pairs": (c_i32, [c_sz, c_vp, c_vp, c_vp]),
     "emerald_index_pairs_workspace": (c_i32, [c_sz, ctypes.POINTER(c_sz)]),
+    "emerald_sort_index_pairs_inject": (c_i32, [c_sz, c_vp, c_vp, c_sz, c_vp, c_vp]),
     "emerald_sort_index_pairs": (c_i32, [c_sz, c_vp, c_vp, c_sz, c_vp]),
     "emerald_compute_block_indices": (c_i32, [c_sz, c_vp, c_vp, c_vp, c_sz, c_vp]),
     "emerald_fill_blocks": (c_i32, [c_sz, c_vp, c_vp, c_vp]),

@@ -764,6 +764,7 @@ void Engine::inject(int what, uint32_t value) {
     switch (what) {
     case EMERALD_INJECT_BARRIER_POLLS: a_.barrier_polls = value; break;
     case EMERALD_INJECT_VALUE_POLLS: a_.value_polls = value; break;
+    case EMERALD_INJECT_SORT_POLLS: order_sort_.polls = sort_.polls = value; break;
     default: throw std::invalid_argument("unknown injection");
     }
     destroy_graphs();  // they hold the arena's values
@@ -1980,6 +1981,7 @@ void Engine::ensure_sort_scratch(uint32_t n) {
     }
     sort_cap_ = n;
     sort_scratch_carve(sort_buf_, n, sort_);
+    sort_.polls = order_sort_.polls;
 }
 
 size_t Engine::get_sort(int id, bool solid, int32_t* gc, uint64_t* z, uint64_t* pair_z,
@@ -2010,13 +2012,16 @@ size_t Engine::get_sort(int id, bool solid, int32_t* gc, uint64_t* z, uint64_t* 
     uint32_t* d_bl = reinterpret_cast<uint32_t*>(p);
     p += 8 * words;
     uint32_t* d_nb = reinterpret_cast<uint32_t*>(p);
+    uint32_t const* gave_up = nullptr;
     launch("sort_products", [&] {
         if (!solid) launch_order_members(a_, P.ftab_begin, sc.ftab_size, st_);
-        launch_sort_products(a_, solid, id, solid ? P.solid_begin : P.fluid_begin, n,
-                             solid ? P.stab_begin : P.ftab_begin, solid ? sc.stab_size : sc.ftab_size,
-                             P.cell_size, sort_, d_gc, d_z, d_pz, d_pi, d_bi, d_bl, d_nb, st_);
+        gave_up = launch_sort_products(
+          a_, solid, id, solid ? P.solid_begin : P.fluid_begin, n,
+          solid ? P.stab_begin : P.ftab_begin, solid ? sc.stab_size : sc.ftab_size, P.cell_size,
+          sort_, d_gc, d_z, d_pz, d_pi, d_bi, d_bl, d_nb, st_);
     });
-    uint32_t nb = 0;
+    uint32_t nb = 0, unsorted = 0;
+    if (gave_up) cudaMemcpyAsync(&unsorted, gave_up, 4, cudaMemcpyDeviceToHost, st_);
     std::vector<uint32_t> hpi(n), hbl(2 * size_t(n));
     cudaMemcpyAsync(&nb, d_nb, 4, cudaMemcpyDeviceToHost, st_);
     if (gc) cudaMemcpyAsync(gc, d_gc, 8 * words, cudaMemcpyDeviceToHost, st_);
@@ -2028,6 +2033,7 @@ size_t Engine::get_sort(int id, bool solid, int32_t* gc, uint64_t* z, uint64_t* 
     host_wait(st_);
     cudaFree(out);
     check("get_sort");
+    if (unsorted) throw std::runtime_error("z-order sort: a wait gave up");
     if (pair_index) {
         for (uint32_t k = 0; k < n; ++k) pair_index[k] = hpi[k];
     }

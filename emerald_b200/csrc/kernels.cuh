@@ -31,18 +31,32 @@ struct SortScratch {
     uint32_t* offsets;
     uint32_t* hist;
     uint32_t* scan;
+    void* control;   // of the sort in one launch
+    uint32_t polls;  // of its barriers before they give up
     uint32_t capacity;
 };
 size_t sort_scratch_bytes(uint32_t n);
 void sort_scratch_carve(void* base, uint32_t n, SortScratch& s);
 // Stable LSD radix sort of (key, value) pairs on the low `bits` key bits;
-// returns the buffer index (0 or 1) holding the result.
-int launch_radix_sort(SortScratch& s, uint32_t n, int bits, cudaStream_t st);
+// returns the buffer index (0 or 1) holding the result. gave_up (where it is
+// not null): a device word that is not zero when a wait of the sort gave up and
+// the buffers hold no order; whoever reads them looks there first. With `again`
+// a second sort of the same scratch, which gives up where the first did.
+struct SortResult {
+    int cur;
+    uint32_t const* gave_up;
+};
+SortResult launch_radix_sort(SortScratch& s, uint32_t n, int bits, cudaStream_t st,
+                             bool again = false);
+__device__ __forceinline__ bool sort_gave_up(uint32_t const* gave_up) {
+    return gave_up && *gave_up;
+}
 // Reference sort products of one scene's fluid (solid=false) or boundary set:
 // per particle grid coords (int2) and z keys, the sorted (z, index) pairs
 // with scene-local indices, block indices and the [begin, end) block ranges.
-// Returns the number of blocks through *nblocks (device word).
-void launch_sort_products(Arena const& a, bool solid, int scene, uint32_t begin, uint32_t count,
+// Returns the number of blocks through *nblocks (device word), and the sort's
+// gave_up word: the products hold nothing where it is set.
+uint32_t const* launch_sort_products(Arena const& a, bool solid, int scene, uint32_t begin, uint32_t count,
                           uint32_t tab_begin, uint32_t tab_size, float cell, SortScratch& s,
                           int2* grid_coords, uint64_t* z, uint64_t* pair_z, uint32_t* pair_index,
                           uint32_t* block_indices, uint32_t* blocks, uint32_t* nblocks,

@@ -46,9 +46,10 @@ __global__ void k_order_keys(Arena a, uint64_t* keys, uint32_t* vals, uint32_t n
 // order; scenes keep their ranges (the sort's leading key is the scene's
 // first tile, and scene s's particles start at sort_base within the sorted
 // list).
-__global__ void k_permute(Arena a, uint64_t const* keys, uint32_t const* vals, uint32_t n) {
+__global__ void k_permute(Arena a, uint64_t const* keys, uint32_t const* vals, uint32_t n,
+                          uint32_t const* gave_up) {
     uint32_t const p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n || keys[p] == ~0ull) return;
+    if (p >= n || sort_gave_up(gave_up) || keys[p] == ~0ull) return;
     uint32_t const old = vals[p];
     int32_t const s = a.tile_scene[old / kTile];
     SceneParams const& P = a.sp[s];
@@ -61,9 +62,9 @@ __global__ void k_permute(Arena a, uint64_t const* keys, uint32_t const* vals, u
     a.tx64[dst] = a.x64[old];
 }
 
-__global__ void k_commit_order(Arena a, uint32_t n) {
+__global__ void k_commit_order(Arena a, uint32_t n, uint32_t const* gave_up) {
     uint32_t const t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
+    if (t >= n || sort_gave_up(gave_up)) return;
     int32_t const s = a.tile_scene[t / kTile];
     if (s < 0) return;
     SceneParams const& P = a.sp[s];
@@ -139,9 +140,10 @@ __global__ void k_identity_order(Arena a, uint32_t begin, uint32_t count) {
 
 void launch_reorder(Arena const& a, SortScratch& s, uint32_t n, int key_bits, cudaStream_t st) {
     k_order_keys<<<(n + 255) / 256, 256, 0, st>>>(a, s.keys[0], s.vals[0], n);
-    int const cur = launch_radix_sort(s, n, key_bits, st);
-    k_permute<<<(n + 255) / 256, 256, 0, st>>>(a, s.keys[cur], s.vals[cur], n);
-    k_commit_order<<<(n + 255) / 256, 256, 0, st>>>(a, n);
+    // (a sort that gave up leaves the storage as it was, which changes no result)
+    SortResult const r = launch_radix_sort(s, n, key_bits, st);
+    k_permute<<<(n + 255) / 256, 256, 0, st>>>(a, s.keys[r.cur], s.vals[r.cur], n, r.gave_up);
+    k_commit_order<<<(n + 255) / 256, 256, 0, st>>>(a, n, r.gave_up);
 }
 
 void launch_gather_f(Arena const& a, uint32_t begin, uint32_t count, float const* src, float* out,

@@ -11,6 +11,7 @@
 #include "sph_math.cuh"
 
 #include <algorithm>
+#include <cstddef>
 
 namespace emerald {
 
@@ -72,31 +73,33 @@ __global__ void k_rank_scatter(uint64_t const* kin, uint32_t const* vin, uint64_
     }
 }
 
-// Words of the resident sort at the start of the scan scratch, zero at launch.
+// Words of the resident sort, zero at launch.
 struct SortControl {
     unsigned long long any;      // OR of the keys
     unsigned long long any_not;  // OR of their complements
     uint32_t arrived;            // blocks at the grid barriers so far
-    uint32_t stalled;            // a barrier ran out of polls: every block returns
+    // a barrier ran out of polls: every block returns (last: a second sort of
+    // the same scratch leaves it as it is)
+    uint32_t stalled;
 };
 
 constexpr int kSortThreads = 1024;
 constexpr int kSortWarps = kSortThreads / 32;
 constexpr uint32_t kSortPolls = 1u << 22;
 
-// False when a block did not come: the launch is cooperative, so all are
-// resident and this only bounds the wait.
-__device__ __forceinline__ bool sort_barrier(SortControl* c, uint32_t target) {
+// False when a block did not come within `limit` polls (0: none does): the
+// launch is cooperative, so all are resident and this only bounds the wait.
+__device__ __forceinline__ bool sort_barrier(SortControl* c, uint32_t target, uint32_t limit) {
     __syncthreads();
     uint32_t bad = 0;
     if (threadIdx.x == 0) {
         __threadfence();
         atomicAdd(&c->arrived, 1u);
         uint32_t polls = 0;
-        while (*reinterpret_cast<uint32_t volatile*>(&c->arrived) < target) {
+        while (!limit || *reinterpret_cast<uint32_t volatile*>(&c->arrived) < target) {
             bad = *reinterpret_cast<uint32_t volatile*>(&c->stalled);
             if (bad) break;
-            if (++polls == kSortPolls) {
+            if (++polls > limit) {
                 atomicExch(&c->stalled, 1u);
                 bad = 1;
                 break;
@@ -116,7 +119,7 @@ __device__ __forceinline__ bool sort_barrier(SortControl* c, uint32_t target) {
 // two barriers. The result is put in buffer `out`.
 __global__ void __launch_bounds__(kSortThreads, 1)
   k_sort_resident(uint64_t* k0, uint64_t* k1, uint32_t* v0, uint32_t* v1, uint32_t n, int bits,
-                  uint32_t tiles, uint32_t* hist, SortControl* ctl, int out) {
+                  uint32_t tiles, uint32_t* hist, SortControl* ctl, uint32_t polls, int out) {
     __shared__ uint32_t wcnt[kSortWarps][kDigits];  // also the partial sums of the offsets
     __shared__ uint32_t base[kDigits];
     __shared__ uint32_t wsum[kDigits / 32];
@@ -139,7 +142,7 @@ __global__ void __launch_bounds__(kSortThreads, 1)
         if (any_not) atomicOr(&ctl->any_not, static_cast<unsigned long long>(any_not));
     }
     uint32_t target = nb;
-    if (!sort_barrier(ctl, target)) return;
+    if (!sort_barrier(ctl, target, polls)) return;
     uint64_t const differ = __ldcg(&ctl->any) & __ldcg(&ctl->any_not);
     int cur = 0;
     for (int shift = 0; shift < bits; shift += 8) {
@@ -156,7 +159,7 @@ __global__ void __launch_bounds__(kSortThreads, 1)
         __syncthreads();
         if (t < kDigits) __stcg(hist + static_cast<size_t>(b) * kDigits + t, base[t]);
         target += nb;
-        if (!sort_barrier(ctl, target)) return;
+        if (!sort_barrier(ctl, target, polls)) return;
         // digit d over all blocks, and over the blocks before this one
         {
             uint32_t const d = t % kDigits, part = t / kDigits, parts = kSortThreads / kDigits;
@@ -221,7 +224,7 @@ __global__ void __launch_bounds__(kSortThreads, 1)
             }
         }
         target += nb;
-        if (!sort_barrier(ctl, target)) return;
+        if (!sort_barrier(ctl, target, polls)) return;
         cur ^= 1;
     }
     if (cur != out) {
@@ -258,10 +261,11 @@ __global__ void k_fill_tail(uint64_t* keys, uint32_t* vals, uint32_t const* ncel
 }
 
 __global__ void k_cell_counts(uint32_t const* sorted_slots, uint32_t const* count,
-                              uint32_t const* ncells, uint32_t limit, uint32_t* cell_count) {
+                              uint32_t const* ncells, uint32_t limit, uint32_t* cell_count,
+                              uint32_t const* gave_up) {
     uint32_t const c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= limit) return;
-    cell_count[c] = c < *ncells ? count[sorted_slots[c]] : 0u;
+    cell_count[c] = c < *ncells && !sort_gave_up(gave_up) ? count[sorted_slots[c]] : 0u;
 }
 
 __global__ void k_expand_pairs(uint64_t const* sorted_z, uint32_t const* sorted_slots,
@@ -269,9 +273,10 @@ __global__ void k_expand_pairs(uint64_t const* sorted_z, uint32_t const* sorted_
                                uint32_t const* start, uint32_t const* members,
                                uint32_t const* oid, uint32_t const* ncells, uint32_t limit,
                                uint32_t first, uint64_t* pair_z, uint32_t* pair_index,
-                               uint32_t* block_indices, uint32_t* blocks) {
+                               uint32_t* block_indices, uint32_t* blocks,
+                               uint32_t const* gave_up) {
     uint32_t const c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= limit || c >= *ncells) return;
+    if (c >= limit || c >= *ncells || sort_gave_up(gave_up)) return;
     uint32_t const slot = sorted_slots[c];
     uint32_t const n = count[slot];
     uint32_t const b = cell_start[c];
@@ -327,7 +332,10 @@ static size_t carve(char* base, uint32_t n, SortScratch* s) {
     char* fl = take(words * 4);
     char* of = take(words * 4);
     char* hi = take(kDigits * nb * 8);
-    char* sc = take((scan_scratch_words(static_cast<uint32_t>(kDigits * nb + words)) + 16) * 4);
+    // the scan's words, then (from a multiple of eight) the sort's control words
+    size_t const scan = scan_scratch_words(static_cast<uint32_t>(kDigits * nb + words));
+    char* sc = take((scan + 16) * 4);
+    static_assert(sizeof(SortControl) <= 4 * 8, "seven words to the next multiple, eight for it");
     if (s) {
         s->keys[0] = reinterpret_cast<uint64_t*>(k0);
         s->keys[1] = reinterpret_cast<uint64_t*>(k1);
@@ -337,6 +345,8 @@ static size_t carve(char* base, uint32_t n, SortScratch* s) {
         s->offsets = reinterpret_cast<uint32_t*>(of);
         s->hist = reinterpret_cast<uint32_t*>(hi);
         s->scan = reinterpret_cast<uint32_t*>(sc);
+        s->control = sc + (scan + 7) / 8 * 8 * 4;
+        s->polls = kSortPolls;
         s->capacity = n;
     }
     return off;
@@ -359,7 +369,8 @@ void sort_scratch_carve(void* base, uint32_t n, SortScratch& s) {
 constexpr uint32_t kResidentKeysShort = 1u << 19;
 constexpr uint32_t kResidentKeysLong = 1u << 22;
 
-static bool launch_sort_resident(SortScratch& s, uint32_t n, int bits, int out, cudaStream_t st) {
+static bool launch_sort_resident(SortScratch& s, uint32_t n, int bits, int out, bool again,
+                                 cudaStream_t st) {
     int dev = 0, coop = 0, sms = 0;
     if (n > (bits > 40 ? kResidentKeysLong : kResidentKeysShort) ||
         cudaGetDevice(&dev) != cudaSuccess ||
@@ -370,8 +381,8 @@ static bool launch_sort_resident(SortScratch& s, uint32_t n, int bits, int out, 
     }
     uint32_t const tiles = (n + kItems - 1) / kItems;
     uint32_t const blocks = std::min<uint32_t>(tiles, static_cast<uint32_t>(sms));
-    SortControl* const ctl = reinterpret_cast<SortControl*>(s.scan);
-    cudaMemsetAsync(ctl, 0, sizeof(SortControl), st);
+    SortControl* const ctl = static_cast<SortControl*>(s.control);
+    cudaMemsetAsync(ctl, 0, again ? offsetof(SortControl, stalled) : sizeof(SortControl), st);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(kSortThreads);
@@ -382,17 +393,20 @@ static bool launch_sort_resident(SortScratch& s, uint32_t n, int bits, int out, 
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     if (cudaLaunchKernelEx(&cfg, k_sort_resident, s.keys[0], s.keys[1], s.vals[0], s.vals[1], n,
-                           bits, tiles, s.hist, ctl, out) != cudaSuccess) {
+                           bits, tiles, s.hist, ctl, s.polls, out) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
     return true;
 }
 
-int launch_radix_sort(SortScratch& s, uint32_t n, int bits, cudaStream_t st) {
+SortResult launch_radix_sort(SortScratch& s, uint32_t n, int bits, cudaStream_t st, bool again) {
     int cur = 0;
-    if (n <= 1) return cur;
-    if (launch_sort_resident(s, n, bits, ((bits + 7) / 8) & 1, st)) return ((bits + 7) / 8) & 1;
+    if (n <= 1) return {cur, nullptr};
+    int const out = ((bits + 7) / 8) & 1;
+    if (launch_sort_resident(s, n, bits, out, again, st)) {
+        return {out, &static_cast<SortControl*>(s.control)->stalled};
+    }
     uint32_t const nb = (n + kItems - 1) / kItems;
     uint32_t* offsets = s.hist + static_cast<size_t>(kDigits) * nb;
     for (int shift = 0; shift < bits; shift += 8) {
@@ -402,10 +416,10 @@ int launch_radix_sort(SortScratch& s, uint32_t n, int bits, cudaStream_t st) {
                                                 s.vals[cur ^ 1], n, shift, offsets, nb);
         cur ^= 1;
     }
-    return cur;
+    return {cur, nullptr};
 }
 
-void launch_sort_products(Arena const& a, bool solid, int scene, uint32_t begin, uint32_t count,
+uint32_t const* launch_sort_products(Arena const& a, bool solid, int scene, uint32_t begin, uint32_t count,
                           uint32_t tab_begin, uint32_t tab_size, float cell, SortScratch& s,
                           int2* grid_coords, uint64_t* z, uint64_t* pair_z, uint32_t* pair_index,
                           uint32_t* block_indices, uint32_t* blocks, uint32_t* nblocks,
@@ -432,15 +446,18 @@ void launch_sort_products(Arena const& a, bool solid, int scene, uint32_t begin,
     // The tail [ncells, limit) gets the largest key; the stable sort keeps it
     // behind every real cell, including a real cell with that key.
     k_fill_tail<<<(limit + 255) / 256, 256, 0, st>>>(s.keys[0], s.vals[0], nblocks, limit);
-    int const cur = launch_radix_sort(s, limit, 64, st);
+    SortResult const sorted = launch_radix_sort(s, limit, 64, st);
+    int const cur = sorted.cur;
     uint32_t* cell_count = s.flags;
     uint32_t* cell_start = s.offsets;
-    k_cell_counts<<<(limit + 255) / 256, 256, 0, st>>>(s.vals[cur], cnt, nblocks, limit, cell_count);
+    k_cell_counts<<<(limit + 255) / 256, 256, 0, st>>>(s.vals[cur], cnt, nblocks, limit, cell_count,
+                                                     sorted.gave_up);
     launch_exclusive_scan(cell_count, limit, cell_start, s.scan, st);
     k_expand_pairs<<<(limit + 255) / 256, 256, 0, st>>>(s.keys[cur], s.vals[cur], cell_start, cnt,
                                                        start, members, solid ? nullptr : a.oid,
                                                        nblocks, limit, begin, pair_z, pair_index,
-                                                       block_indices, blocks);
+                                                       block_indices, blocks, sorted.gave_up);
+    return sorted.gave_up;
 }
 
 }  // namespace emerald

@@ -97,18 +97,33 @@ __global__ void k_keys_index(uint32_t n, uint64_t const* pairs, uint64_t* copy, 
 // Second sort key: the z key of the pair at each position of the first
 // order (read before the slot is rewritten, so in and out may alias).
 __global__ void k_keys_z(uint32_t n, uint64_t const* copy, uint32_t const* perm, uint64_t* keys,
-                         uint32_t* vals) {
+                         uint32_t* vals, uint32_t const* gave_up) {
     uint32_t const i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= n || sort_gave_up(gave_up)) return;
     uint32_t const p = perm[i];
     keys[i] = copy[2 * size_t(p)];
     vals[i] = p;
 }
 
+// Where a wait of one of the sorts gave up there is no order: every pair then
+// counts the pairs before it (n passes over the copy; the sorts that can give
+// up are of 2^22 pairs at most).
 __global__ void k_gather_pairs(uint32_t n, uint64_t const* copy, uint32_t const* perm,
-                               uint64_t* pairs) {
+                               uint64_t* pairs, uint32_t const* gave_up) {
     uint32_t const i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    if (sort_gave_up(gave_up)) {
+        uint64_t const z = copy[2 * size_t(i)], idx = copy[2 * size_t(i) + 1];
+        uint32_t before = 0;
+#pragma unroll 1
+        for (uint32_t k = 0; k < n; ++k) {
+            uint64_t const zk = copy[2 * size_t(k)], ik = copy[2 * size_t(k) + 1];
+            before += zk < z || (zk == z && (ik < idx || (ik == idx && k < i))) ? 1u : 0u;
+        }
+        pairs[2 * size_t(before)] = z;
+        pairs[2 * size_t(before) + 1] = idx;
+        return;
+    }
     uint32_t const p = perm[i];
     pairs[2 * size_t(i)] = copy[2 * size_t(p)];
     pairs[2 * size_t(i) + 1] = copy[2 * size_t(p) + 1];
@@ -400,8 +415,8 @@ int emerald_index_pairs_workspace(size_t n, size_t* bytes) {
     return EMERALD_OK;
 }
 
-int emerald_sort_index_pairs(size_t n, uint64_t* index_pairs, void* workspace,
-                             size_t workspace_size, void* stream) {
+int emerald_sort_index_pairs_inject(size_t n, uint64_t* index_pairs, void* workspace,
+                                    size_t workspace_size, void* stream, uint32_t const* polls) {
     if (n <= 1) return EMERALD_OK;  // neighborhood.cpp:20
     if (n >= UINT32_MAX) return set_last_error(EMERALD_EINVAL, "n must be below 2^32 - 1");
     if (!index_pairs || !workspace) {
@@ -417,15 +432,23 @@ int emerald_sort_index_pairs(size_t n, uint64_t* index_pairs, void* workspace,
     char* base = static_cast<char*>(workspace);
     SortScratch s;
     sort_scratch_carve(base, m, s);
+    if (polls) s.polls = *polls;
     uint64_t* copy = reinterpret_cast<uint64_t*>(base + align256(sort_scratch_bytes(m)));
     cudaStream_t const st = S(stream);
     unsigned const g = grid(n);
     k_keys_index<<<g, kThreads, 0, st>>>(m, index_pairs, copy, s.keys[0], s.vals[0]);
-    int const a = launch_radix_sort(s, m, 64, st);
-    k_keys_z<<<g, kThreads, 0, st>>>(m, copy, s.vals[a], s.keys[0], s.vals[0]);
-    int const b = launch_radix_sort(s, m, 64, st);
-    k_gather_pairs<<<g, kThreads, 0, st>>>(m, copy, s.vals[b], index_pairs);
+    SortResult const a = launch_radix_sort(s, m, 64, st);
+    k_keys_z<<<g, kThreads, 0, st>>>(m, copy, s.vals[a.cur], s.keys[0], s.vals[0], a.gave_up);
+    SortResult const b = launch_radix_sort(s, m, 64, st, a.gave_up != nullptr);
+    k_gather_pairs<<<g, kThreads, 0, st>>>(m, copy, s.vals[b.cur], index_pairs,
+                                           b.gave_up ? b.gave_up : a.gave_up);
     return cuda_status();
+}
+
+int emerald_sort_index_pairs(size_t n, uint64_t* index_pairs, void* workspace,
+                             size_t workspace_size, void* stream) {
+    return emerald_sort_index_pairs_inject(n, index_pairs, workspace, workspace_size, stream,
+                                           nullptr);
 }
 
 int emerald_compute_block_indices(size_t n, uint32_t* block_indices,

@@ -314,9 +314,12 @@ int emerald_sim_kernel_times(emerald_sim* sim, char* names, size_t names_len, do
 
 /* Fault injection for tests: `what` set to `value` for this simulation.
  * BARRIER_POLLS and VALUE_POLLS: how often a wait of the resident
- * solve's blocks for one another looks before it gives up (2^22). */
+ * solve's blocks for one another looks before it gives up (2^22); SORT_POLLS:
+ * the same of the z-order sort's (a re-sort of the storage that gives up is
+ * left out, emerald_sim_get_sort fails). */
 #define EMERALD_INJECT_BARRIER_POLLS 0
 #define EMERALD_INJECT_VALUE_POLLS 1
+#define EMERALD_INJECT_SORT_POLLS 2
 int emerald_sim_inject(emerald_sim* sim, int32_t what, uint32_t value);
 /* Execution mode: graphs != 0 (default) runs each sub-step as one CUDA graph
  * launch with the solver loops as conditional nodes; graphs == 0 launches
@@ -541,6 +544,11 @@ int emerald_index_pairs_workspace(size_t n, size_t* bytes);
  * the order std::sort gives the pairs, in place. */
 int emerald_sort_index_pairs(size_t n, uint64_t* index_pairs, void* workspace,
                              size_t workspace_bytes, void* stream);
+/* The same with the sort's poll limit (fault injection for tests; NULL: the
+ * default). The order does not depend on it: where a wait gives up, every
+ * pair's place is counted instead, which is slow. */
+int emerald_sort_index_pairs_inject(size_t n, uint64_t* index_pairs, void* workspace,
+                                    size_t workspace_size, void* stream, uint32_t const* polls);
 /* compute_block_indices (neighborhood.cpp:28-64): per sorted pair, the
  * number of z changes before it (0 0 0 1 1 2 ...). The block count is
  * block_indices[n - 1] + 1, read by the caller as the reference's driver

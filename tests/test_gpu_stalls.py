@@ -99,3 +99,41 @@ def test_batch_that_gives_up(E, method, which):
         b.step(method, 1)
         b.synchronize()
     b.close()
+
+
+@pytest.mark.parametrize("n", [2, 2048, 2049, 30000])
+def test_pair_sort_that_gives_up_is_sorted_all_the_same(E, n):
+    import ctypes
+
+    import torch
+    rng = np.random.Generator(np.random.PCG64(n))
+    z = rng.integers(0, max(n // 3, 1), n).astype(np.uint64)
+    index = rng.integers(0, max(n // 2, 1), n).astype(np.uint64)   # some pairs twice
+    pairs = np.stack([z, index], 1)
+    size = ctypes.c_size_t()
+    assert E.lib.emerald_index_pairs_workspace(n, ctypes.byref(size)) == 0
+    work = torch.full((size.value,), 0xA5, dtype=torch.uint8, device="cuda")
+    none = ctypes.c_uint32(0)
+    for polls in (ctypes.byref(none), None):
+        d = torch.from_numpy(pairs.view(np.int64).copy()).cuda()
+        assert E.lib.emerald_sort_index_pairs_inject(
+            n, d.data_ptr(), work.data_ptr(), work.numel(),
+            torch.cuda.current_stream().cuda_stream, polls) == 0
+        assert np.array_equal(d.cpu().numpy().view(np.uint64), pairs[np.lexsort((index, z))])
+
+
+def test_storage_sort_that_gives_up_is_left_out(E):
+    """The order of the storage changes no result; the sort products fail."""
+    sc = scene(E, 97, 61)
+    a = E.Simulation.from_block_scene(sc)
+    b = E.Simulation.from_block_scene(sc)
+    b.inject(E.INJECT_SORT_POLLS, 0)
+    for sim in (a, b):
+        sim.advance("dfsph_p", 20)
+    for name, x, y in zip("xv", a.state(), b.state()):
+        assert_bitwise(x, y, name)
+    with pytest.raises(E.EmeraldError):
+        b.sort()
+    b.inject(E.INJECT_SORT_POLLS, POLLS)
+    for x, y in zip(a.sort(), b.sort()):
+        assert np.array_equal(x, y)
