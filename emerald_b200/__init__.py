@@ -20,6 +20,7 @@ PRECISION_COMPENSATED = 1
 INJECT_BARRIER_POLLS = 0
 INJECT_VALUE_POLLS = 1
 INJECT_SORT_POLLS = 2
+INJECT_REFUSE = 3
 FLICKS_PER_SECOND = 705600000
 
 c_f = ctypes.c_float

@@ -107,6 +107,15 @@ uint32_t max_parts(uint32_t fluid_capacity, int max_scenes) {
 
 }  // namespace
 
+// A cooperative launch of as many blocks as the device reports multiprocessors
+// was refused (a process may be given fewer); while a graph is recorded, the
+// recording starts again without it.
+struct ResidentRefused : std::runtime_error {
+    ResidentRefused() : std::runtime_error("resident solve: launch refused") {}
+};
+
+struct NoFrameGraph {};
+
 int64_t kernel_launch_count() { return g_launches.load(); }
 
 // ------------------------------------------------------------ allocator
@@ -764,6 +773,10 @@ void Engine::inject(int what, uint32_t value) {
     switch (what) {
     case EMERALD_INJECT_BARRIER_POLLS: a_.barrier_polls = value; break;
     case EMERALD_INJECT_VALUE_POLLS: a_.value_polls = value; break;
+    case EMERALD_INJECT_REFUSE:
+        refuse_ = value != 0u;
+        refused_ = false;
+        break;
     case EMERALD_INJECT_SORT_POLLS: order_sort_.polls = sort_.polls = value; break;
     default: throw std::invalid_argument("unknown injection");
     }
@@ -1056,13 +1069,19 @@ void Engine::emit_substep(int32_t method, bool reorder) {
                [&] { launch_neighbors(a_, tiles, true, kernels, st, compensated_); });
     }
     if (resident) {
+        cudaError_t e = cudaSuccess;
         launch("solve", [&] {
-            cudaError_t const e = launch_resident_solve(a_, plans_[method], method, compensated_, st);
-            if (e != cudaSuccess) {
-                throw std::runtime_error(std::string("resident solve: ") + cudaGetErrorString(e));
-            }
+            e = refuse_ ? cudaErrorCooperativeLaunchTooLarge
+                        : launch_resident_solve(a_, plans_[method], method, compensated_, st);
         });
-        return;
+        if (e == cudaSuccess) return;
+        cudaGetLastError();
+        if (capturing_) throw ResidentRefused();
+        // nothing of the solve has run: the kernels per phase do it
+        refused_ = true;
+        for (int id = 0; id < max_scenes_; ++id) {
+            if (scenes_[id].used) launch_clear_stall(a_, id, st);
+        }
     }
     switch (method) {
     case kDfsph:
@@ -1136,6 +1155,7 @@ void Engine::capture_substep(int32_t method, bool reorder) {
     cudaError_t const e = cudaGraphInstantiate(&exec, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) {
+        if (use_resident(method)) throw ResidentRefused();
         throw std::runtime_error(std::string("graph instantiate: ") + cudaGetErrorString(e));
     }
     graphs_[graph_key(method, reorder)] = exec;
@@ -1232,10 +1252,25 @@ void Engine::capture_frame(int32_t method, bool reorder) {
     cudaError_t const e = cudaGraphInstantiate(&exec, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) {
+        if (use_resident(method)) throw ResidentRefused();
         throw std::runtime_error(std::string("frame graph instantiate: ") + cudaGetErrorString(e));
     }
     frame_graphs_[graph_key(method, reorder)] = exec;
     frame_fixed_kernels_[graph_key(method, reorder)] = capture_kernels_;
+}
+
+// f(), and once more with the kernels per phase where the device refused the
+// resident solve (for good: it would refuse it again).
+template <class F>
+int Engine::with_refusals(F&& f) {
+    try {
+        return f();
+    } catch (ResidentRefused const&) {
+        cudaGetLastError();
+        refused_ = true;
+        destroy_graphs();
+        return f();
+    }
 }
 
 int Engine::frame(int id, int32_t method, SceneState& out) {
@@ -1255,23 +1290,32 @@ int Engine::frame(int id, int32_t method, SceneState& out) {
     if (reorder) storage_in_order();
     prepare_substep(method);
     ++frames_launched_;
-    int const key = graph_key(method, reorder);
-    auto it = frame_graphs_.find(key);
-    if (it == frame_graphs_.end()) {
-        try {
-            capture_frame(method, reorder);
-        } catch (std::runtime_error const&) {
-            // a device or driver without the frame graph's nested
-            // conditional nodes: frames keep the host loop from now on
-            frame_graphs_ok_ = false;
-            --frames_launched_;
-            return frame(id, method, out);
-        }
-        it = frame_graphs_.find(key);
-    }
-    if (cudaGraphLaunch(it->second, st_) != cudaSuccess) {
-        check("frame graph launch");
-        throw std::runtime_error("frame graph launch failed");
+    int key;
+    try {
+        key = with_refusals([&] {
+            int const k = graph_key(method, reorder);
+            if (!frame_graphs_.count(k)) {
+                try {
+                    capture_frame(method, reorder);
+                } catch (ResidentRefused const&) {
+                    throw;
+                } catch (std::runtime_error const&) {
+                    throw NoFrameGraph();
+                }
+            }
+            if (cudaGraphLaunch(frame_graphs_[k], st_) != cudaSuccess) {
+                if (use_resident(method)) throw ResidentRefused();
+                check("frame graph launch");
+                throw std::runtime_error("frame graph launch failed");
+            }
+            return k;
+        });
+    } catch (NoFrameGraph const&) {
+        // a device or driver without the frame graph's nested conditional
+        // nodes: frames keep the host loop from now on
+        frame_graphs_ok_ = false;
+        --frames_launched_;
+        return frame(id, method, out);
     }
     int64_t const fixed = frame_fixed_kernels_[key];
     host_launches_ += fixed;
@@ -1345,7 +1389,7 @@ ResidentLimits const& Engine::limits_of(int32_t method) {
 // force callbacks (which interrupt the sub-step) take those; so do scenes
 // whose shares are above the method's limit.
 bool Engine::use_resident(int32_t method) {
-    if (timing_ || !tuning_.resident || has_force_callbacks()) return false;
+    if (timing_ || refused_ || !tuning_.resident || has_force_callbacks()) return false;
     ResidentLimits const& lim = limits_of(method);
     if (!lim.blocks) return false;
     if (!parts_valid_) divide_scenes(lim.blocks);
@@ -1437,16 +1481,16 @@ void Engine::substep(int32_t method) {
     prepare_substep(method);
     ++substeps_launched_;
     if (use_graphs_ && !timing_ && !has_force_callbacks()) {
-        int const key = graph_key(method, reorder);
-        auto it = graphs_.find(key);
-        if (it == graphs_.end()) {
-            capture_substep(method, reorder);
-            it = graphs_.find(key);
-        }
-        if (cudaGraphLaunch(it->second, st_) != cudaSuccess) {
-            check("graph launch");
-            throw std::runtime_error("graph launch failed");
-        }
+        int const key = with_refusals([&] {
+            int const k = graph_key(method, reorder);
+            if (!graphs_.count(k)) capture_substep(method, reorder);
+            if (cudaGraphLaunch(graphs_[k], st_) != cudaSuccess) {
+                if (use_resident(method)) throw ResidentRefused();
+                check("graph launch");
+                throw std::runtime_error("graph launch failed");
+            }
+            return k;
+        });
         int64_t const fixed = graph_fixed_kernels_[key];
         host_launches_ += fixed;
         g_launches.fetch_add(fixed, std::memory_order_relaxed);

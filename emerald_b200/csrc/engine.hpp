@@ -255,6 +255,10 @@ private:
     // The resident solve (resident_kernels.cu): whether sub-steps of `method`
     // run it now, and its division of the active scenes among blocks.
     bool use_resident(int32_t method);
+    template <class F>
+    int with_refusals(F&& f);
+    bool refused_ = false;  // the device refuses the resident solve's launch
+    bool refuse_ = false;   // (injected)
     int graph_key(int32_t method, bool reorder);
     void plan_resident(int32_t method);
     void divide_scenes(uint32_t blocks);

@@ -316,10 +316,12 @@ int emerald_sim_kernel_times(emerald_sim* sim, char* names, size_t names_len, do
  * BARRIER_POLLS and VALUE_POLLS: how often a wait of the resident
  * solve's blocks for one another looks before it gives up (2^22); SORT_POLLS:
  * the same of the z-order sort's (a re-sort of the storage that gives up is
- * left out, emerald_sim_get_sort fails). */
+ * left out, emerald_sim_get_sort fails). REFUSE: not 0 stands for a device that
+ * refuses the resident solve's cooperative launch. */
 #define EMERALD_INJECT_BARRIER_POLLS 0
 #define EMERALD_INJECT_VALUE_POLLS 1
 #define EMERALD_INJECT_SORT_POLLS 2
+#define EMERALD_INJECT_REFUSE 3
 int emerald_sim_inject(emerald_sim* sim, int32_t what, uint32_t value);
 /* Execution mode: graphs != 0 (default) runs each sub-step as one CUDA graph
  * launch with the solver loops as conditional nodes; graphs == 0 launches

@@ -137,3 +137,25 @@ def test_storage_sort_that_gives_up_is_left_out(E):
     b.inject(E.INJECT_SORT_POLLS, POLLS)
     for x, y in zip(a.sort(), b.sort()):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("method", METHODS)
+@pytest.mark.parametrize("graphs", (True, False))
+def test_refused_launch_takes_the_kernels_per_phase(E, method, graphs):
+    """A device that refuses the cooperative launch steps a scene all the
+    same, from the first call on or from a later one."""
+    sc = scene(E, 97, 61)
+    want = E.Simulation.from_block_scene(sc)
+    want.frame(method)
+    want.advance(method, 3)
+    for early in (True, False):
+        sim = E.Simulation.from_block_scene(sc)
+        sim.set_graphs(graphs)
+        if early:
+            sim.inject(E.INJECT_REFUSE, 1)
+        assert sim.frame(method)["error_flags"] == 0
+        sim.inject(E.INJECT_REFUSE, 1)
+        assert sim.advance(method, 3)["error_flags"] == 0
+        for name, x, y in zip("xv", sim.state(), want.state()):
+            assert_bitwise(x, y, "%s %s" % (method, name))
+        sim.close()
