@@ -32,16 +32,28 @@ constexpr uint32_t kMinShare = 4;
 // the longest list of 32).
 constexpr uint32_t kHeldTiles = 56;
 // Between re-sorts of the storage a violent flow mixes the particles, and a
-// share's halo grows: the exchanges with it, and in the end it has no room. The
-// lists of a share above kTightShare tiles leave little of it, so those scenes
-// report the largest halo of their shares (256ths of the share, 0xffff when a
-// gang took the plain form), and above kDrifted they take the kernels per phase
-// until the storage is in order again. 262k DFSPH particles, a sub-step
-// resident against per phase: halo 63-67 (calm) 0.56-0.62 against 0.62-0.89 ms,
-// 78 1.08 and 0.92-0.98, 93-104 0.97-1.18 and 0.96-1.05, plain form 1.2-2.2 and
-// 1.0-1.3. At 8 tiles a share the resident solve stays ahead throughout.
-constexpr uint32_t kTightShare = 24;
-constexpr uint32_t kDrifted = 84;
+// share's halo grows: the exchanges with it, and in the end it has no room and
+// its gang takes the plain form (as it does where lists are cut at 64). Sub-steps
+// of shares above `plain` tiles are watched: after a plain form the kernels per
+// phase are faster; above `halo` tiles they also are after a halo of more than
+// kDriftRoots roots of the share's particles. Sub-step time resident / per
+// phase in the default dam break (60 sub-steps a frame, violent from the first)
+// on B200, by tiles a share, plain form / halo of 10 to 18 roots:
+//   DFSPH_P  6 0.76 / 0.52,  14 0.85 / 0.53,  20 1.02 / 0.60,  28 1.03 / 0.65,
+//            41 1.47 / 0.9 rising to 1.05 past 14 roots,  55 1.40 / 0.95 to 1.05,
+//            76 1.77 / 1.2,  104 1.78 / 1.14,  135 1.78 / 0.95
+//   AP       14 0.58 / 0.46,  23 0.72 / 0.55,  34 1.17 / 0.78,  55 1.15 / 0.98
+//   IISPH    14 never / 0.68,  23 1.68 / 1.02 (12 roots) to 1.15 (16)
+//   PCISPH   3.5 1.53 / 0.76,  8 1.48 / 0.75,  15 2.27 / 1.1
+// Eight such frames against the kernels per phase of the build before the
+// resident solve, without the watch: DFSPH_P 14 tiles 0.84, 20 1.01, 28 1.09,
+// 41 1.61, 55 1.62, 104 2.13; AP 23 0.86, 34 1.25, 55 1.38; IISPH 14 0.68,
+// 23 1.57; PCISPH 8 0.70, 15 1.22.
+struct DriftRule {
+    uint32_t plain, halo;
+};
+constexpr DriftRule kDriftRules[5] = {{12, 12}, {16, 16}, {28, 48}, {28, 48}, {16, 36}};
+constexpr uint32_t kDriftRoots = 14;
 // Batches of fewer warp tiles (2,048 particles) keep the launch-per-phase
 // kernels. The resident solve is the faster one there too (48 requests of 128
 // to 512 particles through one lane: 17.5 against 20.4 ms on B200), but a
@@ -94,8 +106,8 @@ uint32_t resident_smem(int method, uint32_t tiles, uint32_t most) {
     EMLD_RESIDENT(method, resident_smem_of, tiles, most)
 }
 cudaError_t launch_resident_solve(Arena const& a, ResidentPlan const& p, int method, bool comp,
-                                  cudaStream_t st) {
-    EMLD_RESIDENT(method, launch_resident_of, a, p, comp, st)
+                                  bool watched, cudaStream_t st) {
+    EMLD_RESIDENT(method, launch_resident_of, a, p, comp, watched, st)
 }
 #undef EMLD_RESIDENT
 
@@ -212,7 +224,7 @@ size_t Engine::footprint(uint32_t fluid_capacity, uint32_t solid_capacity, int m
              r(sizeof(unsigned long long) * kLoopSlots);
     bytes += r(4 * M) + r(4 * (M + 1)) + r(4);              // solver-loop work list
     size_t const parts = max_parts(uint32_t(N), int(M));    // resident solve
-    bytes += r(sizeof(GangState) * M) + 2 * r(4) + r(sizeof(GangPart) * parts) +
+    bytes += r(sizeof(GangState) * M) + r(sizeof(SolveControl)) + r(4 * 6) + r(sizeof(GangPart) * parts) +
              r(2 * sizeof(GangRecord) * parts);
     return bytes;
 }
@@ -335,9 +347,9 @@ Engine::Engine(uint32_t fluid_capacity, uint32_t solid_capacity, int max_scenes)
     cudaMemset(a_.loop_wt0, 0, 4);
     a_.batch = max_scenes_ > 1 ? 1 : 0;
     a_.gangs = static_cast<GangState*>(dev(sizeof(GangState) * max_scenes_));
-    a_.gang_ticket = static_cast<uint32_t*>(dev(8));
-    cudaMemset(a_.gang_ticket, 0, 8);
-    d_nparts_ = static_cast<uint32_t*>(dev(4));
+    a_.control = static_cast<SolveControl*>(dev(sizeof(SolveControl)));
+    cudaMemset(a_.control, 0, sizeof(SolveControl));
+    d_nparts_ = static_cast<uint32_t*>(dev(4 * 6));
     parts_cap_ = max_parts(fluid_cap_, max_scenes_);
     d_parts_ = static_cast<GangPart*>(dev(sizeof(GangPart) * parts_cap_));
     a_.records = static_cast<GangRecord*>(dev(2 * sizeof(GangRecord) * parts_cap_));
@@ -345,17 +357,20 @@ Engine::Engine(uint32_t fluid_capacity, uint32_t solid_capacity, int max_scenes)
         cudaStreamCreateWithFlags(&body_st_, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&frame_st_, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&side_st_, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&path_st_, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming) != cudaSuccess) {
         throw std::runtime_error("stream creation failed");
     }
     if (cudaMallocHost(reinterpret_cast<void**>(&h_running_), sizeof(int)) != cudaSuccess ||
         cudaMallocHost(reinterpret_cast<void**>(&h_flag_), sizeof(uint32_t)) != cudaSuccess ||
-        cudaMallocHost(reinterpret_cast<void**>(&h_gave_up_), sizeof(uint32_t)) != cudaSuccess) {
+        cudaMallocHost(reinterpret_cast<void**>(&h_gave_up_), 2 * sizeof(uint32_t)) !=
+          cudaSuccess) {
         throw std::bad_alloc();
     }
-    *h_gave_up_ = 0u;
+    h_gave_up_[0] = h_gave_up_[1] = 0u;
     a_.gave_up = h_gave_up_;
+    a_.drift_seen = h_gave_up_ + 1;
     a_.barrier_polls = a_.value_polls = kMaxPolls;
     cudaMemset(d_ss_, 0, sizeof(SceneState) * max_scenes_);
     cudaMemset(a_.vs, 0, 8 * S);
@@ -397,6 +412,7 @@ Engine::~Engine() {
     if (body_st_) cudaStreamDestroy(body_st_);
     if (frame_st_) cudaStreamDestroy(frame_st_);
     if (side_st_) cudaStreamDestroy(side_st_);
+    if (path_st_) cudaStreamDestroy(path_st_);
     if (ev_fork_) cudaEventDestroy(ev_fork_);
     if (ev_join_) cudaEventDestroy(ev_join_);
     for (auto& p : pending_) {
@@ -503,12 +519,17 @@ void Engine::upload_params(int id) {
     cudaMemcpyAsync(d_sp_ + id, &scenes_[id].p, sizeof(SceneParams), cudaMemcpyHostToDevice, st_);
 }
 
-// The scenes or their positions are new: what was known of the storage order's
-// drift is not theirs.
-void Engine::forget_drift() {
-    cudaMemsetAsync(a_.gang_ticket + 1, 0, 4, st_);
-    drifted_ = false;
-    retry_wait_ = retry_in_ = 0;
+// The engine's only scene is new, or has gone: what was known of the storage
+// order's drift was another's. (A batch keeps its record: the scenes in it go
+// on.) The new particles are not in the storage order yet.
+void Engine::scenes_changed(bool added) {
+    order_stale_ = order_stale_ || added;
+    int used = 0;
+    for (auto const& sc : scenes_) used += sc.used ? 1 : 0;
+    changing_ = max_scenes_ > 1 && (changing_ || substeps_launched_ > 0);
+    if (used > 1) return;
+    cudaMemsetAsync(a_.control, 0, sizeof(SolveControl), st_);
+    h_gave_up_[1] = 0u;
 }
 
 int Engine::add_scene(SceneSpec const& spec) {
@@ -631,7 +652,7 @@ int Engine::add_scene(SceneSpec const& spec) {
     }
     update_sort_bases();
     update_extent();
-    forget_drift();
+    scenes_changed(true);
     rebuild_solids();
     if (spec.n_solid) {
         if (spec.solid_volumes) {
@@ -765,7 +786,7 @@ void Engine::remove_scene(int id) {
     parts_valid_ = false;
     update_sort_bases();
     update_extent();
-    forget_drift();
+    scenes_changed(false);
     rebuild_solids();
 }
 
@@ -959,7 +980,8 @@ int64_t Engine::kernel_launches() {
     host_wait(st_);
     int64_t n = host_launches_;
     for (int k = 0; k < 4; ++k) n += int64_t(it[k]) * loop_kernels_[k];
-    for (int m = 0; m < 5; ++m) n += int64_t(it[4 + m]) * frame_body_kernels_[m];
+    for (int k = 0; k < 5 * kPaths; ++k) n += int64_t(it[kFrameSlots + k]) * frame_body_kernels_[k];
+    for (int m = 0; m < 5; ++m) n += int64_t(it[kChoiceSlots + m]) * choice_kernels_[m];
     return n;
 }
 
@@ -970,37 +992,10 @@ void Engine::run_loop(int kind, int max_iter, int32_t method) {
     if (capturing_) {
         // while (any scene iterates) { body; check } as a conditional node,
         // opened by the reset kernel every time the loop is reached
-        cudaStreamCaptureStatus status;
-        cudaGraph_t g = nullptr;
-        cudaGraphNode_t const* deps = nullptr;
-        size_t ndeps = 0;
-        if (cudaStreamGetCaptureInfo(cur_, &status, nullptr, &g, &deps, &ndeps) != cudaSuccess ||
-            status != cudaStreamCaptureStatusActive) {
-            throw std::runtime_error("graph capture: no active capture");
-        }
-        cudaGraphConditionalHandle cond;
-        if (cudaGraphConditionalHandleCreate(&cond, g, 1, cudaGraphCondAssignDefault) != cudaSuccess) {
-            throw std::runtime_error("graph capture: conditional handle");
-        }
+        cudaGraphConditionalHandle const cond = condition();
         launch("iter_reset", [&] { launch_iter_reset(a_, max_scenes_, kind, cur_, cond, 1); });
-        if (cudaStreamGetCaptureInfo(cur_, &status, nullptr, &g, &deps, &ndeps) != cudaSuccess ||
-            status != cudaStreamCaptureStatusActive) {
-            throw std::runtime_error("graph capture: no active capture");
-        }
-        cudaGraphNodeParams params{};
-        params.type = cudaGraphNodeTypeConditional;
-        params.conditional.handle = cond;
-        params.conditional.type = cudaGraphCondTypeWhile;
-        params.conditional.size = 1;
-        cudaGraphNode_t node;
-        if (cudaGraphAddNode(&node, g, deps, ndeps, &params) != cudaSuccess) {
-            throw std::runtime_error("graph capture: conditional node");
-        }
-        if (cudaStreamUpdateCaptureDependencies(cur_, &node, 1, cudaStreamSetCaptureDependencies) !=
-            cudaSuccess) {
-            throw std::runtime_error("graph capture: dependencies");
-        }
-        cudaGraph_t body = params.conditional.phGraph_out[0];
+        cudaGraph_t body;
+        conditional_node(cond, cudaGraphCondTypeWhile, &body);
         cudaStream_t const outer = cur_;
         if (cudaStreamBeginCaptureToGraph(body_st_, body, nullptr, nullptr, 0,
                                           cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
@@ -1037,10 +1032,14 @@ void Engine::emit_substep(int32_t method, bool reorder) {
         launch("reorder", [&] { launch_reorder(a_, order_sort_, tiles * kTile, bits, st); },
                3 + 3 * (bits / 8));
     }
-    bool const resident = use_resident(method);
+    int const path = path_;
+    cudaGraphConditionalHandle cond = 0;
+    if (path == kWatched && capturing_) cond = condition();
+    SolveChoice const choice{d_nparts_ + 1 + method, cond, capturing_ ? 1 : 0,
+                             kChoiceSlots + method};
     auto begin = [&](cudaStream_t s) {
         launch("max_v2", [&] { launch_max_v2(a_, tiles, s); });
-        launch("begin_substep", [&] { launch_begin_substep(a_, max_scenes_, resident, s); });
+        launch("begin_substep", [&] { launch_begin_substep(a_, max_scenes_, path, choice, s); });
     };
     Arena const ext = extent_arena();
     bool const kernels = method != kPcisph;
@@ -1068,21 +1067,109 @@ void Engine::emit_substep(int32_t method, bool reorder) {
         launch("neighbors_solid",
                [&] { launch_neighbors(a_, tiles, true, kernels, st, compensated_); });
     }
-    if (resident) {
-        cudaError_t e = cudaSuccess;
-        launch("solve", [&] {
-            e = refuse_ ? cudaErrorCooperativeLaunchTooLarge
-                        : launch_resident_solve(a_, plans_[method], method, compensated_, st);
-        });
-        if (e == cudaSuccess) return;
-        cudaGetLastError();
-        if (capturing_) throw ResidentRefused();
-        // nothing of the solve has run: the kernels per phase do it
-        refused_ = true;
-        for (int id = 0; id < max_scenes_; ++id) {
-            if (scenes_[id].used) launch_clear_stall(a_, id, st);
-        }
+    if (path == kPhases) return emit_phases(method);
+    if (path == kResident || path == kReported) return emit_resident(method);
+    if (!capturing_) {
+        cudaMemcpyAsync(h_running_, &a_.control->drifted, 4, cudaMemcpyDeviceToHost, st);
+        host_wait(st);
+        return *h_running_ ? emit_phases(method) : emit_resident(method);
     }
+    // Both side by side: the resident solve, which returns at once where the
+    // choice is the other, and a node that holds the kernels per phase and is
+    // passed over where it is not. (Two bodies of one node, the solve in the
+    // first, cost a sub-step of 700 us another 12 us.)
+    cudaEventRecord(ev_fork_, st);
+    cudaStreamWaitEvent(side_st_, ev_fork_, 0);
+    cur_ = side_st_;
+    emit_resident(method);
+    cur_ = st;
+    cudaEventRecord(ev_join_, side_st_);
+    cudaGraph_t body;
+    conditional_node(cond, cudaGraphCondTypeIf, &body);
+    if (cudaStreamBeginCaptureToGraph(path_st_, body, nullptr, nullptr, 0,
+                                      cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+        throw std::runtime_error("graph capture: path");
+    }
+    int64_t const outside = capture_kernels_;
+    cur_ = path_st_;
+    emit_phases(method);
+    cur_ = st;
+    choice_kernels_[method] = capture_kernels_ - outside;
+    capture_kernels_ = outside;
+    if (cudaStreamEndCapture(path_st_, &body) != cudaSuccess) {
+        throw std::runtime_error("graph capture: path end");
+    }
+    cudaStreamWaitEvent(st, ev_join_, 0);
+}
+
+// A condition of the graph that cur_ is recording.
+cudaGraphConditionalHandle Engine::condition() {
+    cudaStreamCaptureStatus status;
+    cudaGraph_t g = nullptr;
+    cudaGraphNode_t const* deps = nullptr;
+    size_t ndeps = 0;
+    cudaGraphConditionalHandle cond;
+    if (cudaStreamGetCaptureInfo(cur_, &status, nullptr, &g, &deps, &ndeps) != cudaSuccess ||
+        status != cudaStreamCaptureStatusActive) {
+        throw std::runtime_error("graph capture: no active capture");
+    }
+    if (cudaGraphConditionalHandleCreate(&cond, g, 1, cudaGraphCondAssignDefault) != cudaSuccess) {
+        throw std::runtime_error("graph capture: conditional handle");
+    }
+    return cond;
+}
+
+// Adds a conditional node behind what cur_ has recorded.
+void Engine::conditional_node(cudaGraphConditionalHandle cond, cudaGraphConditionalNodeType type,
+                              cudaGraph_t* body) {
+    cudaStreamCaptureStatus status;
+    cudaGraph_t g = nullptr;
+    cudaGraphNode_t const* deps = nullptr;
+    size_t ndeps = 0;
+    if (cudaStreamGetCaptureInfo(cur_, &status, nullptr, &g, &deps, &ndeps) != cudaSuccess ||
+        status != cudaStreamCaptureStatusActive) {
+        throw std::runtime_error("graph capture: no active capture");
+    }
+    cudaGraphNodeParams params{};
+    params.type = cudaGraphNodeTypeConditional;
+    params.conditional.handle = cond;
+    params.conditional.type = type;
+    params.conditional.size = 1;
+    cudaGraphNode_t node;
+    if (cudaGraphAddNode(&node, g, deps, ndeps, &params) != cudaSuccess) {
+        throw std::runtime_error("graph capture: conditional node");
+    }
+    if (cudaStreamUpdateCaptureDependencies(cur_, &node, 1, cudaStreamSetCaptureDependencies) !=
+        cudaSuccess) {
+        throw std::runtime_error("graph capture: dependencies");
+    }
+    *body = params.conditional.phGraph_out[0];
+}
+
+// The solve as one cooperative launch.
+void Engine::emit_resident(int32_t method) {
+    cudaStream_t const st = cur_;
+    cudaError_t e = cudaSuccess;
+    launch("solve", [&] {
+        e = refuse_ ? cudaErrorCooperativeLaunchTooLarge
+                    : launch_resident_solve(a_, plans_[method], method, compensated_,
+                                            capturing_ && path_ == kWatched, st);
+    });
+    if (e == cudaSuccess) return;
+    cudaGetLastError();
+    if (capturing_) throw ResidentRefused();
+    // nothing of the solve has run: the kernels per phase do it
+    refused_ = true;
+    for (int id = 0; id < max_scenes_; ++id) {
+        if (scenes_[id].used) launch_clear_stall(a_, id, st);
+    }
+    emit_phases(method);
+}
+
+// The solve as kernels per phase.
+void Engine::emit_phases(int32_t method) {
+    uint32_t const tiles = ext_tiles_;
+    cudaStream_t const st = cur_;
     switch (method) {
     case kDfsph:
         launch("dfsph_density_alpha", [&] {
@@ -1123,6 +1210,21 @@ void Engine::emit_substep(int32_t method, bool reorder) {
     }
 }
 
+void Engine::abort_capture() {
+    for (cudaStream_t sst : {body_st_, path_st_, frame_st_, cap_st_}) {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(sst, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) {
+            cudaGraph_t dead = nullptr;
+            cudaStreamEndCapture(sst, &dead);
+            // (the graphs of the conditional nodes belong to the outermost one)
+            if (dead && sst == cap_st_) cudaGraphDestroy(dead);
+        }
+    }
+    cudaGetLastError();
+    capturing_ = false;
+    cur_ = st_;
+}
+
 // Records one sub-step of `method` into a graph. Kernel arguments are the
 // arena pointers and the tile count, which never change for an engine, and
 // every kernel reads scene membership and parameters from device memory, so
@@ -1138,11 +1240,7 @@ void Engine::capture_substep(int32_t method, bool reorder) {
     try {
         emit_substep(method, reorder);
     } catch (...) {
-        cudaGraph_t g = nullptr;
-        cudaStreamEndCapture(cap_st_, &g);
-        if (g) cudaGraphDestroy(g);
-        capturing_ = false;
-        cur_ = st_;
+        abort_capture();
         throw;
     }
     capturing_ = false;
@@ -1155,7 +1253,7 @@ void Engine::capture_substep(int32_t method, bool reorder) {
     cudaError_t const e = cudaGraphInstantiate(&exec, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) {
-        if (use_resident(method)) throw ResidentRefused();
+        if (path_ != kPhases) throw ResidentRefused();
         throw std::runtime_error(std::string("graph instantiate: ") + cudaGetErrorString(e));
     }
     graphs_[graph_key(method, reorder)] = exec;
@@ -1176,20 +1274,6 @@ void Engine::capture_frame(int32_t method, bool reorder) {
     capture_kernels_ = 0;
     cur_ = cap_st_;
     cudaGraph_t g = nullptr;
-    auto abort = [&] {
-        for (cudaStream_t sst : {body_st_, frame_st_, cap_st_}) {
-            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-            if (cudaStreamIsCapturing(sst, &cs) == cudaSuccess &&
-                cs != cudaStreamCaptureStatusNone) {
-                cudaGraph_t dead = nullptr;
-                cudaStreamEndCapture(sst, &dead);
-                if (dead) cudaGraphDestroy(dead);
-            }
-        }
-        cudaGetLastError();
-        capturing_ = false;
-        cur_ = st_;
-    };
     try {
         launch("frame_begin", [&] { launch_frame_begin(a_, max_scenes_, cap_st_); });
         if (reorder) {
@@ -1198,49 +1282,27 @@ void Engine::capture_frame(int32_t method, bool reorder) {
                    [&] { launch_reorder(a_, order_sort_, ext_tiles_ * kTile, bits, cap_st_); },
                    3 + 3 * (bits / 8));
         }
-        cudaStreamCaptureStatus status;
-        cudaGraph_t outer = nullptr;
-        cudaGraphNode_t const* deps = nullptr;
-        size_t ndeps = 0;
-        if (cudaStreamGetCaptureInfo(cap_st_, &status, nullptr, &outer, &deps, &ndeps) !=
-              cudaSuccess ||
-            status != cudaStreamCaptureStatusActive) {
-            throw std::runtime_error("frame capture: no active capture");
-        }
-        cudaGraphConditionalHandle cond;
-        if (cudaGraphConditionalHandleCreate(&cond, outer, 1, cudaGraphCondAssignDefault) !=
-            cudaSuccess) {
-            throw std::runtime_error("frame capture: conditional handle");
-        }
-        cudaGraphNodeParams params{};
-        params.type = cudaGraphNodeTypeConditional;
-        params.conditional.handle = cond;
-        params.conditional.type = cudaGraphCondTypeWhile;
-        params.conditional.size = 1;
-        cudaGraphNode_t node;
-        if (cudaGraphAddNode(&node, outer, deps, ndeps, &params) != cudaSuccess ||
-            cudaStreamUpdateCaptureDependencies(cap_st_, &node, 1,
-                                                cudaStreamSetCaptureDependencies) != cudaSuccess) {
-            throw std::runtime_error("frame capture: conditional node");
-        }
-        cudaGraph_t body = params.conditional.phGraph_out[0];
+        cudaGraphConditionalHandle const cond = condition();
+        cudaGraph_t body;
+        conditional_node(cond, cudaGraphCondTypeWhile, &body);
         if (cudaStreamBeginCaptureToGraph(frame_st_, body, nullptr, nullptr, 0,
                                           cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
             throw std::runtime_error("frame capture: body");
         }
         int64_t const outside = capture_kernels_;
+        int const slot = method * kPaths + path_;
         cur_ = frame_st_;
         emit_substep(method, false);
         launch("frame_check",
-               [&] { launch_frame_check(a_, max_scenes_, method, cond, frame_st_); });
-        frame_body_kernels_[method] = capture_kernels_ - outside;
+               [&] { launch_frame_check(a_, max_scenes_, kFrameSlots + slot, cond, frame_st_); });
+        frame_body_kernels_[slot] = capture_kernels_ - outside;
         capture_kernels_ = outside;
         if (cudaStreamEndCapture(frame_st_, &body) != cudaSuccess) {
             throw std::runtime_error("frame capture: body end");
         }
         cur_ = cap_st_;
     } catch (...) {
-        abort();
+        abort_capture();
         throw;
     }
     capturing_ = false;
@@ -1252,7 +1314,7 @@ void Engine::capture_frame(int32_t method, bool reorder) {
     cudaError_t const e = cudaGraphInstantiate(&exec, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) {
-        if (use_resident(method)) throw ResidentRefused();
+        if (path_ != kPhases) throw ResidentRefused();
         throw std::runtime_error(std::string("frame graph instantiate: ") + cudaGetErrorString(e));
     }
     frame_graphs_[graph_key(method, reorder)] = exec;
@@ -1268,6 +1330,7 @@ int Engine::with_refusals(F&& f) {
     } catch (ResidentRefused const&) {
         cudaGetLastError();
         refused_ = true;
+        path_ = kPhases;
         destroy_graphs();
         return f();
     }
@@ -1286,8 +1349,7 @@ int Engine::frame(int id, int32_t method, SceneState& out) {
         return n;
     }
     check_solved(-1);
-    bool const reorder = reorder_every_ > 0 && (frames_launched_ % 2) == 0;
-    if (reorder) storage_in_order();
+    bool const reorder = reorder_every_ > 0 && (frames_launched_ % 2 == 0 || order_stale_);
     prepare_substep(method);
     ++frames_launched_;
     int key;
@@ -1304,7 +1366,7 @@ int Engine::frame(int id, int32_t method, SceneState& out) {
                 }
             }
             if (cudaGraphLaunch(frame_graphs_[k], st_) != cudaSuccess) {
-                if (use_resident(method)) throw ResidentRefused();
+                if (path_ != kPhases) throw ResidentRefused();
                 check("frame graph launch");
                 throw std::runtime_error("frame graph launch failed");
             }
@@ -1317,6 +1379,7 @@ int Engine::frame(int id, int32_t method, SceneState& out) {
         --frames_launched_;
         return frame(id, method, out);
     }
+    order_stale_ = order_stale_ && !reorder;
     int64_t const fixed = frame_fixed_kernels_[key];
     host_launches_ += fixed;
     g_launches.fetch_add(fixed, std::memory_order_relaxed);
@@ -1364,11 +1427,12 @@ void Engine::prepare_substep(int32_t method) {
             upload_params(id);
         }
     }
-    if (use_resident(method)) plan_resident(method);
+    path_ = solve_path(method);
+    if (path_ != kPhases) plan_resident(method);
 }
 
 int Engine::graph_key(int32_t method, bool reorder) {
-    return method * 4 + (reorder ? 2 : 0) + (use_resident(method) ? 1 : 0);
+    return (method * 2 + (reorder ? 1 : 0)) * kPaths + path_;
 }
 
 ResidentLimits const& Engine::limits_of(int32_t method) {
@@ -1393,8 +1457,19 @@ bool Engine::use_resident(int32_t method) {
     ResidentLimits const& lim = limits_of(method);
     if (!lim.blocks) return false;
     if (!parts_valid_) divide_scenes(lim.blocks);
-    if (max_scenes_ == 1) return largest_share_ <= lim.share && !(drifted_ && watch_drift_);
+    if (max_scenes_ == 1) return largest_share_ <= lim.share;
     return total_tiles_ >= kMinBatchTiles && largest_share_ <= std::min(kHeldTiles, lim.share);
+}
+
+int Engine::solve_path(int32_t method) {
+    if (!use_resident(method)) return kPhases;
+    if (!drift_limit_[method]) return kResident;
+    // A batch whose scenes come and go records its graphs often, and one that
+    // holds both solves takes a millisecond more than one with the resident
+    // solve alone (16 served requests 16.8 against 18.0 ms): it gets the former
+    // when a drift has been reported.
+    bool const seen = reinterpret_cast<uint32_t volatile*>(h_gave_up_)[1] != 0u;
+    return changing_ && !seen ? kReported : kWatched;
 }
 
 // Divides the active scenes' warp tiles among the resident blocks: a scene's
@@ -1434,11 +1509,18 @@ void Engine::divide_scenes(uint32_t blocks) {
             largest_share_ = std::max(largest_share_, e - b);
         }
     }
-    watch_drift_ = max_scenes_ == 1 && largest_share_ > kTightShare;
+    for (int m = 0; m < 5; ++m) {
+        DriftRule const& rule = kDriftRules[m];
+        drift_limit_[m] = largest_share_ > rule.halo    ? 16u * kDriftRoots
+                          : largest_share_ > rule.plain ? kPlainForm - 1u
+                                                        : 0u;
+    }
     if (parts_.size() > parts_cap_) throw std::runtime_error("resident solve: too many shares");
     uint32_t const n = uint32_t(parts_.size());
     cudaMemcpyAsync(d_parts_, parts_.data(), sizeof(GangPart) * n, cudaMemcpyHostToDevice, st_);
-    cudaMemcpyAsync(d_nparts_, &n, 4, cudaMemcpyHostToDevice, st_);
+    uint32_t words[6] = {n};
+    std::copy(drift_limit_, drift_limit_ + 5, words + 1);
+    cudaMemcpyAsync(d_nparts_, words, sizeof(words), cudaMemcpyHostToDevice, st_);
     parts_valid_ = true;
 }
 
@@ -1463,29 +1545,20 @@ void Engine::plan_resident(int32_t method) {
     now = p;
 }
 
-// The storage is about to be put in order: a scene that had drifted gets
-// another chance, the later the more often it has drifted in a row.
-void Engine::storage_in_order() {
-    if (!drifted_) {
-        retry_wait_ = 0;
-    } else if (retry_in_-- <= 0) {
-        drifted_ = false;
-    }
-}
-
 void Engine::substep(int32_t method) {
     if (active_scenes() == 0) return;
     check_solved(-1);
-    bool const reorder = reorder_every_ > 0 && (substeps_launched_ % reorder_every_) == 0;
-    if (reorder) storage_in_order();
+    bool const reorder =
+      reorder_every_ > 0 && (substeps_launched_ % reorder_every_ == 0 || order_stale_);
     prepare_substep(method);
     ++substeps_launched_;
+    order_stale_ = order_stale_ && !reorder;
     if (use_graphs_ && !timing_ && !has_force_callbacks()) {
         int const key = with_refusals([&] {
             int const k = graph_key(method, reorder);
             if (!graphs_.count(k)) capture_substep(method, reorder);
             if (cudaGraphLaunch(graphs_[k], st_) != cudaSuccess) {
-                if (use_resident(method)) throw ResidentRefused();
+                if (path_ != kPhases) throw ResidentRefused();
                 check("graph launch");
                 throw std::runtime_error("graph launch failed");
             }
@@ -1522,6 +1595,7 @@ Engine::TuneReport Engine::autotune(int32_t method, int substeps) {
     Region const regions[] = {{a_.x, 8 * N},      {a_.v, 8 * N},         {a_.kdiv, 4 * N},
                               {a_.kdens, 4 * N},  {a_.x64, 16 * N},      {a_.oid, 4 * N},
                               {a_.slot_of, 4 * N}, {d_ss_, sizeof(SceneState) * size_t(max_scenes_)},
+                              {a_.control, sizeof(SolveControl)},
                               {d_loop_iters_, sizeof(unsigned long long) * kLoopSlots}};
     size_t bytes = 0;
     for (auto const& r : regions) bytes += r.size;
@@ -1543,6 +1617,7 @@ Engine::TuneReport Engine::autotune(int32_t method, int substeps) {
     };
     copy(true);
     int64_t const launched0 = substeps_launched_;
+    bool const stale0 = order_stale_;
     int64_t const host0 = host_launches_;
     int64_t const global0 = g_launches.load();
     std::vector<Tuning> cand;
@@ -1614,6 +1689,7 @@ Engine::TuneReport Engine::autotune(int32_t method, int substeps) {
         for (int q = 0; q < substeps; ++q) substep(method);
         copy(false);
         substeps_launched_ = launched0;
+        order_stale_ = stale0;
         cudaEventRecord(e0, st_);
         for (int q = 0; q < substeps; ++q) substep(method);
         cudaEventRecord(e1, st_);
@@ -1623,6 +1699,7 @@ Engine::TuneReport Engine::autotune(int32_t method, int substeps) {
         cudaEventElapsedTime(&ms, e0, e1);
         copy(false);
         substeps_launched_ = launched0;
+        order_stale_ = stale0;
         return ms / float(substeps);
     };
     try {
@@ -1677,19 +1754,9 @@ void Engine::set_tuning(Tuning const* t) {
 
 SceneState Engine::scene_state(int id) {
     SceneState s{};
-    uint32_t drift = 0;
     cudaMemcpyAsync(&s, d_ss_ + id, sizeof(SceneState), cudaMemcpyDeviceToHost, st_);
-    if (watch_drift_) {
-        cudaMemcpyAsync(&drift, a_.gang_ticket + 1, 4, cudaMemcpyDeviceToHost, st_);
-        cudaMemsetAsync(a_.gang_ticket + 1, 0, 4, st_);
-    }
     host_wait(st_);
     check("scene_state");
-    if (watch_drift_ && drift > kDrifted) {
-        drifted_ = true;
-        retry_wait_ = std::min(2 * retry_wait_ + 1, 31);
-        retry_in_ = retry_wait_;
-    }
     check_solved(id);
     return s;
 }
@@ -1743,7 +1810,10 @@ bool Engine::set_state(int id, float const* x, float const* v, bool sync) {
     if (x) {
         launch_scatter_f2(a_, b, n, a_.tx + b, a_.x, st_);
         launch_positions_to_double(a_, b, n, st_);
-        if (watch_drift_) forget_drift();
+        // another flow, perhaps: the next re-sort gives it a try
+        if (drift_limit_[scenes_[id].p.method]) {
+            cudaMemsetAsync(&a_.control->wait, 0, 8, st_);  // and left
+        }
     }
     if (v) launch_scatter_f2(a_, b, n, a_.tv + b, a_.v, st_);
     if (x && v && gave_up()) launch_clear_stall(a_, id, st_);

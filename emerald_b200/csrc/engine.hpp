@@ -245,6 +245,12 @@ private:
     void upload_tiles();
     void run_loop(int kind, int max_iter, int32_t method);
     void emit_substep(int32_t method, bool reorder);
+    void emit_resident(int32_t method);
+    void emit_phases(int32_t method);
+    cudaGraphConditionalHandle condition();
+    void conditional_node(cudaGraphConditionalHandle cond, cudaGraphConditionalNodeType type,
+                          cudaGraph_t* body);
+    void abort_capture();
     void emit_loop_body(int kind, int32_t method, cudaGraphConditionalHandle cond, bool use_cond);
     void capture_substep(int32_t method, bool reorder);
     void update_sort_bases();
@@ -275,20 +281,23 @@ private:
     std::vector<GangPart> parts_;
     bool parts_valid_ = false;  // false: the scenes changed since parts_ was made
     uint32_t largest_share_ = 1;
-    void storage_in_order();
-    void forget_drift();
-    bool watch_drift_ = false;  // the share is large enough for drift to matter
-    bool drifted_ = false;      // kernels per phase until storage is in order again
-    int retry_wait_ = 0;        // re-sorts to let pass after the next drift
-    int retry_in_ = 0;
+    // How sub-steps of `method` are solved now (a SolvePath); path_: how this
+    // call's are.
+    int solve_path(int32_t method);
+    int path_ = kPhases;
+    void scenes_changed(bool added);
+    bool order_stale_ = false;              // particles were added since the last re-sort
+    uint32_t drift_limit_[5] = {0, 0, 0, 0, 0};  // per method; 0: not watched
+    bool changing_ = false;  // a batch whose scenes come and go
     uint64_t total_tiles_ = 0;
     GangPart* d_parts_ = nullptr;
-    uint32_t* d_nparts_ = nullptr;
+    uint32_t* d_nparts_ = nullptr;  // the shares, then the methods' drift limits
     uint32_t parts_cap_ = 0;
     cudaStream_t frame_st_ = nullptr;                  // frame-loop body capture
     std::map<int32_t, cudaGraphExec_t> frame_graphs_;  // key: graph_key
     std::map<int32_t, int64_t> frame_fixed_kernels_;   // per graph, outside the loop
-    int64_t frame_body_kernels_[5] = {0, 0, 0, 0, 0};  // per method, one frame iteration
+    int64_t frame_body_kernels_[5 * kPaths] = {};  // per method and path, one frame iteration
+    int64_t choice_kernels_[5] = {};       // per method, those of a watched sub-step's node
     int max_iterations(int kind) const;
     void rebuild_solids();
     // Boundary-proximity map of a scene from its boundary positions.
@@ -317,7 +326,7 @@ private:
     int* h_running_ = nullptr;
     uint32_t* d_flag_ = nullptr;
     uint32_t* h_flag_ = nullptr;
-    uint32_t* h_gave_up_ = nullptr;  // written by the resident solve
+    uint32_t* h_gave_up_ = nullptr;  // two words, written by kernels: gave_up, drift_seen
     bool gave_up() const { return *reinterpret_cast<uint32_t volatile*>(h_gave_up_) != 0u; }
     unsigned int* d_check_counter_ = nullptr;  // finished blocks of a fused exit test
     int loop_kernels_[4] = {3, 3, 3, 4};        // kernels per iteration of each loop kind
@@ -333,6 +342,7 @@ private:
     cudaStream_t cap_st_ = nullptr;
     cudaStream_t body_st_ = nullptr;
     cudaStream_t side_st_ = nullptr;  // parallel branch of a sub-step
+    cudaStream_t path_st_ = nullptr;  // the two ways to solve a watched sub-step
     cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
     std::map<int32_t, cudaGraphExec_t> graphs_;        // key: graph_key
     std::map<int32_t, int64_t> graph_fixed_kernels_;

@@ -23,7 +23,10 @@ namespace emerald {
 constexpr int kTile = 128;
 constexpr int kMaxNeighbors = 64;
 constexpr uint64_t kEmptyKey = ~0ull;
-constexpr int kLoopSlots = 9;  // Arena::loop_iterations entries
+// Arena::loop_iterations entries: iterations of the four loop kinds, frame
+// graphs' sub-steps by method and path, and watched sub-steps that chose the
+// kernels per phase by method.
+constexpr int kFrameSlots = 4, kChoiceSlots = 4 + 5 * 4, kLoopSlots = 4 + 5 * 4 + 5;
 
 enum Method : int { kPcisph = 0, kIisph = 1, kIisphAp = 2, kIisphPseudoAp = 3, kDfsph = 4 };
 
@@ -142,6 +145,22 @@ struct GangPart {
     uint32_t base;  // index of the gang's first share
 };
 
+// Of the resident solve, per engine. What follows `ticket` decides between it
+// and the kernels per phase where a drifted storage order makes the latter
+// faster (choose_solve).
+struct SolveControl {
+    uint32_t ticket;    // the next share to take
+    uint32_t drift;     // the largest reported since the last choice
+    uint32_t in_order;  // the storage has been sorted since the last choice
+    uint32_t drifted;   // the choice: 1 for the kernels per phase
+    uint32_t wait;      // re-sorts to let pass after the next drift
+    uint32_t left;      // and still to pass after this one
+};
+// SolveControl::drift: neighbours outside the share in 16ths of the root of its
+// particles (the storage order in order: about 10.5 roots), or that a gang took
+// the plain form.
+constexpr uint32_t kPlainForm = 0xffffu;
+
 // Raw device pointers of an arena, passed by value to every kernel.
 struct Arena {
     SceneParams const* sp;
@@ -156,12 +175,13 @@ struct Arena {
     int32_t* loop_scene;
     uint32_t* loop_wt0;
     uint32_t* loop_n;
-    // resident solve: per-scene gang states, the next share to take, and the
-    // shares' error records (two each)
+    // resident solve: per-scene gang states, the engine's control words, and
+    // the shares' error records (two each)
     GangState* gangs;
-    uint32_t* gang_ticket;  // and, after it, the largest drift reported since the host last looked
+    SolveControl* control;
     GangRecord* records;
     uint32_t* gave_up;       // host memory: some wait of a resident solve has given up
+    uint32_t* drift_seen;    // host memory: a resident solve has reported a drift above its limit
     uint32_t barrier_polls;  // polls of a barrier, and of a value, before it gives up
     uint32_t value_polls;
     int32_t batch;  // the arena holds more than one scene slot (loop kernels walk the work list)

@@ -88,9 +88,20 @@ void launch_max_v2(Arena const& a, uint32_t tiles, cudaStream_t st);
 // frame graphs: zero the per-launch sub-step counts; after each sub-step,
 // count it and set `cond` while an active scene's frame has sub-steps left
 void launch_frame_begin(Arena const& a, int nscenes, cudaStream_t st);
-void launch_frame_check(Arena const& a, int nscenes, int method, cudaGraphConditionalHandle cond,
+void launch_frame_check(Arena const& a, int nscenes, int slot, cudaGraphConditionalHandle cond,
                         cudaStream_t st);
-void launch_begin_substep(Arena const& a, int nscenes, bool resident, cudaStream_t st);
+// How a sub-step is solved: by the kernels per phase, the resident solve,
+// whichever of the two its first kernel chooses, or the resident solve while
+// that kernel tells the host (Arena::drift_seen) when it would choose otherwise.
+enum SolvePath : int { kPhases = 0, kResident = 1, kWatched = 2, kReported = 3, kPaths = 4 };
+struct SolveChoice {
+    uint32_t const* limit;  // device: drift above which the kernels per phase are faster
+    cudaGraphConditionalHandle cond;  // of their node (use_cond: inside a graph)
+    int use_cond;
+    int slot;  // of Arena::loop_iterations that counts them
+};
+void launch_begin_substep(Arena const& a, int nscenes, int path, SolveChoice const& choice,
+                          cudaStream_t st);
 void launch_zero_kappas(Arena const& a, uint32_t tiles, cudaStream_t st);
 // use_cond: also set `cond` (the loop's while condition) to 1
 void launch_iter_reset(Arena const& a, int nscenes, int kind, cudaStream_t st,
@@ -181,7 +192,9 @@ bool resident_limits_of(bool comp, ResidentLimits& l);
 // tiles: room for 24 list rows a tile, `most` at most.
 template <int METHOD>
 uint32_t resident_smem_of(uint32_t tiles, uint32_t most);
+// `watched`: returns at once where the kernels per phase were chosen.
 template <int METHOD>
-cudaError_t launch_resident_of(Arena const& a, ResidentPlan const& p, bool comp, cudaStream_t st);
+cudaError_t launch_resident_of(Arena const& a, ResidentPlan const& p, bool comp, bool watched,
+                               cudaStream_t st);
 
 }  // namespace emerald

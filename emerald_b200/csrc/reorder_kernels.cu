@@ -65,6 +65,7 @@ __global__ void k_permute(Arena a, uint64_t const* keys, uint32_t const* vals, u
 __global__ void k_commit_order(Arena a, uint32_t n, uint32_t const* gave_up) {
     uint32_t const t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n || sort_gave_up(gave_up)) return;
+    if (t == 0) a.control->in_order = 1u;
     int32_t const s = a.tile_scene[t / kTile];
     if (s < 0) return;
     SceneParams const& P = a.sp[s];

@@ -6,7 +6,7 @@ namespace emerald {
 
 template bool resident_limits_of<kDfsph>(bool, ResidentLimits&);
 template uint32_t resident_smem_of<kDfsph>(uint32_t, uint32_t);
-template cudaError_t launch_resident_of<kDfsph>(Arena const&, ResidentPlan const&, bool,
+template cudaError_t launch_resident_of<kDfsph>(Arena const&, ResidentPlan const&, bool, bool,
                                             cudaStream_t);
 
 }  // namespace emerald

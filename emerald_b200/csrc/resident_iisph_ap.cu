@@ -6,7 +6,7 @@ namespace emerald {
 
 template bool resident_limits_of<kIisphAp>(bool, ResidentLimits&);
 template uint32_t resident_smem_of<kIisphAp>(uint32_t, uint32_t);
-template cudaError_t launch_resident_of<kIisphAp>(Arena const&, ResidentPlan const&, bool,
+template cudaError_t launch_resident_of<kIisphAp>(Arena const&, ResidentPlan const&, bool, bool,
                                             cudaStream_t);
 
 }  // namespace emerald

@@ -6,7 +6,7 @@ namespace emerald {
 
 template bool resident_limits_of<kIisphPseudoAp>(bool, ResidentLimits&);
 template uint32_t resident_smem_of<kIisphPseudoAp>(uint32_t, uint32_t);
-template cudaError_t launch_resident_of<kIisphPseudoAp>(Arena const&, ResidentPlan const&, bool,
+template cudaError_t launch_resident_of<kIisphPseudoAp>(Arena const&, ResidentPlan const&, bool, bool,
                                             cudaStream_t);
 
 }  // namespace emerald

@@ -6,7 +6,7 @@ namespace emerald {
 
 template bool resident_limits_of<kPcisph>(bool, ResidentLimits&);
 template uint32_t resident_smem_of<kPcisph>(uint32_t, uint32_t);
-template cudaError_t launch_resident_of<kPcisph>(Arena const&, ResidentPlan const&, bool,
+template cudaError_t launch_resident_of<kPcisph>(Arena const&, ResidentPlan const&, bool, bool,
                                             cudaStream_t);
 
 }  // namespace emerald

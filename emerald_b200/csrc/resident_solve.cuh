@@ -549,9 +549,10 @@ __device__ __forceinline__ void stage_lists(Arena const& a, Layout const& l, Sha
     block_sync();
     if (threadIdx.x == 0) {
         s.halo_n = min(s.halo_n, l.halo_max);
-        // how far the storage order has drifted, for the host's choice of path
-        uint32_t const drift = s.plain ? 0xffffu : s.halo_n * 256u / max(sh.own(), 1u);
-        atomicMax(a.gang_ticket + 1, drift);
+        // how far the storage order has drifted, for the choice of path
+        uint32_t const drift = static_cast<uint32_t>(
+          16.0f * static_cast<float>(s.halo_n) / sqrtf(static_cast<float>(max(sh.own(), 1u))));
+        atomicMax(&a.control->drift, s.plain ? kPlainForm : min(drift, kPlainForm - 1u));
     }
 }
 
@@ -1530,12 +1531,13 @@ __device__ __forceinline__ bool solve(Arena const& a, Layout const& l, Share& sh
 // kErrUnsolved that k_begin_substep gave it.
 template <int METHOD, int MODE, int FORM>
 __global__ void __launch_bounds__(Form<METHOD, MODE, FORM>::kThreads, 1)
-  k_resident_solve(Arena a, GangPart const* parts, uint32_t const* nparts, Layout l) {
+  k_resident_solve(Arena a, GangPart const* parts, uint32_t const* nparts, Layout l, int watched) {
     __shared__ Shared s;
+    if (watched && a.control->drifted) return;
     for (;;) {
         block_sync();
         if (threadIdx.x == 0) {
-            s.ticket = atomicAdd(a.gang_ticket, 1u);
+            s.ticket = atomicAdd(&a.control->ticket, 1u);
             s.used = 0u;
             s.wanted = 0u;
             s.halo_n = 0u;
@@ -1630,7 +1632,7 @@ constexpr uint32_t best_share(int method) {
 }
 
 template <int METHOD, int MODE, int FORM>
-cudaError_t launch_form(Arena const& a, ResidentPlan const& p, cudaStream_t st) {
+cudaError_t launch_form(Arena const& a, ResidentPlan const& p, bool watched, cudaStream_t st) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(p.grid);
     cfg.blockDim = dim3(p.threads);
@@ -1642,16 +1644,16 @@ cudaError_t launch_form(Arena const& a, ResidentPlan const& p, cudaStream_t st) 
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k_resident_solve<METHOD, MODE, FORM>, a, p.parts, p.nparts,
-                              layout_for(METHOD, p.share, p.smem));
+                              layout_for(METHOD, p.share, p.smem), watched ? 1 : 0);
 }
 
 template <int METHOD, int MODE>
-cudaError_t launch_one(Arena const& a, ResidentPlan const& p, cudaStream_t st) {
+cudaError_t launch_one(Arena const& a, ResidentPlan const& p, bool watched, cudaStream_t st) {
     switch (p.form) {
-    case 0: return launch_form<METHOD, MODE, 0>(a, p, st);
-    case 1: return launch_form<METHOD, MODE, 1>(a, p, st);
-    case 2: return launch_form<METHOD, MODE, 2>(a, p, st);
-    default: return launch_form<METHOD, MODE, 3>(a, p, st);
+    case 0: return launch_form<METHOD, MODE, 0>(a, p, watched, st);
+    case 1: return launch_form<METHOD, MODE, 1>(a, p, watched, st);
+    case 2: return launch_form<METHOD, MODE, 2>(a, p, watched, st);
+    default: return launch_form<METHOD, MODE, 3>(a, p, watched, st);
     }
 }
 
@@ -1709,8 +1711,10 @@ uint32_t resident_smem_of(uint32_t tiles, uint32_t most) {
     return uint32_t(std::min<uint64_t>(most, l.rows_at + uint64_t(tiles) * 24u * l.row_bytes));
 }
 template <int METHOD>
-cudaError_t launch_resident_of(Arena const& a, ResidentPlan const& p, bool comp, cudaStream_t st) {
-    return comp ? launch_one<METHOD, 1>(a, p, st) : launch_one<METHOD, 0>(a, p, st);
+cudaError_t launch_resident_of(Arena const& a, ResidentPlan const& p, bool comp, bool watched,
+                               cudaStream_t st) {
+    return comp ? launch_one<METHOD, 1>(a, p, watched, st)
+                : launch_one<METHOD, 0>(a, p, watched, st);
 }
 
 }  // namespace emerald

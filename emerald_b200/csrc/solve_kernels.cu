@@ -118,15 +118,59 @@ __device__ int to_int_x86(double d) {
     return static_cast<int>(d);
 }
 
+// Chooses how a watched sub-step is solved: by the resident solve, until one has
+// reported a drift above the limit, then by the kernels per phase until the
+// storage has been sorted again, after one more sort when it drifts again, then
+// after three, up to 31. One thread; returns whether by the kernels per phase.
+__device__ bool choose_solve(Arena const& a, SolveChoice const& ch) {
+    SolveControl& c = *a.control;
+    if (c.in_order) {
+        if (!c.drifted) {
+            c.wait = 0u;
+        } else if (c.left) {
+            --c.left;
+        } else {
+            c.drifted = 0u;
+        }
+    } else if (c.drift > *ch.limit && !c.drifted) {
+        c.drifted = 1u;
+        c.wait = min(2u * c.wait + 1u, 31u);
+        c.left = c.wait;
+    }
+    c.drift = 0u;
+    c.in_order = 0u;
+    if (ch.use_cond) {
+        a.loop_iterations[ch.slot] += c.drifted;
+        cudaGraphSetConditional(ch.cond, c.drifted);
+    }
+    return c.drifted != 0u;
+}
+
 // One thread per scene: picks the sub-step dt exactly as
 // std_adaptive_time_step (emerald/sph2d_box/adaptive_time_step.h:63-103) with
 // cfl_maximum_time_step (emerald/sph_common/cfl.cpp:12-21), or the fixed
 // PCISPH sub-step (emerald/sph2d_box/pcisph.cpp:166-204), or the caller's dt.
-// `resident`: a resident solve follows, which clears kErrUnsolved.
-__global__ void k_begin_substep(Arena a, int nscenes, int resident) {
-    int const s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nscenes) return;
-    if (s == 0) *a.gang_ticket = 0u;
+// `path` (a SolvePath): whether a resident solve follows, which clears
+// kErrUnsolved; a watched sub-step's is chosen here, by one block for all.
+__device__ void begin_substep(Arena const& a, int s, bool resident);
+__global__ void k_begin_substep(Arena a, int nscenes, int path, SolveChoice ch) {
+    bool resident = path != kPhases;
+    if (path == kReported && blockIdx.x == 0 && threadIdx.x == 0 &&
+        a.control->drift > *ch.limit) {
+        *reinterpret_cast<uint32_t volatile*>(a.drift_seen) = 1u;
+    }
+    if (path == kWatched) {
+        __shared__ bool per_phase;
+        if (threadIdx.x == 0) per_phase = choose_solve(a, ch);
+        __syncthreads();
+        resident = !per_phase;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.control->ticket = 0u;
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nscenes; s += gridDim.x * blockDim.x) {
+        begin_substep(a, s, resident);
+    }
+}
+__device__ void begin_substep(Arena const& a, int s, bool resident) {
     a.gangs[s] = GangState{};
     SceneParams const& P = a.sp[s];
     SceneState& S = a.ss[s];
@@ -195,7 +239,7 @@ __global__ void k_frame_begin(Arena a, int nscenes) {
 // loop going while an active scene's frame has sub-steps left (the host
 // loop of std_adaptive_time_step, emerald/sph2d_box/adaptive_time_step.h:74-103,
 // as a while node).
-__global__ void k_frame_check(Arena a, int nscenes, int method, cudaGraphConditionalHandle cond) {
+__global__ void k_frame_check(Arena a, int nscenes, int slot, cudaGraphConditionalHandle cond) {
     __shared__ int any;
     if (threadIdx.x == 0) any = 0;
     __syncthreads();
@@ -207,7 +251,7 @@ __global__ void k_frame_check(Arena a, int nscenes, int method, cudaGraphConditi
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        a.loop_iterations[4 + method] += 1ull;
+        a.loop_iterations[slot] += 1ull;
         cudaGraphSetConditional(cond, any ? 1u : 0u);
     }
 }
@@ -1302,15 +1346,17 @@ unsigned persistent_grid(K kernel, uint32_t tiles, int threads = kTile) {
 void launch_frame_begin(Arena const& a, int nscenes, cudaStream_t st) {
     k_frame_begin<<<(nscenes + 127) / 128, 128, 0, st>>>(a, nscenes);
 }
-void launch_frame_check(Arena const& a, int nscenes, int method, cudaGraphConditionalHandle cond,
+void launch_frame_check(Arena const& a, int nscenes, int slot, cudaGraphConditionalHandle cond,
                         cudaStream_t st) {
-    k_frame_check<<<1, 128, 0, st>>>(a, nscenes, method, cond);
+    k_frame_check<<<1, 128, 0, st>>>(a, nscenes, slot, cond);
 }
 void launch_max_v2(Arena const& a, uint32_t tiles, cudaStream_t st) {
     k_max_v2<<<tiles, kTile, 0, st>>>(a);
 }
-void launch_begin_substep(Arena const& a, int nscenes, bool resident, cudaStream_t st) {
-    k_begin_substep<<<(nscenes + 127) / 128, 128, 0, st>>>(a, nscenes, resident ? 1 : 0);
+void launch_begin_substep(Arena const& a, int nscenes, int path, SolveChoice const& ch,
+                          cudaStream_t st) {
+    int const blocks = path == kWatched ? 1 : (nscenes + 127) / 128;
+    k_begin_substep<<<blocks, 128, 0, st>>>(a, nscenes, path, ch);
 }
 void launch_zero_kappas(Arena const& a, uint32_t tiles, cudaStream_t st) {
     k_zero_kappas<<<tiles, kTile, 0, st>>>(a);
