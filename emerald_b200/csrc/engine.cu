@@ -7,6 +7,7 @@
 #include <climits>
 #include <cstring>
 #include <mutex>
+#include <set>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -1393,6 +1394,8 @@ int Engine::frame(int id, int32_t method, SceneState& out) {
 namespace {
 std::mutex g_tuning_mutex;
 std::map<uint64_t, Engine::Tuning> g_tuning_cache;
+// (tuning key, precision) where the autotuner found the resident solve slower
+std::set<std::pair<uint64_t, bool>> g_resident_slower;
 }  // namespace
 
 uint64_t Engine::tuning_key(int32_t method) const {
@@ -1453,7 +1456,11 @@ ResidentLimits const& Engine::limits_of(int32_t method) {
 // force callbacks (which interrupt the sub-step) take those; so do scenes
 // whose shares are above the method's limit.
 bool Engine::use_resident(int32_t method) {
-    if (timing_ || refused_ || !tuning_.resident || has_force_callbacks()) return false;
+    if (timing_ || refused_ || tuning_pinned_ || per_phase_ || has_force_callbacks()) return false;
+    if (!tuning_locked_) {
+        std::lock_guard<std::mutex> lock(g_tuning_mutex);
+        if (g_resident_slower.count({tuning_key(method), compensated_})) return false;
+    }
     ResidentLimits const& lim = limits_of(method);
     if (!lim.blocks) return false;
     if (!parts_valid_) divide_scenes(lim.blocks);
@@ -1640,7 +1647,6 @@ Engine::TuneReport Engine::autotune(int32_t method, int substeps) {
             Tuning t = tuning_;
             t.apply = o[0];
             t.divergence = o[1];
-            t.resident = false;
             cand.push_back(t);
         }
     } else {
@@ -1656,7 +1662,6 @@ Engine::TuneReport Engine::autotune(int32_t method, int substeps) {
             Tuning t = tuning_;
             t.iisph_sum = o[0];
             t.iisph_beta = o[1];
-            t.resident = false;
             cand.push_back(t);
         }
     }
@@ -1678,10 +1683,11 @@ Engine::TuneReport Engine::autotune(int32_t method, int substeps) {
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     TuneReport rep{};
-    tuning_locked_ = true;
+    tuning_locked_ = per_phase_ = true;
     float best = 0.0f;
     Tuning best_t = cand[0];
     // mean time of a sub-step under a tuning, from the snapshot and back to it
+    SolveControl control{};
     auto time_of = [&](Tuning const& t) {
         tuning_ = t;
         destroy_graphs();
@@ -1697,6 +1703,7 @@ Engine::TuneReport Engine::autotune(int32_t method, int substeps) {
         cudaEventSynchronize(e1);
         float ms = 0.0f;
         cudaEventElapsedTime(&ms, e0, e1);
+        cudaMemcpy(&control, a_.control, sizeof(control), cudaMemcpyDeviceToHost);
         copy(false);
         substeps_launched_ = launched0;
         order_stale_ = stale0;
@@ -1711,13 +1718,24 @@ Engine::TuneReport Engine::autotune(int32_t method, int substeps) {
                 best_t = cand[k];
             }
         }
-        // the resident solve, where it covers these scenes, against the best
-        // of the launch-per-phase kernels
-        tuning_ = best_t;
-        tuning_.resident = true;
-        if (use_resident(method) && time_of(tuning_) < best) best_t.resident = true;
+        // The resident solve, where it covers these scenes, against the best
+        // of the kernels per phase. Where it does not, or the storage order
+        // has drifted, nothing is known of it.
+        per_phase_ = false;
+        if (use_resident(method)) {
+            bool const slower = time_of(best_t) >= best;
+            if (!control.drifted) {
+                std::pair<uint64_t, bool> const key{tuning_key(method), compensated_};
+                std::lock_guard<std::mutex> lock(g_tuning_mutex);
+                if (slower) {
+                    g_resident_slower.insert(key);
+                } else {
+                    g_resident_slower.erase(key);
+                }
+            }
+        }
     } catch (...) {
-        tuning_locked_ = false;
+        tuning_locked_ = per_phase_ = false;
         cudaFree(snap);
         throw;
     }
@@ -1741,13 +1759,11 @@ Engine::TuneReport Engine::autotune(int32_t method, int substeps) {
 }
 
 void Engine::set_tuning(Tuning const* t) {
-    // a pinned tuning names the launch-per-phase kernels; unpinned, the
-    // sub-steps run the resident solve again
-    Tuning next = t ? *t : tuning_;
-    next.resident = t == nullptr;
-    if (!(next == tuning_)) destroy_graphs();
     tuning_pinned_ = t != nullptr;
-    tuning_ = next;
+    if (t && !(*t == tuning_)) {
+        tuning_ = *t;
+        destroy_graphs();
+    }
 }
 
 // ------------------------------------------------------------ accessors

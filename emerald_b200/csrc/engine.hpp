@@ -68,12 +68,9 @@ public:
     // (request-loop lanes, size classes without a tuned entry) start there.
     struct Tuning {
         int apply = 1, divergence = 4, iisph_sum = 4, iisph_beta = 4;
-        // sub-steps run the resident solve where it fits (the kernels above
-        // then serve what it does not cover)
-        bool resident = true;
         bool operator==(Tuning const& o) const {
             return apply == o.apply && divergence == o.divergence && iisph_sum == o.iisph_sum &&
-                   iisph_beta == o.iisph_beta && resident == o.resident;
+                   iisph_beta == o.iisph_beta;
         }
     };
     struct TuneReport {
@@ -210,10 +207,13 @@ public:
     // Picks the fastest chunk settings of `method`'s gather kernels by timing
     // whole sub-steps on the resident scenes (after at least one sub-step of
     // it), restoring the state after each; the choice is kept for engines of
-    // the same method and size class.
+    // the same method and size class. Where the resident solve covers the
+    // scenes it is timed against the best of them, and left out for that
+    // method, precision and size class if it is slower.
     TuneReport autotune(int32_t method, int substeps = 4);
     Tuning const& tuning() const { return tuning_; }
-    // Pins the gather kernels' settings (no cache lookups until unpinned);
+    // Pins the gather kernels' settings (no cache lookups until unpinned),
+    // which names the kernels per phase: the resident solve does not run;
     // nullptr unpins.
     void set_tuning(Tuning const* t);
 
@@ -222,6 +222,7 @@ private:
     Tuning tuning_{};
     bool tuning_locked_ = false;
     bool tuning_pinned_ = false;
+    bool per_phase_ = false;  // the autotuner is timing the kernels per phase
     int32_t last_method_ = -1;
     struct Scene {
         bool used = false;
