@@ -428,16 +428,19 @@ Engine::~Engine() {
     if (h_gave_up_) cudaFreeHost(h_gave_up_);
 }
 
+void Engine::count_kernels(int kernels) {
+    if (!count_host_) return;
+    if (capturing_) {
+        capture_kernels_ += kernels;
+    } else {
+        g_launches.fetch_add(kernels, std::memory_order_relaxed);
+        host_launches_ += kernels;
+    }
+}
+
 template <class F>
 void Engine::launch(char const* name, F&& f, int kernels) {
-    if (count_host_) {
-        if (capturing_) {
-            capture_kernels_ += kernels;
-        } else {
-            g_launches.fetch_add(kernels, std::memory_order_relaxed);
-            host_launches_ += kernels;
-        }
-    }
+    count_kernels(kernels);
     if (!timing_ || capturing_) {
         f();
         return;
@@ -1024,15 +1027,18 @@ void Engine::run_loop(int kind, int max_iter, int32_t method) {
     }
 }
 
+void Engine::emit_reorder() {
+    int kernels = 0;
+    launch("reorder", [&] {
+        kernels = launch_reorder(a_, order_sort_, ext_tiles_ * kTile, order_key_bits(), cur_);
+    }, 0);
+    count_kernels(kernels);
+}
+
 void Engine::emit_substep(int32_t method, bool reorder) {
     uint32_t const tiles = ext_tiles_;
     cudaStream_t const st = cur_;
-    if (reorder) {
-        // keys, three to five radix passes of three kernels, permute, commit
-        int const bits = order_key_bits();
-        launch("reorder", [&] { launch_reorder(a_, order_sort_, tiles * kTile, bits, st); },
-               3 + 3 * (bits / 8));
-    }
+    if (reorder) emit_reorder();
     int const path = path_;
     cudaGraphConditionalHandle cond = 0;
     if (path == kWatched && capturing_) cond = condition();
@@ -1277,12 +1283,7 @@ void Engine::capture_frame(int32_t method, bool reorder) {
     cudaGraph_t g = nullptr;
     try {
         launch("frame_begin", [&] { launch_frame_begin(a_, max_scenes_, cap_st_); });
-        if (reorder) {
-            int const bits = order_key_bits();
-            launch("reorder",
-                   [&] { launch_reorder(a_, order_sort_, ext_tiles_ * kTile, bits, cap_st_); },
-                   3 + 3 * (bits / 8));
-        }
+        if (reorder) emit_reorder();
         cudaGraphConditionalHandle const cond = condition();
         cudaGraph_t body;
         conditional_node(cond, cudaGraphCondTypeWhile, &body);

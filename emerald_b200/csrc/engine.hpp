@@ -245,6 +245,8 @@ private:
     void upload_params(int id);
     void upload_tiles();
     void run_loop(int kind, int max_iter, int32_t method);
+    void emit_reorder();
+    void count_kernels(int kernels);
     void emit_substep(int32_t method, bool reorder);
     void emit_resident(int32_t method);
     void emit_phases(int32_t method);

@@ -45,6 +45,7 @@ void sort_scratch_carve(void* base, uint32_t n, SortScratch& s);
 struct SortResult {
     int cur;
     uint32_t const* gave_up;
+    int kernels;  // launched
 };
 SortResult launch_radix_sort(SortScratch& s, uint32_t n, int bits, cudaStream_t st,
                              bool again = false);
@@ -63,7 +64,8 @@ uint32_t const* launch_sort_products(Arena const& a, bool solid, int scene, uint
                           cudaStream_t st);
 
 // storage order (reorder_kernels.cu)
-void launch_reorder(Arena const& a, SortScratch& s, uint32_t n, int key_bits, cudaStream_t st);
+// (returns the kernels launched)
+int launch_reorder(Arena const& a, SortScratch& s, uint32_t n, int key_bits, cudaStream_t st);
 void launch_gather_f(Arena const& a, uint32_t begin, uint32_t count, float const* src, float* out,
                      cudaStream_t st);
 void launch_gather_f2(Arena const& a, uint32_t begin, uint32_t count, float2 const* src, float2* out,

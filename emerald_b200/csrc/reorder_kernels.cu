@@ -139,12 +139,13 @@ __global__ void k_identity_order(Arena a, uint32_t begin, uint32_t count) {
 
 }  // namespace
 
-void launch_reorder(Arena const& a, SortScratch& s, uint32_t n, int key_bits, cudaStream_t st) {
+int launch_reorder(Arena const& a, SortScratch& s, uint32_t n, int key_bits, cudaStream_t st) {
     k_order_keys<<<(n + 255) / 256, 256, 0, st>>>(a, s.keys[0], s.vals[0], n);
     // (a sort that gave up leaves the storage as it was, which changes no result)
     SortResult const r = launch_radix_sort(s, n, key_bits, st);
     k_permute<<<(n + 255) / 256, 256, 0, st>>>(a, s.keys[r.cur], s.vals[r.cur], n, r.gave_up);
     k_commit_order<<<(n + 255) / 256, 256, 0, st>>>(a, n, r.gave_up);
+    return 3 + r.kernels;
 }
 
 void launch_gather_f(Arena const& a, uint32_t begin, uint32_t count, float const* src, float* out,

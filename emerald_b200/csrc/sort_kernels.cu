@@ -402,21 +402,23 @@ static bool launch_sort_resident(SortScratch& s, uint32_t n, int bits, int out, 
 
 SortResult launch_radix_sort(SortScratch& s, uint32_t n, int bits, cudaStream_t st, bool again) {
     int cur = 0;
-    if (n <= 1) return {cur, nullptr};
+    if (n <= 1) return {cur, nullptr, 0};
     int const out = ((bits + 7) / 8) & 1;
     if (launch_sort_resident(s, n, bits, out, again, st)) {
-        return {out, &static_cast<SortControl*>(s.control)->stalled};
+        return {out, &static_cast<SortControl*>(s.control)->stalled, 1};
     }
     uint32_t const nb = (n + kItems - 1) / kItems;
     uint32_t* offsets = s.hist + static_cast<size_t>(kDigits) * nb;
+    int kernels = 0;
     for (int shift = 0; shift < bits; shift += 8) {
         k_hist<<<nb, kThreads, 0, st>>>(s.keys[cur], n, shift, s.hist, nb);
         launch_exclusive_scan(s.hist, kDigits * nb, offsets, s.scan, st);
         k_rank_scatter<<<nb, kThreads, 0, st>>>(s.keys[cur], s.vals[cur], s.keys[cur ^ 1],
                                                 s.vals[cur ^ 1], n, shift, offsets, nb);
+        kernels += 5;  // three of them the scan
         cur ^= 1;
     }
-    return {cur, nullptr};
+    return {cur, nullptr, kernels};
 }
 
 uint32_t const* launch_sort_products(Arena const& a, bool solid, int scene, uint32_t begin, uint32_t count,
