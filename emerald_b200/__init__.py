@@ -17,10 +17,9 @@ LIB_PATH = os.path.join(_HERE, "libemerald_b200.so")
 METHODS = {"pcisph": 0, "iisph": 1, "iisph_ap": 2, "iisph_pseudo_ap": 3, "dfsph_p": 4}
 PRECISION_REFERENCE = 0
 PRECISION_COMPENSATED = 1
-INJECT_BARRIER_POLLS = 0
-INJECT_VALUE_POLLS = 1
-INJECT_SORT_POLLS = 2
-INJECT_REFUSE = 3
+INJECT_STALL = 0
+INJECT_SORT_POLLS = 1
+INJECT_REFUSE = 2
 FLICKS_PER_SECOND = 705600000
 
 c_f = ctypes.c_float
@@ -656,8 +655,12 @@ class Simulation:
         """Fault injection for tests (INJECT_*)."""
         _check(lib.emerald_sim_inject(self._h, what, value), "inject")
 
-    def enable_timing(self, on=True):
-        _check(lib.emerald_sim_enable_timing(self._h, int(on)), "enable_timing")
+    def enable_timing(self, on=True, resident=False):
+        """Times every launch of the sub-steps, run as kernels per phase, or
+        with `resident` as they would run untimed (the resident solve as
+        "solve")."""
+        _check(lib.emerald_sim_enable_timing(self._h, 2 if on and resident else int(on)),
+               "enable_timing")
 
     def kernel_times(self):
         count = c_i32(256)

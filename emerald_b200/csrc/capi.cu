@@ -829,7 +829,7 @@ int emerald_sim_enable_timing(emerald_sim* sim, int32_t enable) {
     if (!sim) return fail(EMERALD_EINVAL, "sim is NULL");
     return guarded([&] {
         sim->engine.reset_timing();
-        sim->engine.enable_timing(enable != 0);
+        sim->engine.enable_timing(enable != 0, enable == EMERALD_TIMING_RESIDENT);
         return EMERALD_OK;
     });
 }

@@ -64,9 +64,6 @@ constexpr uint32_t kDriftRoots = 14;
 // tests require.
 constexpr uint32_t kMinBatchTiles = 64;
 
-// Polls of a wait of the resident solve before it gives up (seconds; a phase
-// takes microseconds).
-constexpr uint32_t kMaxPolls = 1u << 22;
 constexpr int kStallBits = kErrStalled | kErrUnsolved;
 
 // How many error sums s = 0, 1, ... pass the solvers' average test
@@ -372,7 +369,6 @@ Engine::Engine(uint32_t fluid_capacity, uint32_t solid_capacity, int max_scenes)
     h_gave_up_[0] = h_gave_up_[1] = 0u;
     a_.gave_up = h_gave_up_;
     a_.drift_seen = h_gave_up_ + 1;
-    a_.barrier_polls = a_.value_polls = kMaxPolls;
     cudaMemset(d_ss_, 0, sizeof(SceneState) * max_scenes_);
     cudaMemset(a_.vs, 0, 8 * S);
     cudaMemset(a_.nf_cnt, 0, N);
@@ -462,7 +458,10 @@ void Engine::launch(char const* name, F&& f, int kernels) {
     pending_.push_back(p);
 }
 
-void Engine::enable_timing(bool on) { timing_ = on; }
+void Engine::enable_timing(bool on, bool resident) {
+    timing_ = on;
+    time_resident_ = resident;
+}
 
 void Engine::reset_timing() {
     kernel_times();
@@ -530,7 +529,6 @@ void Engine::scenes_changed(bool added) {
     order_stale_ = order_stale_ || added;
     int used = 0;
     for (auto const& sc : scenes_) used += sc.used ? 1 : 0;
-    changing_ = max_scenes_ > 1 && (changing_ || substeps_launched_ > 0);
     if (used > 1) return;
     cudaMemsetAsync(a_.control, 0, sizeof(SolveControl), st_);
     h_gave_up_[1] = 0u;
@@ -796,8 +794,7 @@ void Engine::remove_scene(int id) {
 
 void Engine::inject(int what, uint32_t value) {
     switch (what) {
-    case EMERALD_INJECT_BARRIER_POLLS: a_.barrier_polls = value; break;
-    case EMERALD_INJECT_VALUE_POLLS: a_.value_polls = value; break;
+    case EMERALD_INJECT_STALL: a_.inject = value; break;
     case EMERALD_INJECT_REFUSE:
         refuse_ = value != 0u;
         refused_ = false;
@@ -1352,7 +1349,7 @@ int Engine::frame(int id, int32_t method, SceneState& out) {
     }
     check_solved(-1);
     bool const reorder = reorder_every_ > 0 && (frames_launched_ % 2 == 0 || order_stale_);
-    prepare_substep(method);
+    prepare_substep(method, true);
     ++frames_launched_;
     int key;
     try {
@@ -1411,7 +1408,7 @@ uint64_t Engine::tuning_key(int32_t method) const {
 
 // Tuning cache lookup and per-scene method parameters before a sub-step or
 // frame of `method`.
-void Engine::prepare_substep(int32_t method) {
+void Engine::prepare_substep(int32_t method, bool frame) {
     if (!tuning_locked_ && !tuning_pinned_) {
         std::lock_guard<std::mutex> lock(g_tuning_mutex);
         auto const it = g_tuning_cache.find(tuning_key(method));
@@ -1431,7 +1428,7 @@ void Engine::prepare_substep(int32_t method) {
             upload_params(id);
         }
     }
-    path_ = solve_path(method);
+    path_ = solve_path(method, frame);
     if (path_ != kPhases) plan_resident(method);
 }
 
@@ -1457,7 +1454,7 @@ ResidentLimits const& Engine::limits_of(int32_t method) {
 // force callbacks (which interrupt the sub-step) take those; so do scenes
 // whose shares are above the method's limit.
 bool Engine::use_resident(int32_t method) {
-    if (timing_ || refused_ || tuning_pinned_ || per_phase_ || has_force_callbacks()) return false;
+    if ((timing_ && !time_resident_) || refused_ || tuning_pinned_ || per_phase_ || has_force_callbacks()) return false;
     if (!tuning_locked_) {
         std::lock_guard<std::mutex> lock(g_tuning_mutex);
         if (g_resident_slower.count({tuning_key(method), compensated_})) return false;
@@ -1469,15 +1466,11 @@ bool Engine::use_resident(int32_t method) {
     return total_tiles_ >= kMinBatchTiles && largest_share_ <= std::min(kHeldTiles, lim.share);
 }
 
-int Engine::solve_path(int32_t method) {
+int Engine::solve_path(int32_t method, bool frame) {
     if (!use_resident(method)) return kPhases;
     if (!drift_limit_[method]) return kResident;
-    // A batch whose scenes come and go records its graphs often, and one that
-    // holds both solves takes a millisecond more than one with the resident
-    // solve alone (16 served requests 16.8 against 18.0 ms): it gets the former
-    // when a drift has been reported.
     bool const seen = reinterpret_cast<uint32_t volatile*>(h_gave_up_)[1] != 0u;
-    return changing_ && !seen ? kReported : kWatched;
+    return frame || seen ? kWatched : kReported;
 }
 
 // Divides the active scenes' warp tiles among the resident blocks: a scene's
@@ -1558,7 +1551,7 @@ void Engine::substep(int32_t method) {
     check_solved(-1);
     bool const reorder =
       reorder_every_ > 0 && (substeps_launched_ % reorder_every_ == 0 || order_stale_);
-    prepare_substep(method);
+    prepare_substep(method, false);
     ++substeps_launched_;
     order_stale_ = order_stale_ && !reorder;
     if (use_graphs_ && !timing_ && !has_force_callbacks()) {

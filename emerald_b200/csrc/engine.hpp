@@ -178,7 +178,9 @@ public:
         return n;
     }
 
-    void enable_timing(bool on);
+    // Times every launch; the kernels per phase, or with `resident` the
+    // resident solve where sub-steps run it.
+    void enable_timing(bool on, bool resident = false);
     KernelTimes const& kernel_times();
     void reset_timing();
     // Loop control: false runs the exit test on the host after each solver
@@ -260,7 +262,7 @@ private:
     int order_key_bits() const;
     void destroy_graphs();
     void capture_frame(int32_t method, bool reorder);
-    void prepare_substep(int32_t method);
+    void prepare_substep(int32_t method, bool frame);
     // The resident solve (resident_kernels.cu): whether sub-steps of `method`
     // run it now, and its division of the active scenes among blocks.
     bool use_resident(int32_t method);
@@ -286,12 +288,11 @@ private:
     uint32_t largest_share_ = 1;
     // How sub-steps of `method` are solved now (a SolvePath); path_: how this
     // call's are.
-    int solve_path(int32_t method);
+    int solve_path(int32_t method, bool frame);
     int path_ = kPhases;
     void scenes_changed(bool added);
     bool order_stale_ = false;              // particles were added since the last re-sort
     uint32_t drift_limit_[5] = {0, 0, 0, 0, 0};  // per method; 0: not watched
-    bool changing_ = false;  // a batch whose scenes come and go
     uint64_t total_tiles_ = 0;
     GangPart* d_parts_ = nullptr;
     uint32_t* d_nparts_ = nullptr;  // the shares, then the methods' drift limits
@@ -370,6 +371,7 @@ private:
     SortScratch sort_{};
 
     bool timing_ = false;
+    bool time_resident_ = false;
     struct Pending {
         std::string name;
         cudaEvent_t start, stop;

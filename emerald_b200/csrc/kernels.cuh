@@ -95,6 +95,10 @@ void launch_frame_check(Arena const& a, int nscenes, int slot, cudaGraphConditio
 // How a sub-step is solved: by the kernels per phase, the resident solve,
 // whichever of the two its first kernel chooses, or the resident solve while
 // that kernel tells the host (Arena::drift_seen) when it would choose otherwise.
+// A graph that holds both solves takes the host and the device longer to launch
+// (262,144 particles, a sub-step of 640 us as a graph of its own: 130 us more),
+// so frames, whose graph is launched once, choose on the device, and sub-steps
+// begin to when a drift has been seen.
 enum SolvePath : int { kPhases = 0, kResident = 1, kWatched = 2, kReported = 3, kPaths = 4 };
 struct SolveChoice {
     uint32_t const* limit;  // device: drift above which the kernels per phase are faster

@@ -59,6 +59,9 @@ constexpr uint32_t kBoundaryUnits = 2;   // rows of space per boundary row: 32 m
                                          // gradients and velocities (640 bytes)
 constexpr uint32_t kMaxTiles = 256;      // warp tiles of a share at most
 constexpr uint32_t kNoKey = 0xffffffffu;
+// Polls of a wait before it gives up: about a second, where a sub-step's solve
+// takes milliseconds. (A constant: as a parameter it costs spills in the loops.)
+constexpr uint32_t kMaxPolls = 1u << 20;
 constexpr uint32_t kFar = 0xffffu;       // a neighbour without a code
 
 // A particle's published values and the codes of its list that do not fit in
@@ -560,7 +563,7 @@ __device__ __forceinline__ void stage_lists(Arena const& a, Layout const& l, Sha
 
 // Waits until every block of the gang has arrived, making their writes before
 // it visible after it. Returns false when the others did not arrive within the
-// poll limit (Arena::barrier_polls): the caller leaves.
+// poll limit: the caller leaves.
 __device__ __forceinline__ bool gang_sync(Arena const& a, Shared& s) {
     block_sync();
     if (threadIdx.x == 0 && s.part.size > 1) {
@@ -573,7 +576,7 @@ __device__ __forceinline__ bool gang_sync(Arena const& a, Shared& s) {
         for (;;) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(arrive) : "memory");
             if (seen >= target) break;
-            if (++polls > a.barrier_polls) {
+            if (++polls > kMaxPolls) {
                 s.ok = 0;
                 break;
             }
@@ -599,7 +602,9 @@ __device__ __forceinline__ bool agree(Arena const& a, Share& sh, Shared& s) {
         record_of(a, s, s.part.rank, threadIdx.x / 6)->w[threadIdx.x % 6] = 0ull;
     }
     bool const ok = gang_sync(a, s);
-    if (threadIdx.x == 0) s.tagged = __ldcg(&g.plain) ? 0 : 1;
+    // (injected: one block on its own in the other form, whose values never come)
+    bool const astray = a.inject == 2u && s.part.rank == 0u;
+    if (threadIdx.x == 0) s.tagged = __ldcg(&g.plain) || astray ? 0 : 1;
     block_sync();
     sh.tagged = s.tagged != 0;
     return ok;
@@ -688,7 +693,7 @@ __device__ __forceinline__ void receive(Arena const& a, Layout const& l, Share c
         T v;
         uint32_t polls = 0;
         while (!get_value(a, f, halo[h], sh.epoch, v)) {
-            if (++polls > a.value_polls) {
+            if (++polls > kMaxPolls) {
                 s.ok = 0;
                 return;
             }
@@ -787,9 +792,8 @@ __device__ __forceinline__ void post_errors(Arena const& a, Shared const& s, uin
 }
 
 // The two words from word k of a record, waited for until they carry the tag.
-__device__ __forceinline__ void record_words(Arena const& a, GangRecord const* r, int k,
-                                             uint32_t tag, Shared& s, uint32_t& lo,
-                                             uint32_t& hi) {
+__device__ __forceinline__ void record_words(GangRecord const* r, int k, uint32_t tag, Shared& s,
+                                             uint32_t& lo, uint32_t& hi) {
     unsigned long long w0, w1;
     uint32_t polls = 0;
     for (;;) {
@@ -798,7 +802,7 @@ __device__ __forceinline__ void record_words(Arena const& a, GangRecord const* r
                      : "l"(r->w + k)
                      : "memory");
         if (word_tag(w0) == tag && word_tag(w1) == tag) break;
-        if (++polls > a.value_polls) {
+        if (++polls > kMaxPolls) {
             s.ok = 0;
             break;
         }
@@ -837,7 +841,7 @@ __device__ __forceinline__ void decide_exit(Arena const& a, Shared& s, int kind,
                 ready = ready && (k0 + u * 32u + lane >= size ||
                                   (word_tag(w0[u]) == tag && word_tag(w1[u]) == tag));
             }
-            if (++polls > a.value_polls) {
+            if (++polls > kMaxPolls) {
                 s.ok = 0;
                 break;
             }
@@ -850,7 +854,7 @@ __device__ __forceinline__ void decide_exit(Arena const& a, Shared& s, int kind,
             t.max = hi > t.max ? hi : t.max;
             unsigned long long sum = lo;
             if (lo == 0xffffffffu) {
-                record_words(a, record_of(a, s, k, slot), 2, tag, s, lo, hi);
+                record_words(record_of(a, s, k, slot), 2, tag, s, lo, hi);
                 sum = (static_cast<unsigned long long>(hi) << 32) | lo;
             }
             t.sum += sum;
@@ -892,7 +896,7 @@ __device__ __forceinline__ void report_exact(Arena const& a, Share& sh, Shared& 
 #pragma unroll 1
     for (uint32_t k = lane; k < s.part.size && s.ok; k += 32u) {
         uint32_t lo, hi;
-        record_words(a, record_of(a, s, k, slot), 4, sh.epoch, s, lo, hi);
+        record_words(record_of(a, s, k, slot), 4, sh.epoch, s, lo, hi);
         t += __longlong_as_double(
           static_cast<long long>((static_cast<unsigned long long>(hi) << 32) | lo));
     }
@@ -1522,6 +1526,32 @@ __device__ __forceinline__ bool solve(Arena const& a, Layout const& l, Share& sh
     return false;
 }
 
+// Between two shares of a block (one thread): the share before is done, and
+// its scene when it was the last of them, unless a wait gave up after the
+// threads' last look.
+__device__ __forceinline__ void next_share(Arena const& a, Shared& s) {
+    if (s.part.size) {
+        if (!s.ok) {
+            s.ticket = kNoKey;
+            *reinterpret_cast<uint32_t volatile*>(a.gave_up) = 1u;
+            return;
+        }
+        // (both atomics on their way together)
+        uint32_t const done = atomicAdd(&a.gangs[s.part.scene].done, 1u);
+        s.ticket = atomicAdd(&a.control->ticket, 1u);
+        if (done + 1u == s.part.size) atomicAnd(&a.ss[s.part.scene].error, ~kErrUnsolved);
+        s.part.size = 0u;
+    } else {
+        s.ticket = atomicAdd(&a.control->ticket, 1u);
+    }
+    s.used = 0u;
+    s.wanted = 0u;
+    s.halo_n = 0u;
+    s.ok = 1;
+    s.plain = 0;
+    s.target = 0u;
+}
+
 // Every block takes shares in order until none is left. A gang's blocks wait
 // for each other only: shares are taken in order, so when a block waits, every
 // earlier gang is fully staffed and finishes, and its blocks go on to staff
@@ -1534,17 +1564,10 @@ __global__ void __launch_bounds__(Form<METHOD, MODE, FORM>::kThreads, 1)
   k_resident_solve(Arena a, GangPart const* parts, uint32_t const* nparts, Layout l, int watched) {
     __shared__ Shared s;
     if (watched && a.control->drifted) return;
+    if (threadIdx.x == 0) s.part.size = 0u;
     for (;;) {
         block_sync();
-        if (threadIdx.x == 0) {
-            s.ticket = atomicAdd(&a.control->ticket, 1u);
-            s.used = 0u;
-            s.wanted = 0u;
-            s.halo_n = 0u;
-            s.ok = 1;
-            s.plain = 0;
-            s.target = 0u;
-        }
+        if (threadIdx.x == 0) next_share(a, s);
         block_sync();
         uint32_t const ticket = s.ticket;
         if (ticket >= *nparts) return;
@@ -1561,6 +1584,7 @@ __global__ void __launch_bounds__(Form<METHOD, MODE, FORM>::kThreads, 1)
                 s.part = part;
                 s.dt = a.ss[part.scene].dt;
                 s.new_frame = a.ss[part.scene].new_frame;
+                if (a.inject == 1u && part.rank == 0u) s.target = 1u;  // waits for one too many
             }
         }
         block_sync();
@@ -1569,19 +1593,13 @@ __global__ void __launch_bounds__(Form<METHOD, MODE, FORM>::kThreads, 1)
         constexpr int R = Form<METHOD, MODE, FORM>::kTiles, CH = Form<METHOD, MODE, FORM>::kRows;
         bool const ok = (MODE && s.P.precision) ? solve<METHOD, true, R, CH>(a, l, sh, s)
                                                 : solve<METHOD, false, R, CH>(a, l, sh, s);
-        // A thread whose wait gave up, or that saw another's give up, leaves (the
-        // block's barriers then count the threads that are left); the rest
-        // follow at the next of its checks, the last of which is here: the exit
-        // test's warp may have given up after the others' last look.
-        if (ok) block_sync();
-        if (!ok || !s.ok) {
+        // A thread whose wait gave up, or that saw another's give up, leaves; the
+        // block's barriers then count the threads that are left, and no share is
+        // taken any more.
+        if (!ok) {
+            s.ticket = kNoKey;
             *reinterpret_cast<uint32_t volatile*>(a.gave_up) = 1u;
             return;
-        }
-        // the scene is solved when its last share is
-        if (threadIdx.x == 0 &&
-            atomicAdd(&a.gangs[s.part.scene].done, 1u) + 1u == s.part.size) {
-            atomicAnd(&a.ss[s.part.scene].error, ~kErrUnsolved);
         }
     }
 }

@@ -126,7 +126,9 @@ __device__ bool choose_solve(Arena const& a, SolveChoice const& ch) {
     SolveControl& c = *a.control;
     if (c.in_order) {
         if (!c.drifted) {
+            // in order all the while between two sorts
             c.wait = 0u;
+            *reinterpret_cast<uint32_t volatile*>(a.drift_seen) = 0u;
         } else if (c.left) {
             --c.left;
         } else {
@@ -146,39 +148,20 @@ __device__ bool choose_solve(Arena const& a, SolveChoice const& ch) {
     return c.drifted != 0u;
 }
 
-// One thread per scene: picks the sub-step dt exactly as
+// The scene's error word for the sub-step, from the word before it (the cell
+// build may report a full table meanwhile).
+__device__ __forceinline__ void mark_scene(Arena const& a, int s, int before, bool resident) {
+    int const set = ((before & kErrUnsolved) ? kErrStalled : 0) | (resident ? kErrUnsolved : 0);
+    int const clear = before & (kErrNonFinite | kErrUnsolved) & ~set;
+    if (clear) atomicAnd(&a.ss[s].error, ~clear);
+    if (set & ~before) atomicOr(&a.ss[s].error, set);
+}
+
+// Picks the sub-step dt exactly as
 // std_adaptive_time_step (emerald/sph2d_box/adaptive_time_step.h:63-103) with
 // cfl_maximum_time_step (emerald/sph_common/cfl.cpp:12-21), or the fixed
 // PCISPH sub-step (emerald/sph2d_box/pcisph.cpp:166-204), or the caller's dt.
-// `path` (a SolvePath): whether a resident solve follows, which clears
-// kErrUnsolved; a watched sub-step's is chosen here, by one block for all.
-__device__ void begin_substep(Arena const& a, int s, bool resident);
-__global__ void k_begin_substep(Arena a, int nscenes, int path, SolveChoice ch) {
-    bool resident = path != kPhases;
-    if (path == kReported && blockIdx.x == 0 && threadIdx.x == 0 &&
-        a.control->drift > *ch.limit) {
-        *reinterpret_cast<uint32_t volatile*>(a.drift_seen) = 1u;
-    }
-    if (path == kWatched) {
-        __shared__ bool per_phase;
-        if (threadIdx.x == 0) per_phase = choose_solve(a, ch);
-        __syncthreads();
-        resident = !per_phase;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.control->ticket = 0u;
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nscenes; s += gridDim.x * blockDim.x) {
-        begin_substep(a, s, resident);
-    }
-}
-__device__ void begin_substep(Arena const& a, int s, bool resident) {
-    a.gangs[s] = GangState{};
-    SceneParams const& P = a.sp[s];
-    SceneState& S = a.ss[s];
-    if (!S.active) return;
-    // (the cell build may report a full table meanwhile)
-    int const before = atomicAnd(&S.error, ~(kErrNonFinite | kErrUnsolved));
-    int const now = ((before & kErrUnsolved) ? kErrStalled : 0) | (resident ? kErrUnsolved : 0);
-    if (now) atomicOr(&S.error, now);
+__device__ __forceinline__ void begin_scene(Arena const& a, SceneParams const& P, SceneState& S) {
     if (P.mode == kFixedDt) {
         S.dt = P.fixed_dt;
         S.t = P.fixed_t;
@@ -227,6 +210,40 @@ __device__ void begin_substep(Arena const& a, int s, bool resident) {
         S.elapsed = 0;
     }
     S.max_v2 = 0;
+}
+
+// One thread per scene. `path` (a SolvePath): whether a resident solve follows,
+// which clears kErrUnsolved. A watched sub-step's path is chosen meanwhile by
+// another warp, and its scenes are marked afterwards, by one block for all.
+__global__ void k_begin_substep(Arena a, int nscenes, int path, SolveChoice ch) {
+    __shared__ bool per_phase;
+    if (blockIdx.x == 0 && threadIdx.x == 64) {
+        SolveControl& c = *a.control;
+        c.ticket = 0u;
+        if (path == kWatched) {
+            per_phase = choose_solve(a, ch);
+        } else if (path == kReported) {
+            if (c.in_order) {
+                c.in_order = c.drift = 0u;
+            } else if (c.drift > *ch.limit) {
+                *reinterpret_cast<uint32_t volatile*>(a.drift_seen) = 1u;
+            }
+        }
+    }
+    int const first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    for (int s = first; s < nscenes; s += step) {
+        a.gangs[s] = GangState{};
+        SceneState& S = a.ss[s];
+        if (!S.active) continue;
+        int const before = S.error;
+        begin_scene(a, a.sp[s], S);
+        if (path != kWatched) mark_scene(a, s, before, path != kPhases);
+    }
+    if (path != kWatched) return;
+    __syncthreads();
+    for (int s = first; s < nscenes; s += step) {
+        if (a.ss[s].active) mark_scene(a, s, a.ss[s].error, !per_phase);
+    }
 }
 
 // Start of a frame-graph launch: no sub-step of it has run yet.

@@ -307,21 +307,24 @@ int emerald_sim_set_stream(emerald_sim* sim, void* cuda_stream);
 int emerald_sim_device_state(emerald_sim* sim, void** x, void** v);
 
 /* Accumulated device time per kernel name since the last reset, measured
- * with CUDA events around each launch when timing is enabled. */
+ * with CUDA events around each launch when timing is enabled. The sub-steps
+ * then run the kernels per phase, with EMERALD_TIMING_RESIDENT the resident
+ * solve where they would run it untimed (as "solve"). */
+#define EMERALD_TIMING_RESIDENT 2
 int emerald_sim_enable_timing(emerald_sim* sim, int32_t enable);
 int emerald_sim_kernel_times(emerald_sim* sim, char* names, size_t names_len, double* ms,
                              int32_t* launches, int32_t* count);
 
 /* Fault injection for tests: `what` set to `value` for this simulation.
- * BARRIER_POLLS and VALUE_POLLS: how often a wait of the resident
- * solve's blocks for one another looks before it gives up (2^22); SORT_POLLS:
- * the same of the z-order sort's (a re-sort of the storage that gives up is
- * left out, emerald_sim_get_sort fails). REFUSE: not 0 stands for a device that
- * refuses the resident solve's cooperative launch. */
-#define EMERALD_INJECT_BARRIER_POLLS 0
-#define EMERALD_INJECT_VALUE_POLLS 1
-#define EMERALD_INJECT_SORT_POLLS 2
-#define EMERALD_INJECT_REFUSE 3
+ * STALL: a wait of the resident solve's blocks for one another that cannot
+ * end, and gives up after about a second: 1 at their first barrier, 2 for each
+ * other's values, 0 none. SORT_POLLS: how often a wait of the z-order sort looks
+ * before it gives up (2^22; a re-sort of the storage that gives up is left out,
+ * emerald_sim_get_sort fails). REFUSE: not 0 stands for a device that refuses
+ * the resident solve's cooperative launch. */
+#define EMERALD_INJECT_STALL 0
+#define EMERALD_INJECT_SORT_POLLS 1
+#define EMERALD_INJECT_REFUSE 2
 int emerald_sim_inject(emerald_sim* sim, int32_t what, uint32_t value);
 /* Execution mode: graphs != 0 (default) runs each sub-step as one CUDA graph
  * launch with the solver loops as conditional nodes; graphs == 0 launches

@@ -69,9 +69,9 @@ def test_drift_and_back(E, method, n, graphs):
     resident = min(per_step(a, lambda: a.advance(method, 1, stats=False), 3))
     a.advance(method, 60, stats=False)
     counts = per_step(a, lambda: a.advance(method, 1, stats=False), 180)
-    # (a re-sort adds up to fifteen)
-    taken = ["resident" if c <= resident + 15 else "per phase" for c in counts]
-    assert taken.count("per phase") > 30
+    # (a re-sort adds four)
+    taken = ["resident" if c <= resident + 4 else "per phase" for c in counts]
+    assert taken.count("per phase") >= 16        # from one re-sort to the next
     assert any(x == "per phase" and y == "resident" for x, y in zip(taken, taken[1:]))
     b.advance(method, 243, stats=False)
     for name, x, y in zip("xv", a.state(), b.state()):

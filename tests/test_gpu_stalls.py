@@ -1,5 +1,5 @@
-"""Waits inside kernels that give up (their poll limits set to none, so that
-healthy kernels run out of them): the calls that return results say so, the
+"""Waits inside kernels that give up (made to wait for what nobody sends, or
+with a poll limit of none): the calls that return results say so, the
 context stays usable, and a scene goes on from a new state with the bits it
 would have had."""
 import numpy as np
@@ -11,14 +11,7 @@ from test_gpu_resident import METHODS, scene
 pytestmark = pytest.mark.gpu
 
 POLLS = 1 << 22
-# barrier and value polls: the gang's first barrier gives up; or the exchanges
-# do (and the barriers that then miss blocks, after a while)
-GIVE_UP = {"barrier": (0, 100), "value": (20000, 0)}
-
-
-def inject(E, target, barrier=POLLS, value=POLLS):
-    target.inject(E.INJECT_BARRIER_POLLS, barrier)
-    target.inject(E.INJECT_VALUE_POLLS, value)
+GIVE_UP = {"barrier": 1, "values": 2}
 
 
 @pytest.fixture(scope="module")
@@ -34,13 +27,13 @@ def test_solve_that_gives_up(E, method, which):
     sim = E.Simulation.from_block_scene(sc)
     sim.advance(method, 2)
     snap = sim.snapshot()
-    inject(E, sim, *GIVE_UP[which])
+    sim.inject(E.INJECT_STALL, GIVE_UP[which])
     sim.advance(method, 1, stats=False)
     for call in (sim.state, sim.time, sim.snapshot, sim.neighbors, lambda: sim.array("densities"),
                  lambda: sim.advance(method, 1), lambda: sim.frame(method), sim.state):
         with pytest.raises(E.EmeraldError):
             call()
-    inject(E, sim)
+    sim.inject(E.INJECT_STALL, 0)
     with pytest.raises(E.EmeraldError):
         sim.advance(method, 1)
     sim.restore(snap)
@@ -50,10 +43,10 @@ def test_solve_that_gives_up(E, method, which):
     for name, x, y in zip("xv", sim.state(), want.state()):
         assert_bitwise(x, y, "%s %s" % (method, name))
     # positions and velocities are a new state too
-    inject(E, sim, *GIVE_UP[which])
+    sim.inject(E.INJECT_STALL, GIVE_UP[which])
     with pytest.raises(E.EmeraldError):
         sim.advance(method, 1)
-    inject(E, sim)
+    sim.inject(E.INJECT_STALL, 0)
     sim.set_state(sc.fluid, np.zeros_like(sc.fluid))
     assert sim.advance(method, 1)["error_flags"] == 0
 
@@ -71,13 +64,13 @@ def test_batch_that_gives_up(E, method, which):
     ids = [b.add_block_scene(s) for s in scenes]
     b.step(method, 1)
     b.synchronize()
-    inject(E, b, *GIVE_UP[which])
+    b.inject(E.INJECT_STALL, GIVE_UP[which])
     b.step(method, 1)
     with pytest.raises(E.EmeraldError):
         b.synchronize()
     with pytest.raises(E.EmeraldError):
         b.step(method, 1)
-    inject(E, b)
+    b.inject(E.INJECT_STALL, 0)
     failed = []
     for k, sc in enumerate(scenes):
         want = E.Simulation.from_block_scene(sc)
