@@ -140,6 +140,8 @@ def traffic_from_profile(kernel, n=None):
 # What bounds a kernel whose HBM fraction is low by design (from its ncu
 # summary under profiles/).
 LIMITERS = {
+    "solve": "the exchanges of neighbouring blocks' values: the lists and the gathered values "
+             "stay on the chip for all iterations (profiles/k_resident_solve.md)",
     "neighbors_fluid": "instruction issue: 58% of issue slots busy, 3-4% of peak DRAM "
                        "throughput (profiles/k_neighbors.dfsph_262k.md)",
 }
@@ -159,6 +161,9 @@ def algorithmic_bytes(kernel, n, nnz_f, nnz_s, n_s):
         "dfsph_divergence": per_entry + vols + 8.0 * n_s + n * (2 + 8 + 4 + 4 + 4 + 4 + 4),
         "dfsph_density": per_entry + vols + 8.0 * n_s + n * (2 + 8 + 4 + 4 + 4 + 4 + 4),
         "dfsph_density_alpha": 16.0 * (nnz_f + nnz_s) + vols + n * (2 + 4 + 4 + 4 + 4 + 4 + 4),
+        # the resident solve: lists, state and per-particle results once, all
+        # of its iterations on the chip
+        "solve": 16.0 * (nnz_f + nnz_s) + vols + 8.0 * n_s + n * (2 + 16 + 16 + 8 + 8 + 12),
         "neighbors_fluid": 16.0 * nnz_f + n * (8 + 4 + 1),
         "neighbors_solid": 16.0 * nnz_s + n * (8 + 1) + 12.0 * n_s,
     }
@@ -324,16 +329,24 @@ def run_gpu(args):
         dist.all_reduce(t2, op=dist.ReduceOp.MAX)
     e2e_value = world * n * e2e_steps / (float(t2.item()) / 1000.0)
 
-    # per-kernel device times (events around every launch) for the roofline
-    sim.enable_timing(True)
+    # per-kernel device times (events around every launch) for the roofline:
+    # of the kernels the timed region ran, then of the kernels per phase, which
+    # it runs where the resident solve does not cover the scene
     rsteps = max(3, min(args.steps, 50))
     errs, exact = [], []
+    sim.enable_timing(True, resident=True)
     for _ in range(rsteps):
         flush.zero_()
         st = sim.advance("dfsph_p", 1)
         errs.append(st["error_average"])
         exact.append(st["error_average_exact"])
     times = sim.kernel_times()
+    solved_by = "resident solve" if "solve" in times else "kernels per phase"
+    sim.enable_timing(True)
+    for _ in range(rsteps):
+        flush.zero_()
+        sim.advance("dfsph_p", 1)
+    phase_times = sim.kernel_times()
     sim.enable_timing(False)
     counts_f, _, _, _ = sim.neighbors(False)
     counts_s, _, _, _ = sim.neighbors(True)
@@ -355,9 +368,10 @@ def run_gpu(args):
                     "avg_launch_us": round(per_launch_s * 1e6, 2)}
         if top_name in LIMITERS:
             roofline["limiter"] = LIMITERS[top_name]
-    # the same figures for the gather-sum kernel with the largest share (the
-    # solver's memory-bound work)
-    gather = [kv for kv in ranked if kv[0] in GATHER_KERNELS]
+    # the same figures for the gather-sum kernel per phase with the largest
+    # share (the solver's memory-bound work)
+    gather = [kv for kv in sorted(phase_times.items(), key=lambda kv: -kv[1][0])
+              if kv[0] in GATHER_KERNELS]
     gather_roofline = None
     if gather:
         g_name, (g_ms, g_launches) = gather[0]
@@ -385,8 +399,10 @@ def run_gpu(args):
                        "neighbours_per_particle": round(nnz_f / n, 2),
                        "parallelism": "replicas" if world > 1 else "single scene",
                        "l2": "flushed between timed steps (256 MiB write)",
+                       "solved_by": solved_by,
                        "autotuned_chunks": tuning["chunks"],
                        "autotuned_prefetch": tuning["prefetch"],
+                       "autotuned_note": "settings of the kernels per phase",
                        "p50_step_ms": round(float(np.percentile(step_ms, 50)), 4),
                        "p99_step_ms": round(float(np.percentile(step_ms, 99)), 4),
                        "last_step": {k: last[k] for k in ("dt", "pressure_iterations",
@@ -401,7 +417,8 @@ def run_gpu(args):
                                    "of the per-particle errors is beside it"}},
             "roofline": roofline,
             "gather_roofline": gather_roofline,
-            "gather_rooflines": kernel_rooflines(times, n, nnz_f, nnz_s, n_s),
+            "gather_rooflines": kernel_rooflines(phase_times, n, nnz_f, nnz_s, n_s),
+            "gather_note": "kernels per phase, in the sub-steps after the timed region",
             "kernels": kernel_table,
             "e2e": {"value": round(e2e_value, 1), "unit": "particle-steps/s",
                     "h2d_bytes_per_step": int(2 * n * 8), "d2h_bytes_per_step": int(2 * n * 8),
