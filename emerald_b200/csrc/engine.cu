@@ -355,18 +355,18 @@ Engine::Engine(uint32_t fluid_capacity, uint32_t solid_capacity, int max_scenes)
         cudaStreamCreateWithFlags(&body_st_, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&frame_st_, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&side_st_, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&path_st_, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming) != cudaSuccess) {
         throw std::runtime_error("stream creation failed");
     }
-    if (cudaMallocHost(reinterpret_cast<void**>(&h_running_), sizeof(int)) != cudaSuccess ||
-        cudaMallocHost(reinterpret_cast<void**>(&h_flag_), sizeof(uint32_t)) != cudaSuccess ||
-        cudaMallocHost(reinterpret_cast<void**>(&h_gave_up_), 2 * sizeof(uint32_t)) !=
-          cudaSuccess) {
+    // (one allocation: page-locking takes a tenth of a millisecond each time)
+    if (cudaMallocHost(reinterpret_cast<void**>(&h_words_), 4 * sizeof(uint32_t)) != cudaSuccess) {
         throw std::bad_alloc();
     }
-    h_gave_up_[0] = h_gave_up_[1] = 0u;
+    std::fill(h_words_, h_words_ + 4, 0u);
+    h_running_ = reinterpret_cast<int*>(h_words_);
+    h_flag_ = h_words_ + 1;
+    h_gave_up_ = h_words_ + 2;
     a_.gave_up = h_gave_up_;
     a_.drift_seen = h_gave_up_ + 1;
     cudaMemset(d_ss_, 0, sizeof(SceneState) * max_scenes_);
@@ -419,9 +419,7 @@ Engine::~Engine() {
     for (auto e : event_pool_) cudaEventDestroy(e);
     if (sort_buf_) cudaFree(sort_buf_);
     for (void* p : allocations_) cudaFree(p);
-    if (h_running_) cudaFreeHost(h_running_);
-    if (h_flag_) cudaFreeHost(h_flag_);
-    if (h_gave_up_) cudaFreeHost(h_gave_up_);
+    if (h_words_) cudaFreeHost(h_words_);
 }
 
 void Engine::count_kernels(int kernels) {
@@ -1090,6 +1088,9 @@ void Engine::emit_substep(int32_t method, bool reorder) {
     cudaEventRecord(ev_join_, side_st_);
     cudaGraph_t body;
     conditional_node(cond, cudaGraphCondTypeIf, &body);
+    if (!path_st_ && cudaStreamCreateWithFlags(&path_st_, cudaStreamNonBlocking) != cudaSuccess) {
+        throw std::runtime_error("stream creation failed");
+    }
     if (cudaStreamBeginCaptureToGraph(path_st_, body, nullptr, nullptr, 0,
                                       cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
         throw std::runtime_error("graph capture: path");
@@ -1216,6 +1217,7 @@ void Engine::emit_phases(int32_t method) {
 
 void Engine::abort_capture() {
     for (cudaStream_t sst : {body_st_, path_st_, frame_st_, cap_st_}) {
+        if (!sst) continue;
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(sst, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) {
             cudaGraph_t dead = nullptr;

@@ -327,6 +327,7 @@ private:
     int32_t* d_stile_scene_ = nullptr;
     uint32_t* d_scan_ = nullptr;
     int* d_running_ = nullptr;
+    uint32_t* h_words_ = nullptr;  // page-locked: the words below
     int* h_running_ = nullptr;
     uint32_t* d_flag_ = nullptr;
     uint32_t* h_flag_ = nullptr;

@@ -42,3 +42,16 @@ def test_frames_of_either_solve_count_their_own(E):
     want = launches(c, lambda: c.frame("dfsph_p"))
     assert launches(a, lambda: a.frame("dfsph_p")) == want
     assert launches(b, lambda: b.frame("dfsph_p")) == want
+
+
+def test_timing_with_and_without_the_resident_solve(E):
+    """Timed sub-steps run the kernels per phase unless the caller asks for
+    the solve they would run untimed."""
+    sim = E.Simulation.from_block_scene(scene(E, 97, 61))
+    sim.enable_timing(True)
+    sim.advance("dfsph_p", 1)
+    assert "dfsph_density" in sim.kernel_times() and "solve" not in sim.kernel_times()
+    sim.enable_timing(True, resident=True)
+    sim.advance("dfsph_p", 1)
+    assert "solve" in sim.kernel_times() and "dfsph_density" not in sim.kernel_times()
+    sim.enable_timing(False)
