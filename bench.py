@@ -77,7 +77,7 @@ def clock_sampler(gpu_index, path):
     try:
         f = open(path, "w")
         p = subprocess.Popen(["nvidia-smi", "-i", str(gpu_index), "--query-gpu=" + q,
-                              "--format=csv,noheader,nounits", "-lms", "200"], stdout=f,
+                              "--format=csv,noheader,nounits", "-lms", "20"], stdout=f,
                              stderr=subprocess.DEVNULL)
         return p, f
     except Exception:
@@ -140,8 +140,8 @@ def traffic_from_profile(kernel, n=None):
 # What bounds a kernel whose HBM fraction is low by design (from its ncu
 # summary under profiles/).
 LIMITERS = {
-    "solve": "the exchanges of neighbouring blocks' values: the lists and the gathered values "
-             "stay on the chip for all iterations (profiles/k_resident_solve.md)",
+    "solve": "waits at block barriers (48% of the stall) around the exchanges of neighbouring "
+             "blocks' values; lists and gathered values stay on the chip (profiles/k_resident_solve.dfsph_262k.md)",
     "neighbors_fluid": "instruction issue: 58% of issue slots busy, 3-4% of peak DRAM "
                        "throughput (profiles/k_neighbors.dfsph_262k.md)",
 }
@@ -268,12 +268,19 @@ def run_gpu(args):
 
     for _ in range(args.warmup):
         sim.advance("dfsph_p", 1, stats=False)
+    # (the sampler starts with the tuner, which runs the same sub-steps: the
+    # timed region is shorter than the sampler's own start)
+    clocks_path = "/tmp/emerald_clocks_%d.csv" % rank
+    smi, smi_file = clock_sampler(local, clocks_path)
+    t_smi = time.perf_counter()
+    while smi is not None and not os.path.getsize(clocks_path):
+        if time.perf_counter() - t_smi > 3.0:
+            break
+        sim.advance("dfsph_p", 0)
     tuning = sim.autotune("dfsph_p")  # gather-kernel chunks, same bits either way
     barrier()
 
     # device-resident timing: one event pair per sub-step, L2 flushed between
-    clocks_path = "/tmp/emerald_clocks_%d.csv" % rank
-    smi, smi_file = clock_sampler(local, clocks_path)
     # kernels of this simulation, loop bodies counted per executed iteration
     launches0 = sim.kernel_launches()
     ev = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))

@@ -306,8 +306,8 @@ Engine::Engine(uint32_t fluid_capacity, uint32_t solid_capacity, int max_scenes)
     a_.ns_idx = static_cast<uint32_t*>(dev(4 * E));
     a_.ns_w = static_cast<float*>(dev(4 * E));
     a_.ns_gw = static_cast<float2*>(dev(8 * E));
-    // (between binning and scatter only; the staging of the re-sort and of the
-    // accessors is free then)
+    // (from binning to the scatter, the ranks to the fluid search; the staging of
+    // the re-sort and of the accessors is free then)
     a_.slot = reinterpret_cast<uint32_t*>(a_.tkdiv);
     a_.rank = reinterpret_cast<uint32_t*>(a_.tkdens);
     a_.members = static_cast<uint32_t*>(dev(4 * N));

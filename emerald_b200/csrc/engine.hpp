@@ -263,7 +263,7 @@ private:
     void destroy_graphs();
     void capture_frame(int32_t method, bool reorder);
     void prepare_substep(int32_t method, bool frame);
-    // The resident solve (resident_kernels.cu): whether sub-steps of `method`
+    // The resident solve (resident_solve.cuh): whether sub-steps of `method`
     // run it now, and its division of the active scenes among blocks.
     bool use_resident(int32_t method);
     template <class F>

@@ -173,7 +173,7 @@ void launch_pc_density(Arena const& a, uint32_t tiles, cudaStream_t st, bool com
 void launch_pc_forces(Arena const& a, uint32_t tiles, cudaStream_t st, bool comp);
 void launch_pc_final(Arena const& a, uint32_t tiles, cudaStream_t st);
 
-// resident solve (resident_kernels.cu): everything of a sub-step after the
+// resident solve (resident_solve.cuh): everything of a sub-step after the
 // neighbour lists as one cooperative launch
 constexpr int kResidentForms = 4;
 struct ResidentLimits {

@@ -1,6 +1,6 @@
 // Per-particle sums of the five solvers, shared by the launch-per-phase
 // kernels (solve_kernels.cu) and the resident solve kernel
-// (resident_kernels.cu): both run these functions, so their results are the
+// (resident_solve.cuh): both run these functions, so their results are the
 // same operations in the same order, bit for bit.
 //
 // A function takes the particle's own values, and views of what it folds over:
