@@ -599,6 +599,7 @@ int emerald_batch_synchronize(emerald_batch* batch) {
     if (!batch) return fail(EMERALD_EINVAL, "batch is NULL");
     return guarded([&] {
         cudaStreamSynchronize(batch->engine.stream());
+        batch->engine.host_waited();
         batch->engine.check("synchronize");
         batch->engine.check_solved(-1);
         return EMERALD_OK;

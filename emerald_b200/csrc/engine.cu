@@ -50,6 +50,9 @@ constexpr uint32_t kHeldTiles = 56;
 // resident solve, without the watch: DFSPH_P 14 tiles 0.84, 20 1.01, 28 1.09,
 // 41 1.61, 55 1.62, 104 2.13; AP 23 0.86, 34 1.25, 55 1.38; IISPH 14 0.68,
 // 23 1.57; PCISPH 8 0.70, 15 1.22.
+// Sub-steps of a new flow that the host launches without a wait before they
+// choose on the device.
+constexpr int64_t kBlindSubsteps = 32;
 struct DriftRule {
     uint32_t plain, halo;
 };
@@ -527,9 +530,8 @@ void Engine::scenes_changed(bool added) {
     order_stale_ = order_stale_ || added;
     int used = 0;
     for (auto const& sc : scenes_) used += sc.used ? 1 : 0;
-    if (used > 1) return;
-    cudaMemsetAsync(a_.control, 0, sizeof(SolveControl), st_);
-    h_gave_up_[1] = 0u;
+    if (used <= 1) cudaMemsetAsync(a_.control, 0, sizeof(SolveControl), st_);
+    if (used <= 1 || (added && h_gave_up_[1] == kInOrder)) h_gave_up_[1] = kUnknown;
 }
 
 int Engine::add_scene(SceneSpec const& spec) {
@@ -1471,8 +1473,9 @@ bool Engine::use_resident(int32_t method) {
 int Engine::solve_path(int32_t method, bool frame) {
     if (!use_resident(method)) return kPhases;
     if (!drift_limit_[method]) return kResident;
-    bool const seen = reinterpret_cast<uint32_t volatile*>(h_gave_up_)[1] != 0u;
-    return frame || seen ? kWatched : kReported;
+    uint32_t const seen = reinterpret_cast<uint32_t volatile*>(h_gave_up_)[1];
+    bool const far_ahead = substeps_launched_ - seen_substeps_ >= kBlindSubsteps;
+    return frame || seen == kDriftSeen || (seen == kUnknown && far_ahead) ? kWatched : kReported;
 }
 
 // Divides the active scenes' warp tiles among the resident blocks: a scene's
@@ -1825,6 +1828,7 @@ bool Engine::set_state(int id, float const* x, float const* v, bool sync) {
         // another flow, perhaps: the next re-sort gives it a try
         if (drift_limit_[scenes_[id].p.method]) {
             cudaMemsetAsync(&a_.control->wait, 0, 8, st_);  // and left
+            if (h_gave_up_[1] == kInOrder) h_gave_up_[1] = kUnknown;
         }
     }
     if (v) launch_scatter_f2(a_, b, n, a_.tv + b, a_.v, st_);

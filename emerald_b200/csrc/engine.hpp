@@ -204,6 +204,9 @@ public:
     // wait; returns the sub-steps run and the scene's state after them.
     int frame(int id, int32_t method, SceneState& out);
 
+    // The caller has waited for the engine's stream.
+    void host_waited() { seen_substeps_ = substeps_launched_; }
+
     void check(char const* what);
 
     // Picks the fastest chunk settings of `method`'s gather kernels by timing
@@ -279,8 +282,10 @@ private:
     void host_wait(cudaStream_t s) {
         ++host_waits_;
         cudaStreamSynchronize(s);
+        host_waited();
     }
     int64_t host_waits_ = 0;
+    int64_t seen_substeps_ = 0;  // launched when the host last waited for the device
     std::map<int32_t, ResidentLimits> limits_;  // key: method * 2 + compensated
     ResidentPlan plans_[5] = {};       // per method
     std::vector<GangPart> parts_;

@@ -181,7 +181,7 @@ struct Arena {
     SolveControl* control;
     GangRecord* records;
     uint32_t* gave_up;       // host memory: some wait of a resident solve has given up
-    uint32_t* drift_seen;    // host memory: a resident solve has reported a drift above its limit
+    uint32_t* drift_seen;    // host memory: what is known of the drift (DriftSeen)
     uint32_t inject;         // (tests) waits that cannot end: 1 at a barrier, 2 for values
     int32_t batch;  // the arena holds more than one scene slot (loop kernels walk the work list)
     int32_t const* tile_scene;   // fluid tile -> scene (-1: free)

@@ -94,12 +94,16 @@ void launch_frame_check(Arena const& a, int nscenes, int slot, cudaGraphConditio
                         cudaStream_t st);
 // How a sub-step is solved: by the kernels per phase, the resident solve,
 // whichever of the two its first kernel chooses, or the resident solve while
-// that kernel tells the host (Arena::drift_seen) when it would choose otherwise.
-// A graph that holds both solves takes the host and the device longer to launch
-// (262,144 particles, a sub-step of 640 us as a graph of its own: 130 us more),
-// so frames, whose graph is launched once, choose on the device, and sub-steps
-// begin to when a drift has been seen.
+// that kernel tells the host what it would choose (Arena::drift_seen). A graph
+// that holds both solves takes 0.3 ms longer to record and 5 us longer to run,
+// and batches whose scenes come and go record theirs often (16 served requests
+// 18.0 against 16.9 ms). So frames, whose graph is launched once, choose on the
+// device; sub-steps do when a drift has been seen, and when the host has
+// launched many of a new flow without waiting for one.
 enum SolvePath : int { kPhases = 0, kResident = 1, kWatched = 2, kReported = 3, kPaths = 4 };
+// Arena::drift_seen: a drift above its limit was reported, or none between two
+// sorts of the storage; nothing is known of a new flow.
+enum DriftSeen : uint32_t { kUnknown = 0, kDriftSeen = 1, kInOrder = 2 };
 struct SolveChoice {
     uint32_t const* limit;  // device: drift above which the kernels per phase are faster
     cudaGraphConditionalHandle cond;  // of their node (use_cond: inside a graph)

@@ -308,6 +308,7 @@ void Server::loop(Lane& lane) {
                 cudaEventRecord(lane.marks[size_t(s) + 1], lane.stream);
             }
             cudaEventSynchronize(lane.marks[size_t(k)]);
+            engine.host_waited();
             for (int32_t s = 0; s < k; ++s) {
                 cudaEventElapsedTime(&step_ms[size_t(s)], lane.marks[size_t(s)],
                                      lane.marks[size_t(s) + 1]);

@@ -124,17 +124,18 @@ __device__ int to_int_x86(double d) {
 // after three, up to 31. One thread; returns whether by the kernels per phase.
 __device__ bool choose_solve(Arena const& a, SolveChoice const& ch) {
     SolveControl& c = *a.control;
+    uint32_t volatile* const seen = a.drift_seen;
     if (c.in_order) {
         if (!c.drifted) {
-            // in order all the while between two sorts
             c.wait = 0u;
-            *reinterpret_cast<uint32_t volatile*>(a.drift_seen) = 0u;
+            if (c.drift && c.drift <= *ch.limit) *seen = kInOrder;
         } else if (c.left) {
             --c.left;
         } else {
             c.drifted = 0u;
         }
     } else if (c.drift > *ch.limit && !c.drifted) {
+        *seen = kDriftSeen;
         c.drifted = 1u;
         c.wait = min(2u * c.wait + 1u, 31u);
         c.left = c.wait;
@@ -223,10 +224,12 @@ __global__ void k_begin_substep(Arena a, int nscenes, int path, SolveChoice ch) 
         if (path == kWatched) {
             per_phase = choose_solve(a, ch);
         } else if (path == kReported) {
+            uint32_t volatile* const seen = a.drift_seen;
             if (c.in_order) {
+                if (c.drift && c.drift <= *ch.limit) *seen = kInOrder;
                 c.in_order = c.drift = 0u;
             } else if (c.drift > *ch.limit) {
-                *reinterpret_cast<uint32_t volatile*>(a.drift_seen) = 1u;
+                *seen = kDriftSeen;
             }
         }
     }

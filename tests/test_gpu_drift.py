@@ -148,3 +148,18 @@ def test_drift_in_a_batch_whose_scenes_change(E):
     for name, x, y in zip("xv", b.state(sid), p.state()):
         assert_bitwise(x, y, name)
     b.close()
+
+
+def test_drift_within_one_long_call(E):
+    """A mixing flow advanced by one call that the host does not wait in: the
+    sub-steps past the thirty-second choose on the device."""
+    sc = mixing(E, 440)
+    a = E.Simulation.from_block_scene(sc)
+    p = E.Simulation.from_block_scene(sc)
+    p.set_tuning(PINNED)
+    got = launches(a, lambda: a.advance("dfsph_p", 150, stats=False))
+    p.advance("dfsph_p", 60, stats=False)
+    want = launches(p, lambda: p.advance("dfsph_p", 90, stats=False))
+    assert 2 * got > want
+    for name, x, y in zip("xv", a.state(), p.state()):
+        assert_bitwise(x, y, name)
