@@ -1723,7 +1723,8 @@ Engine::TuneReport Engine::autotune(int32_t method, int substeps) {
         per_phase_ = false;
         if (use_resident(method)) {
             bool const slower = time_of(best_t) >= best;
-            if (!control.drifted) {
+            uint32_t const limit = drift_limit_[method];
+            if (!control.drifted && !(limit && control.drift > limit)) {
                 std::pair<uint64_t, bool> const key{tuning_key(method), compensated_};
                 std::lock_guard<std::mutex> lock(g_tuning_mutex);
                 if (slower) {
