@@ -119,10 +119,13 @@ __device__ __forceinline__ int find_neighbors(float2 pos,
     int32_t gx, gy;
     grid_coord(pos, cell, gx, gy);
     int cnt = 0;
-    for (int32_t j = gy - 1; cnt < kMaxNeighbors && j <= gy + 1; ++j) {
-        for (int32_t k = gx - 1; cnt < kMaxNeighbors && k <= gx + 1; ++k) {
+    // (offsets, and cells as their bit patterns: a position too far out is in
+    // the last cell of an int32, whose neighbour wraps)
+    for (uint32_t j = 0; cnt < kMaxNeighbors && j < 3; ++j) {
+        for (uint32_t k = 0; cnt < kMaxNeighbors && k < 3; ++k) {
             uint32_t slot;
-            uint64_t const z = morton2(static_cast<uint32_t>(k), static_cast<uint32_t>(j));
+            uint64_t const z = morton2(static_cast<uint32_t>(gx) + k - 1u,
+                                       static_cast<uint32_t>(gy) + j - 1u);
             if (!table_find(o.keys, o.log2cap, z, slot)) continue;
             uint32_t const b = o.start[slot];
             uint32_t const e = b + o.count[slot];
@@ -240,8 +243,8 @@ __device__ __forceinline__ void cell_ranges(OtherSet const& o, int32_t gx, int32
     uint64_t zx[3], zy[3];
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-        zx[q] = spread_bits(static_cast<uint32_t>(gx - 1 + q));
-        zy[q] = spread_bits(static_cast<uint32_t>(gy - 1 + q)) << 1;
+        zx[q] = spread_bits(static_cast<uint32_t>(gx) + static_cast<uint32_t>(q) - 1u);
+        zy[q] = spread_bits(static_cast<uint32_t>(gy) + static_cast<uint32_t>(q) - 1u) << 1;
     }
     uint32_t slot[9];
     uint64_t k[9];

@@ -21,8 +21,8 @@ namespace {
 __device__ __forceinline__ uint32_t local_morton(float2 p, float cell) {
     int32_t gx, gy;
     grid_coord(p, cell, gx, gy);
-    int32_t const ox = min(max(gx + 64, 0), 4095);
-    int32_t const oy = min(max(gy + 64, 0), 4095);
+    int32_t const ox = min(max(gx, -64), 4031) + 64;
+    int32_t const oy = min(max(gy, -64), 4031) + 64;
     return static_cast<uint32_t>(morton2(static_cast<uint32_t>(ox), static_cast<uint32_t>(oy)));
 }
 

@@ -40,3 +40,31 @@ def test_nan_position_adds_nothing(h, spacing):
     assert_bitwise(g1[:n], g0, "GradW")
     assert c1[n] == near.sum() if near.sum() <= 64 else c1[n] == 64
     assert not w1[n].any() and not g1[n].any()
+
+
+@pytest.mark.parametrize("where", [(1e12, 1e12), (-1e12, 3e11), (0.3, -1e30), (3e38, 0.2)])
+@pytest.mark.parametrize("m", [2, 17, 18, 65, 80])
+def test_coincident_points_too_far_out_for_a_cell(where, m):
+    """Cells are int32; positions past them share the outermost one. Points at
+    the same place there are each other's neighbours like anywhere else: the
+    first 64 by index, at distance 0, W(0) and no gradient."""
+    import torch
+
+    import emerald_b200 as E
+    h = F(0.0123)
+    rng = np.random.Generator(np.random.PCG64(m))
+    far = np.full((m, 2), 0, np.float32) + np.float32(where)
+    near = rng.uniform(0.0, 1.0, (40, 2)).astype(np.float32)
+    xy = np.concatenate([far, near])
+    counts, idx, w, gw = static_lists(E, torch, xy, h)
+    c0, i0, w0, g0 = static_lists(E, torch, near, h)
+    assert_bitwise(counts[m:], c0, "counts of the others")
+    assert_bitwise(w[m:], w0, "W of the others")
+    k = min(m - 1, 64)
+    assert (counts[:m] == k).all()
+    for i in range(m):
+        want = [j for j in range(m) if j != i][:64]
+        assert idx[i, :k].tolist() == want
+    at_zero = F(1) / (h * h * h * F(3.14159274101257324218750))
+    assert (w[:m, :k] == at_zero).all()
+    assert not gw[:m].any()
