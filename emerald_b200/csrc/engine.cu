@@ -50,14 +50,14 @@ constexpr uint32_t kHeldTiles = 56;
 // resident solve, without the watch: DFSPH_P 14 tiles 0.84, 20 1.01, 28 1.09,
 // 41 1.61, 55 1.62, 104 2.13; AP 23 0.86, 34 1.25, 55 1.38; IISPH 14 0.68,
 // 23 1.57; PCISPH 8 0.70, 15 1.22.
-// Sub-steps of a new flow that the host launches without a wait before they
-// choose on the device.
-constexpr int64_t kBlindSubsteps = 32;
 struct DriftRule {
     uint32_t plain, halo;
 };
 constexpr DriftRule kDriftRules[5] = {{12, 12}, {16, 16}, {28, 48}, {28, 48}, {16, 36}};
 constexpr uint32_t kDriftRoots = 14;
+// Sub-steps of a new flow that the host launches without a wait before they
+// choose on the device.
+constexpr int64_t kBlindSubsteps = 32;
 // Batches of fewer warp tiles (2,048 particles) keep the launch-per-phase
 // kernels. The resident solve is the faster one there too (48 requests of 128
 // to 512 particles through one lane: 17.5 against 20.4 ms on B200), but a
@@ -66,7 +66,7 @@ constexpr uint32_t kDriftRoots = 14;
 // stream of them would no longer work side by side, as the request loop's
 // tests require.
 constexpr uint32_t kMinBatchTiles = 64;
-
+// A scene with one of them was not solved to the end in some sub-step.
 constexpr int kStallBits = kErrStalled | kErrUnsolved;
 
 // How many error sums s = 0, 1, ... pass the solvers' average test
